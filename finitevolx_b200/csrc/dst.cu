@@ -16,9 +16,9 @@
 // K-major TMA tile.  Precision: 3xBF16 split (X = Xh + Xl, S = Sh + Sl,
 // C = Xh Sh + Xh Sl + Xl Sh) with FP32 accumulation in TMEM; the epilogue
 // writes the next product's operand already split into bf16 hi/lo.  An FP64
-// SIMT form of the same chain is the correctness path, and the FP64 solve
-// recovers full accuracy by iterative refinement with an FP64 residual.
-#include "fvx_common.cuh"
+// form of the same chain (dst_f64.cuh) is the correctness path, and the FP64
+// solve recovers full accuracy by iterative refinement with an FP64 residual.
+#include "dst_f64.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -56,7 +56,6 @@ struct Epi {
   int off_n, off_r;        // index offsets into the output (e.g. a ghost ring)
   double alpha;
   const float* inv_eig;    // [n_eig][N][R] scale 1/Lambda, or null
-  const double* inv_eig64;
   int n_eig;               // batch b uses grid b % n_eig
   int* err;
   int perm_r = 0;          // store r at its even/odd de-interleaved position (the next product's layout)
@@ -812,82 +811,6 @@ gemm_sym_pair_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_const
   }
 }
 
-// ---- FP64 SIMT GEMM with the same transposed-store epilogue (correctness path)
-// TDT x TDT output tiles, 256 threads, each (TDT / 16)^2 outputs; every
-// output's FMA chain runs over k in order, so the tile size does not change
-// the result.  The largest tile that still gives at least one CTA per SM is
-// used (64, else 32, else 16).
-template <int TDT> struct F64Cfg {
-  // k-block: small tiles stage long k-blocks (few dependent load round trips
-  // per output); large tiles are bound by their FMAs
-  static constexpr int DK = TDT == 16 ? 128 : 16;
-};
-template <int TDT>
-__global__ void __launch_bounds__(256)
-gemm_f64_kernel(const double* A, int lda, const double* __restrict__ S, int lds, int M, int N, int K, Epi ep) {
-  constexpr int R = TDT / 16, DK = F64Cfg<TDT>::DK, NL = TDT * DK / 256;  // loads per thread per operand
-  static_assert(TDT * DK % 256 == 0, "whole loads per thread");
-  __shared__ double As[DK][TDT + 1];
-  __shared__ double Ss[DK][TDT + 1];
-  // launched as a programmatic dependent: A (and the output) belong to the
-  // kernel before until the wait; A is then read through L2 (__ldcg, no
-  // restrict), so no load of it can be placed before the wait
-  grid_dep_wait();
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int m0 = blockIdx.y * TDT, n0 = blockIdx.x * TDT;
-  double acc[R][R] = {};
-  for (int k0 = 0; k0 < K; k0 += DK) {
-    {  // every load of the k-block in flight before any is stored
-      double va[NL], vs[NL];
-#pragma unroll
-      for (int u = 0; u < NL; ++u) {
-        const int t = threadIdx.x + u * 256;
-        const int mm = t / DK, kk = t % DK, gm = m0 + mm, gk = k0 + kk;
-        va[u] = (gm < M && gk < K) ? __ldcg(A + (long long)gm * lda + gk) : 0.0;
-        const int kk2 = t / TDT, nn = t % TDT, gk2 = k0 + kk2, gn = n0 + nn;
-        vs[u] = (gk2 < K && gn < N) ? S[(long long)gk2 * lds + gn] : 0.0;
-      }
-#pragma unroll
-      for (int u = 0; u < NL; ++u) {
-        const int t = threadIdx.x + u * 256;
-        As[t % DK][t / DK] = va[u];
-        Ss[t / TDT][t % TDT] = vs[u];
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < DK; ++kk) {
-      double a[R], s[R];
-#pragma unroll
-      for (int i = 0; i < R; ++i) { a[i] = As[kk][ty + 16 * i]; s[i] = Ss[kk][tx + 16 * i]; }
-#pragma unroll
-      for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < R; ++j) acc[i][j] = fma(a[i], s[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  // the next kernel may launch while this one stores its results
-  grid_dep_launch();
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int m = m0 + ty + 16 * i;
-    if (m >= M) continue;
-    const int b = m / ep.rows_per_batch, r = m - b * ep.rows_per_batch;
-#pragma unroll
-    for (int j = 0; j < R; ++j) {
-      const int n = n0 + tx + 16 * j;
-      if (n >= N) continue;
-      double x = acc[i][j] * ep.alpha;
-      if (ep.inv_eig64) x *= ep.inv_eig64[((long long)(b % ep.n_eig) * ep.n_cols + n) * ep.rows_per_batch + r];
-      long long idx = (long long)b * ep.batch_stride + (long long)(n + ep.off_n) * ep.ld + (r + ep.off_r);
-      if (ep.mode == EPI_F64_ACC) ((double*)ep.out0)[idx] += x;
-      else if (ep.mode == EPI_F32) ((float*)ep.out0)[idx] = (float)x;
-      else ((double*)ep.out0)[idx] = x;
-    }
-  }
-}
-
 // ---- input split / copy / residual kernels ---------------------------------
 // perm: store x at its de-interleaved position (the even/odd product's
 // operand layout).
@@ -1138,21 +1061,6 @@ static int gemm_sym(const bf16* Xh, const bf16* Xl, int M, int K, const bf16* Ph
   return fvx_cuda_status();
 }
 
-static int gemm_f64(const double* A, int lda, int M, int K, const double* S, int N, const Epi& ep, cudaStream_t st) {
-  auto tiles = [&](int t) { return (long long)((N + t - 1) / t) * ((M + t - 1) / t); };
-  const int t = tiles(64) >= 148 ? 64 : (tiles(32) >= 148 ? 32 : 16);
-  dim3 grid((N + t - 1) / t, (M + t - 1) / t);
-  if (grid.y > 65535) return FVX_ERR_SHAPE;
-  // programmatic dependent launch: the set-up overlaps the previous
-  // kernel's tail (the kernel waits before touching its data)
-  cudaError_t e;
-  if (t == 64) e = fvx_launch_pdl(gemm_f64_kernel<64>, grid, dim3(256), 0, st, A, lda, S, N, M, N, K, ep);
-  else if (t == 32) e = fvx_launch_pdl(gemm_f64_kernel<32>, grid, dim3(256), 0, st, A, lda, S, N, M, N, K, ep);
-  else e = fvx_launch_pdl(gemm_f64_kernel<16>, grid, dim3(256), 0, st, A, lda, S, N, M, N, K, ep);
-  if (e != cudaSuccess) return FVX_ERR_CUDA;
-  return fvx_cuda_status();
-}
-
 static int grid1d(long long n) {
   long long b = (n + 255) / 256;
   return (int)(b > 148 * 32 ? 148 * 32 : (b < 1 ? 1 : b));
@@ -1176,12 +1084,14 @@ struct fvx_dst_plan {
   bool sym = false;  // even/odd products (nx, ny multiples of 256); operands x/y de-interleaved
   bf16 *xPh = nullptr, *xPl = nullptr, *xQh = nullptr, *xQl = nullptr;  // [nx/2][nx/2]
   bf16 *yPh = nullptr, *yPl = nullptr, *yQh = nullptr, *yQl = nullptr;  // [ny/2][ny/2]
-  double *Sx64 = nullptr, *Sy64 = nullptr;
   // inverse-transform operands (DCT-II, periodic); the DST-I plan reuses S
   bf16 *Ixh = nullptr, *Ixl = nullptr, *Iyh = nullptr, *Iyl = nullptr;
-  double *Ix64 = nullptr, *Iy64 = nullptr;
+  // FP64 chain: folded tables [hx][kx], [hy][ky] (forward F, inverse I; the
+  // DST-I plan has one) and the eigenvalues along both spectral axes.  kx,
+  // ky: length of a folded axis (2 hx, 2 hy), the table pitch
+  int hx = 0, hy = 0, kx = 0, ky = 0, mirx = 0, miry = 0;
+  double *Fx64 = nullptr, *Fy64 = nullptr, *Ix64 = nullptr, *Iy64 = nullptr, *ex64 = nullptr, *ey64 = nullptr;
   float* inv32 = nullptr;   // [n_lam][ny][nx]
-  double* inv64 = nullptr;  // [n_lam][ny][nx]
   bf16 *W1h = nullptr, *W1l = nullptr, *W2h = nullptr, *W2l = nullptr;
   double *V1 = nullptr, *V2 = nullptr;  // FP64 chain work
   double* norms = nullptr;              // [4]
@@ -1191,10 +1101,10 @@ struct fvx_dst_plan {
 };
 
 static void dst_free(fvx_dst_plan* p) {
-  void* ptrs[] = {p->lam_dev, p->Sxh, p->Sxl, p->Syh, p->Syl, p->Sx64, p->Sy64, p->inv32, p->inv64,
+  void* ptrs[] = {p->lam_dev, p->Sxh, p->Sxl, p->Syh, p->Syl, p->Fx64, p->Fy64, p->inv32,
                   p->W1h,     p->W1l, p->W2h, p->W2l, p->V1,  p->V2,  p->norms, p->err,
                   p->xPh,     p->xPl, p->xQh, p->xQl, p->yPh, p->yPl, p->yQh,   p->yQl,
-                  p->Ixh,     p->Ixl, p->Iyh, p->Iyl, p->Ix64, p->Iy64};
+                  p->Ixh,     p->Ixl, p->Iyh, p->Iyl, p->Ix64, p->Iy64, p->ex64, p->ey64};
   for (void* q : ptrs)
     if (q) cudaFree(q);
 }
@@ -1248,6 +1158,55 @@ static void transform_pair(int kind, int n, double h, std::vector<double>& T, st
   }
 }
 
+// The folded FP64 tables of one axis (forms in dst_f64.cuh), [h][k] with
+// zeros past the last column, and its eigenvalues in the order of the
+// spectral index the forward product writes.
+//   DST-I: row n of S for n < h; F serves both directions.
+//   DCT-II: F[n] = coefficients 2n (even columns) and 2n + 1 (odd columns)
+//          of sample j in column pair j; I[n] = row n of Tinv.
+//   periodic: cosine coefficients in the even columns, sine in the odd ones;
+//          the inverse's weights are 1/n for k = 0 and k = n/2, else 2/n.
+static void upload_folded(int kind, int n, int h, int k, const std::vector<double>& T, const std::vector<double>& Ti,
+                          const std::vector<double>& e, double* F, double* I, double* ed) {
+  std::vector<double> f((size_t)h * k, 0.0), b, es(k, 0.0);
+  if (kind == FVX_SPECTRAL_DST) {
+    for (int r = 0; r < h; ++r)
+      for (int j = 0; j < n; ++j) f[(size_t)r * k + j] = T[(size_t)r * n + j];
+    for (int j = 0; j < n; ++j) es[j] = e[j];
+  } else if (kind == FVX_SPECTRAL_DCT) {
+    b.assign((size_t)h * k, 0.0);
+    for (int r = 0; r < h; ++r) {
+      for (int j = 0; j < h; ++j) {
+        f[(size_t)r * k + 2 * j] = T[(size_t)(2 * r) * n + j];
+        if (2 * r + 1 < n) f[(size_t)r * k + 2 * j + 1] = T[(size_t)(2 * r + 1) * n + j];
+      }
+      for (int j = 0; j < n; ++j) b[(size_t)r * k + j] = Ti[(size_t)r * n + j];
+    }
+    for (int j = 0; j < n; ++j) es[j] = e[j];
+  } else {
+    b.assign((size_t)h * k, 0.0);
+    std::vector<double> cs(n), sn(n);
+    for (int q = 0; q < n; ++q) {
+      const double t = 2.0 * M_PI * (double)q / (double)n;
+      cs[q] = std::cos(t);
+      sn[q] = std::sin(t);
+    }
+    for (int r = 0; r < h; ++r)
+      for (int j = 0; j < h; ++j) {
+        const int q = (int)(((long long)r * j) % n);
+        const double w = (j == 0 || 2 * j == n ? 1.0 : 2.0) / n;
+        f[(size_t)r * k + 2 * j] = cs[q];
+        f[(size_t)r * k + 2 * j + 1] = sn[q];
+        b[(size_t)r * k + 2 * j] = w * cs[q];
+        b[(size_t)r * k + 2 * j + 1] = w * sn[q];
+      }
+    for (int j = 0; j < h; ++j) es[2 * j] = es[2 * j + 1] = e[j < n ? j : 0];
+  }
+  cudaMemcpy(F, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice);
+  if (I) cudaMemcpy(I, b.data(), sizeof(double) * b.size(), cudaMemcpyHostToDevice);
+  cudaMemcpy(ed, es.data(), sizeof(double) * es.size(), cudaMemcpyHostToDevice);
+}
+
 extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, double dy, int batch_max,
                                         const double* lambdas, int n_lambda, int want_fp64, fvx_dst_plan** out);
 
@@ -1271,17 +1230,17 @@ extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, dou
   p->cfin = kind == FVX_SPECTRAL_DST ? 4.0 / ((double)(ny + 1) * (double)(nx + 1)) : 1.0;
   const bool dst = kind == FVX_SPECTRAL_DST;
   const size_t plane = (size_t)ny * nx, work = plane * batch_max;
+  // half lengths and mirror indices of the folded FP64 products (dst_f64.cuh)
+  const bool per = kind == FVX_SPECTRAL_PERIODIC;
+  p->hx = per ? nx / 2 + 1 : (nx + 1) / 2;
+  p->hy = per ? ny / 2 + 1 : (ny + 1) / 2;
+  p->kx = 2 * p->hx; p->ky = 2 * p->hy;
+  p->mirx = per ? nx : nx - 1; p->miry = per ? ny : ny - 1;
+  const bool want64 = want_fp64 || !p->split_ok;
   bool ok = true;
   auto A = [&](void** q, size_t bytes) { if (ok && cudaMalloc(q, bytes) != cudaSuccess) ok = false; };
   A((void**)&p->lam_dev, sizeof(double) * n_lambda);
-  A((void**)&p->Sx64, sizeof(double) * nx * nx);
-  A((void**)&p->Sy64, sizeof(double) * ny * ny);
-  if (!dst) {
-    A((void**)&p->Ix64, sizeof(double) * nx * nx);
-    A((void**)&p->Iy64, sizeof(double) * ny * ny);
-  }
   A((void**)&p->inv32, sizeof(float) * plane * n_lambda);
-  A((void**)&p->inv64, sizeof(double) * plane * n_lambda);
   A((void**)&p->norms, sizeof(double) * 4);
   A((void**)&p->err, sizeof(int));
   if (p->split_ok) {
@@ -1301,47 +1260,35 @@ extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, dou
     A((void**)&p->yPh, sizeof(bf16) * hy); A((void**)&p->yPl, sizeof(bf16) * hy);
     A((void**)&p->yQh, sizeof(bf16) * hy); A((void**)&p->yQl, sizeof(bf16) * hy);
   }
-  if (want_fp64 || !p->split_ok) {
-    A((void**)&p->V1, sizeof(double) * work);
-    A((void**)&p->V2, sizeof(double) * work);
+  if (want64) {
+    const size_t work64 = (size_t)p->kx * p->ky * batch_max;  // kx >= nx, ky >= ny
+    const size_t tx = (size_t)p->hx * p->kx, ty = (size_t)p->hy * p->ky;
+    A((void**)&p->V1, sizeof(double) * work64);
+    A((void**)&p->V2, sizeof(double) * work64);
+    A((void**)&p->Fx64, sizeof(double) * tx); A((void**)&p->Fy64, sizeof(double) * ty);
+    if (!dst) { A((void**)&p->Ix64, sizeof(double) * tx); A((void**)&p->Iy64, sizeof(double) * ty); }
+    A((void**)&p->ex64, sizeof(double) * p->kx); A((void**)&p->ey64, sizeof(double) * p->ky);
   }
   if (!ok) { dst_free(p); delete p; return FVX_ERR_CUDA; }
-  // host-side tables in FP64.  Operands: the tensor-core products read B
-  // as [out][in] (T itself for the forward, Tinv for the inverse); the FP64
-  // products read [in][out] (the transposes).
+  // host-side tables in FP64; the tensor-core products read B as [out][in]
+  // (T itself for the forward, Tinv for the inverse)
   std::vector<double> Tx, Tix, ex, Ty, Tiy, ey;
   transform_pair(kind, nx, dx, Tx, Tix, ex);
   transform_pair(kind, ny, dy, Ty, Tiy, ey);
-  auto transpose = [](const std::vector<double>& M, int n) {
-    std::vector<double> R(M.size());
-    for (int a = 0; a < n; ++a)
-      for (int b = 0; b < n; ++b) R[(size_t)b * n + a] = M[(size_t)a * n + b];
-    return R;
-  };
-  const std::vector<double> Sx = Tx, Sy = Ty;  // split operands [out][in]
-  std::vector<double> inv64(plane * n_lambda);
+  const std::vector<double>&Sx = Tx, &Sy = Ty;  // split operands [out][in]
   std::vector<float> inv32(plane * n_lambda);
   for (int l = 0; l < n_lambda; ++l)
     for (int j = 0; j < ny; ++j)
       for (int i = 0; i < nx; ++i) {
         // the null mode (Neumann / periodic Poisson) gets 0: the zero-mean solution
         const double d = (ey[j] + ex[i]) - lambdas[l];
-        const double v = d == 0.0 ? 0.0 : 1.0 / d;
-        inv64[(size_t)l * plane + (size_t)j * nx + i] = v;
-        inv32[(size_t)l * plane + (size_t)j * nx + i] = (float)v;
+        inv32[(size_t)l * plane + (size_t)j * nx + i] = (float)(d == 0.0 ? 0.0 : 1.0 / d);
       }
   cudaMemcpy(p->lam_dev, lambdas, sizeof(double) * n_lambda, cudaMemcpyHostToDevice);
-  {
-    const std::vector<double> fx = transpose(Tx, nx), fy = transpose(Ty, ny);
-    cudaMemcpy(p->Sx64, fx.data(), sizeof(double) * fx.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(p->Sy64, fy.data(), sizeof(double) * fy.size(), cudaMemcpyHostToDevice);
-    if (!dst) {
-      const std::vector<double> ix = transpose(Tix, nx), iy = transpose(Tiy, ny);
-      cudaMemcpy(p->Ix64, ix.data(), sizeof(double) * ix.size(), cudaMemcpyHostToDevice);
-      cudaMemcpy(p->Iy64, iy.data(), sizeof(double) * iy.size(), cudaMemcpyHostToDevice);
-    }
+  if (want64) {
+    upload_folded(kind, nx, p->hx, p->kx, Tx, Tix, ex, p->Fx64, p->Ix64, p->ex64);
+    upload_folded(kind, ny, p->hy, p->ky, Ty, Tiy, ey, p->Fy64, p->Iy64, p->ey64);
   }
-  cudaMemcpy(p->inv64, inv64.data(), sizeof(double) * inv64.size(), cudaMemcpyHostToDevice);
   cudaMemcpy(p->inv32, inv32.data(), sizeof(float) * inv32.size(), cudaMemcpyHostToDevice);
   if (p->split_ok) {
     auto split = [](const std::vector<double>& S, std::vector<bf16>& h, std::vector<bf16>& l) {
@@ -1440,7 +1387,7 @@ static Epi make_epi(fvx_dst_plan* p, int mode, int R, int M, int N, void* o0, vo
   Epi e;
   e.mode = mode; e.rows_per_batch = R; e.m_total = M; e.n_cols = N; e.out0 = o0; e.out1 = o1;
   e.batch_stride = bstride; e.ld = ld; e.off_n = off_n; e.off_r = off_r; e.alpha = alpha;
-  e.inv_eig = eig ? p->inv32 : nullptr; e.inv_eig64 = eig ? p->inv64 : nullptr; e.n_eig = p->n_lam;
+  e.inv_eig = eig ? p->inv32 : nullptr; e.n_eig = p->n_lam;
   e.err = p->err;
   e.wait_cycles = p->wait_cycles;
   e.stall = p->stall;
@@ -1485,20 +1432,53 @@ static int chain_split(fvx_dst_plan* p, int B, int out_mode, void* out, long lon
   return gemm_split(p->W2h, p->W2l, B * nx, ny, Iyh, Iyl, ny, e4, st);
 }
 
-static int chain_f64(fvx_dst_plan* p, int B, int out_mode, void* out, long long ob, long long old, cudaStream_t st) {
+// The FP64 chain: folded products (dst_f64.cuh) from the interior view
+// ``src`` (element (b, y, x) at src[b * sbs + y * sld + x]) to ``out``.  DST-I
+// reads src in place; the cosine and periodic chains fold it first.
+template <typename T>
+static int chain_f64(fvx_dst_plan* p, int B, const T* src, long long sbs, long long sld, bool out_f32, void* out,
+                     long long ob, long long old, cudaStream_t st) {
   const int ny = p->ny, nx = p->nx;
-  const double c = p->cfin;
   const bool dst = p->kind == FVX_SPECTRAL_DST;
-  const double* Ix = dst ? p->Sx64 : p->Ix64;
-  const double* Iy = dst ? p->Sy64 : p->Iy64;
+  auto product = [&](const double* X, long long xbs, long long xld, int R, int K, bool along_x, bool inverse, void* o,
+                     long long obs, long long old_, bool f32, double alpha, bool eig) {
+    FoldArgs a = {};
+    a.X = X; a.xbs = xbs; a.xld = xld; a.R = R; a.M = B * R; a.K = K;
+    a.T = along_x ? (inverse && !dst ? p->Ix64 : p->Fx64) : (inverse && !dst ? p->Iy64 : p->Fy64);
+    a.tld = along_x ? p->kx : p->ky;
+    a.NH = along_x ? p->hx : p->hy;
+    a.mir = dst || inverse ? (along_x ? p->mirx : p->miry) : -1;
+    a.n_out = along_x ? nx : ny;
+    a.out = o; a.obs = obs; a.old = old_; a.out_f32 = f32; a.alpha = alpha;
+    if (eig) { a.en = along_x ? p->ex64 : p->ey64; a.er = along_x ? p->ey64 : p->ex64; a.lam = p->lam_dev; a.n_lam = p->n_lam; }
+    return gemm_f64_fold(a, st);
+  };
   int rc;
-  Epi e1 = make_epi(p, EPI_F64, ny, B * ny, nx, p->V2, nullptr, (long long)nx * ny, ny, 0, 0, 1.0, false);
-  if ((rc = gemm_f64(p->V1, nx, B * ny, nx, p->Sx64, nx, e1, st))) return rc;
-  Epi e2 = make_epi(p, EPI_F64, nx, B * nx, ny, p->V1, nullptr, (long long)ny * nx, nx, 0, 0, 1.0, true);
-  if ((rc = gemm_f64(p->V2, ny, B * nx, ny, p->Sy64, ny, e2, st))) return rc;
-  if ((rc = gemm_f64(p->V1, nx, B * ny, nx, Ix, nx, e1, st))) return rc;
-  Epi e4 = make_epi(p, out_mode, nx, B * nx, ny, out, nullptr, ob, old, 0, 0, c, false);
-  return gemm_f64(p->V2, ny, B * nx, ny, Iy, ny, e4, st);
+  if (dst) {
+    const double* in = (const double*)src;
+    if constexpr (sizeof(T) != 8) {
+      if (fvx_launch_pdl(copy_in_f64_kernel<T>, dim3(copy_rows_grid((long long)B * ny)), dim3(256), 0, st, src, sbs,
+                         sld, ny, nx, B, p->V1) != cudaSuccess)
+        return FVX_ERR_CUDA;
+      if ((rc = fvx_cuda_status())) return rc;
+      in = p->V1; sbs = (long long)ny * nx; sld = nx;
+    }
+    const long long pl = (long long)ny * nx;
+    if ((rc = product(in, sbs, sld, ny, nx, true, false, p->V2, pl, ny, false, 1.0, false))) return rc;
+    if ((rc = product(p->V2, pl, ny, nx, ny, false, false, p->V1, pl, nx, false, 1.0, true))) return rc;
+    if ((rc = product(p->V1, pl, nx, ny, nx, true, true, p->V2, pl, ny, false, 1.0, false))) return rc;
+    return product(p->V2, pl, ny, nx, ny, false, true, out, ob, old, out_f32, p->cfin, false);
+  }
+  const long long pl = (long long)p->ky * p->kx;
+  if (fvx_launch_pdl(fold_in_f64_kernel<T>, dim3(copy_rows_grid((long long)B * p->hy)), dim3(256), 0, st, src, sbs, sld,
+                     ny, nx, p->hy, p->hx, p->miry, p->mirx, B, p->V2) != cudaSuccess)
+    return FVX_ERR_CUDA;
+  if ((rc = fvx_cuda_status())) return rc;
+  if ((rc = product(p->V2, pl, p->kx, p->ky, p->kx, true, false, p->V1, pl, p->ky, false, 1.0, false))) return rc;
+  if ((rc = product(p->V1, pl, p->ky, p->kx, p->ky, false, false, p->V2, pl, p->kx, false, 1.0, true))) return rc;
+  const long long pi = (long long)nx * p->ky;
+  if ((rc = product(p->V2, pl, p->kx, p->ky, p->kx, true, true, p->V1, pi, p->ky, false, 1.0, false))) return rc;
+  return product(p->V1, pi, p->ky, nx, p->ky, false, true, out, ob, old, out_f32, p->cfin, false);
 }
 
 // FP32 solve through the split-BF16 tensor-core chain.  rhs / psi are
@@ -1509,14 +1489,8 @@ extern "C" int fvx_dst_solve_f32(fvx_dst_plan* p, const float* rhs, long long rh
   if (batch < 1 || batch > p->batch_max) return FVX_ERR_SHAPE;
   cudaStream_t st = fvx_stream(stream);
   long long n = (long long)batch * p->ny * p->nx;
-  if (!p->split_ok) {  // sizes the TMA tiles cannot address: FP64 SIMT chain, FP32 output
-    if (fvx_launch_pdl(copy_in_f64_kernel<float>, dim3(copy_rows_grid((long long)batch * p->ny)), dim3(256), 0, st,
-                       rhs, rhs_bstride, rhs_ld, p->ny, p->nx, batch, p->V1) != cudaSuccess)
-      return FVX_ERR_CUDA;
-    int rc0 = fvx_cuda_status();
-    if (rc0) return rc0;
-    return chain_f64(p, batch, EPI_F32, psi, psi_bstride, psi_ld, st);
-  }
+  if (!p->split_ok)  // sizes the TMA tiles cannot address: FP64 chain, FP32 output
+    return chain_f64(p, batch, rhs, rhs_bstride, rhs_ld, true, psi, psi_bstride, psi_ld, st);
   split_input_kernel<float><<<grid1d(n), 256, 0, st>>>(rhs, rhs_bstride, rhs_ld, p->ny, p->nx, batch, p->W1h,
                                                         p->W1l, 1.0, p->sym ? 1 : 0);
   int rc = fvx_cuda_status();
@@ -1564,7 +1538,8 @@ extern "C" int fvx_dst_solve_presplit_f64(fvx_dst_plan* p, double* psi, long lon
                                           int batch, void* stream) {
   if (!p || !psi || !p->V1) return FVX_ERR_ARG;
   if (batch < 1 || batch > p->batch_max) return FVX_ERR_SHAPE;
-  return chain_f64(p, batch, EPI_F64, psi, psi_bstride, psi_ld, fvx_stream(stream));
+  return chain_f64(p, batch, (const double*)p->V1, (long long)p->ny * p->nx, p->nx, false, psi, psi_bstride, psi_ld,
+                   fvx_stream(stream));
 }
 
 // The FP64 chain's input workspace: [batch_max][ny][nx] doubles, natural
@@ -1588,7 +1563,7 @@ extern "C" int fvx_dst_workspace(fvx_dst_plan* p, void** w1_hi, void** w1_lo) {
   return p->split_ok ? FVX_OK : FVX_ERR_SHAPE;
 }
 
-// FP64 solve.  method 0: FP64 SIMT chain (one pass).  method 1: split-BF16
+// FP64 solve.  method 0: FP64 chain (one pass, dst_f64.cuh).  method 1: split-BF16
 // chain + iterative refinement on the FP64 residual until the normwise
 // backward error ||r|| / (||A|| ||psi|| + ||f||) <= tol (||A|| the 2-norm
 // bound 8/h^2 + lambda) or max_iter passes.  info (host, may be null):
@@ -1604,11 +1579,7 @@ extern "C" int fvx_dst_solve_f64(fvx_dst_plan* p, const double* rhs, long long r
   int rc;
   if (method == 0 || !p->split_ok) {
     if (!p->V1) return FVX_ERR_ARG;
-    if (fvx_launch_pdl(copy_in_f64_kernel<double>, dim3(copy_rows_grid((long long)batch * ny)), dim3(256), 0, st,
-                       rhs, rhs_bstride, rhs_ld, ny, nx, batch, p->V1) != cudaSuccess)
-      return FVX_ERR_CUDA;
-    if ((rc = fvx_cuda_status())) return rc;
-    rc = chain_f64(p, batch, EPI_F64, psi, psi_bstride, psi_ld, st);
+    rc = chain_f64(p, batch, rhs, rhs_bstride, rhs_ld, false, psi, psi_bstride, psi_ld, st);
     if (info) { info[0] = 1; info[1] = -1; info[2] = -1; }
     return rc;
   }
@@ -1804,7 +1775,7 @@ extern "C" int fvx_dst_solve_noalloc_f32(const float* rhs, long long rhs_ld, flo
     Epi e;
     e.mode = mode; e.rows_per_batch = R; e.m_total = M; e.n_cols = N; e.out0 = o0; e.out1 = o1;
     e.batch_stride = bs; e.ld = ld; e.off_n = 0; e.off_r = 0; e.alpha = alpha;
-    e.inv_eig = eig ? inv : nullptr; e.inv_eig64 = nullptr; e.n_eig = 1; e.err = err;
+    e.inv_eig = eig ? inv : nullptr; e.n_eig = 1; e.err = err;
     return e;
   };
   const double c = 4.0 / ((double)(ny + 1) * (double)(nx + 1));

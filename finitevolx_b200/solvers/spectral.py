@@ -14,7 +14,7 @@ same linear map as the FFT solve on real data.
 
 * float32 input: 3xBF16-split tcgen05 GEMM chain, FP32 accumulation
   (relative error ~1e-5 of the FP64 answer);
-* float64 input: the FP64 SIMT chain (``method="fp64"``, default) or the
+* float64 input: the FP64 chain (``method="fp64"``, default) or the
   split chain with FP64 iterative refinement (``method="refine"``) to a
   normwise backward error ``tol``.
 ``lambda_`` may be a scalar or one value per layer (shape [nl], matching

@@ -200,7 +200,7 @@ int fvx_dst_plan_inject_stall(fvx_dst_plan* plan, int on);
  * FP64 chain with FP32 output).  Element (b,y,x) at ptr[b*bstride + y*ld + x]. */
 int fvx_dst_solve_f32(fvx_dst_plan* plan, const float* rhs, long long rhs_bstride, long long rhs_ld, float* psi,
                       long long psi_bstride, long long psi_ld, int batch, void* stream);
-/* FP64: method 0 = FP64 SIMT chain; 1 = split chain + FP64 iterative
+/* FP64: method 0 = FP64 chain; 1 = split chain + FP64 iterative
  * refinement to normwise backward error <= tol (info: passes, backward
  * error, ||r||/||f||; returns 5 if max_iter passes do not reach tol). */
 int fvx_dst_solve_f64(fvx_dst_plan* plan, const double* rhs, long long rhs_bstride, long long rhs_ld, double* psi,
