@@ -24,6 +24,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <cstdio>
@@ -811,29 +812,31 @@ gemm_sym_pair_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_const
   }
 }
 
+#include "dst_fold.cuh"
+
 // ---- input split / copy / residual kernels ---------------------------------
-// perm: store x at its de-interleaved position (the even/odd product's
-// operand layout).
+// half > 0: de-interleaved rows (even x first, odd x from element half on,
+// the folded products' operand layout); pitch: elements per output row.
 template <typename T>
 __global__ void split_input_kernel(const T* __restrict__ in, long long bstride, long long ld, int ny, int nx,
-                                   int batch, bf16* __restrict__ hi, bf16* __restrict__ lo, double scale,
-                                   int perm = 0) {
+                                   int batch, bf16* __restrict__ hi, bf16* __restrict__ lo, int pitch,
+                                   int half) {
   // rows of the [batch][ny][nx] input over the grid, (even, odd) pairs of a
-  // row over the threads: no 64-bit divisions, and with perm the two halves
+  // row over the threads: no 64-bit divisions, and the two halves
   // of the de-interleaved row are written by consecutive threads
-  const int rows = batch * ny, half = (nx + 1) >> 1;
+  const int rows = batch * ny, pairs = (nx + 1) >> 1;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const int b = r / ny, y = r - b * ny;
     const T* src = in + (long long)b * bstride + (long long)y * ld;
-    const long long o = (long long)r * nx;
-    for (int p = threadIdx.x; p < half; p += blockDim.x) {
+    const long long o = (long long)r * pitch;
+    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int x = 2 * p + e;
         if (x >= nx) break;
-        const float v = (float)((double)src[x] * scale);
+        const float v = (float)src[x];
         const bf16 h = __float2bfloat16_rn(v);
-        const long long d = o + (perm ? (e ? (nx >> 1) + p : p) : x);
+        const long long d = o + (half ? (e ? half + p : p) : x);
         hi[d] = h;
         lo[d] = __float2bfloat16_rn(v - __bfloat162float(h));
       }
@@ -877,14 +880,14 @@ DEV double warp_sum(double v) {
 }
 
 // r = f - (lap - lambda) psi (5-point, zero outside), FP64; writes r split
-// into bf16 hi/lo (the next correction's GEMM operand, scaled by 1/rscale)
+// into bf16 hi/lo (the next correction's de-interleaved GEMM operand)
 // and accumulates sum r^2, sum f^2, sum psi^2, sum |A|^2-weighted norm parts
 // into norms[0..3] with warp-shuffle reductions.
 template <typename T, typename PT>
 __global__ void residual_kernel(const T* __restrict__ f, long long fb, long long fld, const PT* __restrict__ psi,
                                 long long pb, long long pld, int ny, int nx, int batch, double dx, double dy,
                                 const double* __restrict__ lam, int nlam, bf16* __restrict__ hi,
-                                bf16* __restrict__ lo, double* norms, int perm) {
+                                bf16* __restrict__ lo, double* norms, int pitch, int half) {
   // a row (b, y) per block iteration, its x over the threads: no 64-bit
   // index divisions
   double s_r = 0, s_f = 0, s_p = 0;
@@ -895,7 +898,7 @@ __global__ void residual_kernel(const T* __restrict__ f, long long fb, long long
     const double lb = lam[b % nlam];
     const PT* P = psi + b * pb + (long long)y * pld;
     const T* F = f + b * fb + (long long)y * fld;
-    const long long o0 = (long long)row * nx;
+    const long long o0 = (long long)row * pitch;
     for (int x = threadIdx.x; x < nx; x += blockDim.x) {
       const PT* Px = P + x;
       const double c = (double)Px[0];
@@ -906,7 +909,7 @@ __global__ void residual_kernel(const T* __restrict__ f, long long fb, long long
       const double r = fv - (lap - lb * c);
       const float rv = (float)r;
       const bf16 h = __float2bfloat16_rn(rv);
-      const long long o = o0 + (perm ? deinterleave(x, nx) : x);
+      const long long o = o0 + ((x & 1) ? half : 0) + (x >> 1);
       hi[o] = h;
       lo[o] = __float2bfloat16_rn(rv - __bfloat162float(h));
       s_r += r * r;
@@ -943,13 +946,14 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 // 2-D bf16 tensor map over [outer][inner] (inner contiguous), box
 // {BK, box_outer}, 128-byte swizzle, zero fill out of bounds.
 static bool make_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint32_t box_outer,
-                     uint32_t box_inner = BK) {
+                     uint32_t box_inner = BK, uint64_t pitch = 0) {
   auto enc = encode_fn();
   if (!enc) return false;
-  if (((uintptr_t)base & 15) != 0 || (inner * 2) % 16 != 0) return false;
+  if (!pitch) pitch = inner;
+  if (((uintptr_t)base & 15) != 0 || (pitch * 2) % 16 != 0) return false;
   if (box_inner != 64 && box_inner != 32) return false;
   cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {inner * 2};
+  cuuint64_t strides[1] = {pitch * 2};
   cuuint32_t box[2] = {box_inner, box_outer};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
@@ -1061,6 +1065,41 @@ static int gemm_sym(const bf16* Xh, const bf16* Xl, int M, int K, const bf16* Ph
   return fvx_cuda_status();
 }
 
+// Folded tables of one axis and direction, hi / lo: [h][half] each for P and Q.
+struct FoldTables {
+  bf16 *Ph = nullptr, *Pl = nullptr, *Qh = nullptr, *Ql = nullptr;
+};
+
+template <int NT>
+static int launch_fold_bf16(const bf16* Xh, const bf16* Xl, int h, int half, const FoldTables& t, const FoldEpi& fe,
+                            cudaStream_t st) {
+  using C = FoldCfg<NT>;
+  static fvx_once_per_device attr;
+  if (fvx_once_on_device(attr, [] { return fvx_set_max_smem(gemm_fold_bf16_kernel<NT>, C::SMEM); }))
+    return FVX_ERR_CUDA;
+  const int M = fe.e.m_total;
+  CUtensorMap aph, apl, aqh, aql, ph, pl, qh, ql;
+  if (!make_map(&aph, Xh, h, M, BM, BK, 2 * half) || !make_map(&apl, Xl, h, M, BM, BK, 2 * half) ||
+      !make_map(&aqh, Xh + half, h, M, BM, BK, 2 * half) || !make_map(&aql, Xl + half, h, M, BM, BK, 2 * half) ||
+      !make_map(&ph, t.Ph, h, h, NT, BK, half) || !make_map(&pl, t.Pl, h, h, NT, BK, half) ||
+      !make_map(&qh, t.Qh, h, h, NT, BK, half) || !make_map(&ql, t.Ql, h, h, NT, BK, half))
+    return FVX_ERR_ARG;
+  const dim3 grid((fe.nh + NT - 1) / NT, (M + BM - 1) / BM);
+  if (grid.y > 65535) return FVX_ERR_SHAPE;
+  if (fvx_launch_pdl(gemm_fold_bf16_kernel<NT>, grid, dim3(C::THREADS), C::SMEM, st, aph, apl, aqh, aql, ph, pl, qh,
+                     ql, h, fe) != cudaSuccess)
+    return FVX_ERR_CUDA;
+  return fvx_cuda_status();
+}
+
+// What the folded product on NT-row tiles costs: rounds of CTAs times the
+// bytes a CTA loads per K element (in rows of 4 bytes) plus its fixed part
+// (set-up, first loads, epilogue) in the same unit.
+static long long fold_cost(int NT, int nh, int M) {
+  const long long ctas = (long long)((nh + NT - 1) / NT) * ((M + BM - 1) / BM);
+  return (ctas + 147) / 148 * (BM + NT + 40);
+}
+
 static int grid1d(long long n) {
   long long b = (n + 255) / 256;
   return (int)(b > 148 * 32 ? 148 * 32 : (b < 1 ? 1 : b));
@@ -1080,18 +1119,19 @@ struct fvx_dst_plan {
   bool split_ok;
   std::vector<double> lam_host;
   double* lam_dev = nullptr;
-  bf16 *Sxh = nullptr, *Sxl = nullptr, *Syh = nullptr, *Syl = nullptr;
-  bool sym = false;  // even/odd products (nx, ny multiples of 256); operands x/y de-interleaved
-  bf16 *xPh = nullptr, *xPl = nullptr, *xQh = nullptr, *xQl = nullptr;  // [nx/2][nx/2]
-  bf16 *yPh = nullptr, *yPl = nullptr, *yQh = nullptr, *yQl = nullptr;  // [ny/2][ny/2]
-  // inverse-transform operands (DCT-II, periodic); the DST-I plan reuses S
-  bf16 *Ixh = nullptr, *Ixl = nullptr, *Iyh = nullptr, *Iyl = nullptr;
-  // FP64 chain: folded tables [hx][kx], [hy][ky] (forward F, inverse I; the
-  // DST-I plan has one) and the eigenvalues along both spectral axes.  kx,
-  // ky: length of a folded axis (2 hx, 2 hy), the table pitch
+  bool sym = false;  // nx, ny multiples of 256: the workspace W1 is public in the products' layout
+  // Folded transforms (dst_f64.cuh): hx, hy table rows (half lengths), kx,
+  // ky folded axis lengths 2 hx, 2 hy (the spectral axes: nx, ny except for
+  // the periodic plan), mirx, miry mirrored-index sums.
   int hx = 0, hy = 0, kx = 0, ky = 0, mirx = 0, miry = 0;
+  // split products: halves of an operand row start at 0 and halfx (halfy),
+  // multiples of 8 elements (TMA's 16 bytes), rows are 2 halfx long
+  int halfx = 0, halfy = 0;
+  FoldTables fx, fy, ix, iy;  // forward, inverse (the DST-I plan's ix, iy are fx, fy)
+  // FP64 chain: tables [hx][kx], [hy][ky] (forward F, inverse I; the DST-I
+  // plan has one) and the eigenvalues along both spectral axes
   double *Fx64 = nullptr, *Fy64 = nullptr, *Ix64 = nullptr, *Iy64 = nullptr, *ex64 = nullptr, *ey64 = nullptr;
-  float* inv32 = nullptr;   // [n_lam][ny][nx]
+  float* inv32 = nullptr;   // [n_lam][ky][kx] 1 / Lambda (DST-I, DCT-II: [ny][nx])
   bf16 *W1h = nullptr, *W1l = nullptr, *W2h = nullptr, *W2l = nullptr;
   double *V1 = nullptr, *V2 = nullptr;  // FP64 chain work
   double* norms = nullptr;              // [4]
@@ -1101,110 +1141,121 @@ struct fvx_dst_plan {
 };
 
 static void dst_free(fvx_dst_plan* p) {
-  void* ptrs[] = {p->lam_dev, p->Sxh, p->Sxl, p->Syh, p->Syl, p->Fx64, p->Fy64, p->inv32,
-                  p->W1h,     p->W1l, p->W2h, p->W2l, p->V1,  p->V2,  p->norms, p->err,
-                  p->xPh,     p->xPl, p->xQh, p->xQl, p->yPh, p->yPl, p->yQh,   p->yQl,
-                  p->Ixh,     p->Ixl, p->Iyh, p->Iyl, p->Ix64, p->Iy64, p->ex64, p->ey64};
+  std::vector<void*> ptrs = {p->lam_dev, p->Fx64, p->Fy64, p->inv32, p->W1h,  p->W1l,  p->W2h,  p->W2l, p->V1,
+                             p->V2,      p->norms, p->err, p->Ix64,  p->Iy64, p->ex64, p->ey64};
+  for (const FoldTables* t : {&p->fx, &p->fy, &p->ix, &p->iy})
+    if (p->kind != FVX_SPECTRAL_DST || t == &p->fx || t == &p->fy) {
+      ptrs.push_back(t->Ph); ptrs.push_back(t->Pl); ptrs.push_back(t->Qh); ptrs.push_back(t->Ql);
+    }
   for (void* q : ptrs)
     if (q) cudaFree(q);
 }
 
-// Transform pairs of one axis of length n: forward T[k][j] (coefficient k
-// of sample j) and inverse Tinv[j][k] (sample j from coefficient k), FP64,
-// row-major, with the 1-D eigenvalues of the 3-point second difference they
-// diagonalise.
-//   DST-I  (Dirichlet, n interior points): T = sin(pi (j+1)(k+1)/(n+1)),
-//          Tinv = T (the 2/(n+1) factors go to the last product's scale),
+// The folded tables of one axis of length n (forms in dst_f64.cuh), FP64
+// [h][k] with zeros past the last column -- even columns belong to P, odd
+// ones to Q -- and the 1-D eigenvalues of the 3-point second difference, in
+// the order of the spectral index.
+//   DST-I  (Dirichlet, n interior points): S[k][j] = sin(pi (j+1)(k+1)/(n+1)),
+//          its own inverse up to the 2/(n+1) factors that go to the last
+//          product's scale; F[r] = row r of S for r < h (both directions),
 //          e_k = -4/h^2 sin^2(pi (k+1) / (2(n+1)))
-//   DCT-II (Neumann, cell-centred): T = cos(pi k (2j+1) / (2n)),
-//          Tinv[j][k] = w_k T[k][j], w_0 = 1/n, w_k = 2/n,
-//          e_k = -4/h^2 sin^2(pi k / (2n))
-//   periodic: the real Hartley basis T = cos(2 pi k j / n) + sin(2 pi k j / n)
-//          (symmetric, T T = n I, and it diagonalises the periodic second
-//          difference because e_k = e_{n-k}), Tinv = T / n,
-//          e_k = -4/h^2 sin^2(pi k / n)
-// Arguments are reduced exactly in integers before the FP64 sin / cos.
-static void transform_pair(int kind, int n, double h, std::vector<double>& T, std::vector<double>& Ti,
-                           std::vector<double>& e) {
-  T.assign((size_t)n * n, 0.0);
-  Ti.assign((size_t)n * n, 0.0);
-  e.assign(n, 0.0);
-  for (int k = 0; k < n; ++k) {
-    double sarg;
-    if (kind == FVX_SPECTRAL_DST) sarg = M_PI * (k + 1) / (2.0 * (n + 1));
-    else if (kind == FVX_SPECTRAL_DCT) sarg = M_PI * k / (2.0 * n);
-    else sarg = M_PI * k / (double)n;
-    const double sv = std::sin(sarg);
-    e[k] = -4.0 / (h * h) * sv * sv;
-    for (int j = 0; j < n; ++j) {
-      double t;
-      if (kind == FVX_SPECTRAL_DST) {
-        const long long q = ((long long)(j + 1) * (k + 1)) % (2LL * (n + 1));
-        t = std::sin(M_PI * (double)q / (double)(n + 1));
-      } else if (kind == FVX_SPECTRAL_DCT) {
-        const long long q = ((long long)k * (2 * j + 1)) % (4LL * n);
-        t = std::cos(M_PI * (double)q / (2.0 * n));
-      } else {
-        const long long q = ((long long)k * j) % (long long)n;
-        const double a = 2.0 * M_PI * (double)q / (double)n;
-        t = std::cos(a) + std::sin(a);
-      }
-      T[(size_t)k * n + j] = t;
-      double w = 1.0;
-      if (kind == FVX_SPECTRAL_DCT) w = (k == 0 ? 1.0 : 2.0) / n;
-      else if (kind == FVX_SPECTRAL_PERIODIC) w = 1.0 / n;
-      Ti[(size_t)j * n + k] = w * t;
-    }
-  }
-}
-
-// The folded FP64 tables of one axis (forms in dst_f64.cuh), [h][k] with
-// zeros past the last column, and its eigenvalues in the order of the
-// spectral index the forward product writes.
-//   DST-I: row n of S for n < h; F serves both directions.
-//   DCT-II: F[n] = coefficients 2n (even columns) and 2n + 1 (odd columns)
-//          of sample j in column pair j; I[n] = row n of Tinv.
-//   periodic: cosine coefficients in the even columns, sine in the odd ones;
-//          the inverse's weights are 1/n for k = 0 and k = n/2, else 2/n.
-static void upload_folded(int kind, int n, int h, int k, const std::vector<double>& T, const std::vector<double>& Ti,
-                          const std::vector<double>& e, double* F, double* I, double* ed) {
-  std::vector<double> f((size_t)h * k, 0.0), b, es(k, 0.0);
+//   DCT-II (Neumann, cell-centred): T[k][j] = cos(pi k (2j+1) / (2n)) and
+//          Tinv[j][k] = w_k T[k][j], w_0 = 1/n, w_k = 2/n; F[r] holds the
+//          coefficients 2r (even columns) and 2r + 1 (odd) of sample j in
+//          column pair j, I[r] = row r of Tinv, e_k = -4/h^2 sin^2(pi k / (2n))
+//   periodic: cosine coefficients in the even columns, sine in the odd ones
+//          (the cas transform of real data by parity), inverse weights 1/n
+//          for k = 0 and k = n/2, else 2/n, e_k = -4/h^2 sin^2(pi k / n)
+// Arguments are reduced exactly in integers; every value is one of the 2n or
+// 4n tabulated FP64 sines.
+static void folded_tables(int kind, int n, double d, int h, int k, std::vector<double>& F, std::vector<double>& I,
+                          std::vector<double>& e) {
+  F.assign((size_t)h * k, 0.0);
+  I.clear();
+  e.assign(k, 0.0);
+  auto eig = [&](double arg) {
+    const double sv = std::sin(arg);
+    return -4.0 / (d * d) * sv * sv;
+  };
   if (kind == FVX_SPECTRAL_DST) {
-    for (int r = 0; r < h; ++r)
-      for (int j = 0; j < n; ++j) f[(size_t)r * k + j] = T[(size_t)r * n + j];
-    for (int j = 0; j < n; ++j) es[j] = e[j];
-  } else if (kind == FVX_SPECTRAL_DCT) {
-    b.assign((size_t)h * k, 0.0);
+    std::vector<double> s(2 * (size_t)(n + 1));
+    for (size_t q = 0; q < s.size(); ++q) s[q] = std::sin(M_PI * (double)q / (double)(n + 1));
+    for (int r = 0; r < h; ++r) {
+      size_t q = 0;
+      for (int j = 0; j < n; ++j) {
+        q += r + 1;  // (j + 1)(r + 1) mod 2 (n + 1)
+        if (q >= s.size()) q -= s.size();
+        F[(size_t)r * k + j] = s[q];
+      }
+    }
+    for (int j = 0; j < n; ++j) e[j] = eig(M_PI * (j + 1) / (2.0 * (n + 1)));
+    return;
+  }
+  I.assign((size_t)h * k, 0.0);
+  if (kind == FVX_SPECTRAL_DCT) {
+    std::vector<double> c(4 * (size_t)n);
+    for (size_t q = 0; q < c.size(); ++q) c[q] = std::cos(M_PI * (double)q / (2.0 * n));
+    auto T = [&](int kk, int j) { return c[(size_t)(((long long)kk * (2 * j + 1)) % (4LL * n))]; };
     for (int r = 0; r < h; ++r) {
       for (int j = 0; j < h; ++j) {
-        f[(size_t)r * k + 2 * j] = T[(size_t)(2 * r) * n + j];
-        if (2 * r + 1 < n) f[(size_t)r * k + 2 * j + 1] = T[(size_t)(2 * r + 1) * n + j];
+        F[(size_t)r * k + 2 * j] = T(2 * r, j);
+        if (2 * r + 1 < n) F[(size_t)r * k + 2 * j + 1] = T(2 * r + 1, j);
       }
-      for (int j = 0; j < n; ++j) b[(size_t)r * k + j] = Ti[(size_t)r * n + j];
+      for (int j = 0; j < n; ++j) I[(size_t)r * k + j] = (j == 0 ? 1.0 : 2.0) / n * T(j, r);
     }
-    for (int j = 0; j < n; ++j) es[j] = e[j];
-  } else {
-    b.assign((size_t)h * k, 0.0);
-    std::vector<double> cs(n), sn(n);
-    for (int q = 0; q < n; ++q) {
-      const double t = 2.0 * M_PI * (double)q / (double)n;
-      cs[q] = std::cos(t);
-      sn[q] = std::sin(t);
-    }
-    for (int r = 0; r < h; ++r)
-      for (int j = 0; j < h; ++j) {
-        const int q = (int)(((long long)r * j) % n);
-        const double w = (j == 0 || 2 * j == n ? 1.0 : 2.0) / n;
-        f[(size_t)r * k + 2 * j] = cs[q];
-        f[(size_t)r * k + 2 * j + 1] = sn[q];
-        b[(size_t)r * k + 2 * j] = w * cs[q];
-        b[(size_t)r * k + 2 * j + 1] = w * sn[q];
-      }
-    for (int j = 0; j < h; ++j) es[2 * j] = es[2 * j + 1] = e[j < n ? j : 0];
+    for (int j = 0; j < n; ++j) e[j] = eig(M_PI * j / (2.0 * n));
+    return;
   }
-  cudaMemcpy(F, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice);
-  if (I) cudaMemcpy(I, b.data(), sizeof(double) * b.size(), cudaMemcpyHostToDevice);
-  cudaMemcpy(ed, es.data(), sizeof(double) * es.size(), cudaMemcpyHostToDevice);
+  std::vector<double> cs(n), sn(n);
+  for (int q = 0; q < n; ++q) {
+    const double t = 2.0 * M_PI * (double)q / (double)n;
+    cs[q] = std::cos(t);
+    sn[q] = std::sin(t);
+  }
+  for (int r = 0; r < h; ++r)
+    for (int j = 0; j < h; ++j) {
+      const int q = (int)(((long long)r * j) % n);
+      const double w = (j == 0 || 2 * j == n ? 1.0 : 2.0) / n;
+      F[(size_t)r * k + 2 * j] = cs[q];
+      F[(size_t)r * k + 2 * j + 1] = sn[q];
+      I[(size_t)r * k + 2 * j] = w * cs[q];
+      I[(size_t)r * k + 2 * j + 1] = w * sn[q];
+    }
+  for (int j = 0; j < h; ++j) e[2 * j] = e[2 * j + 1] = eig(M_PI * j / (double)n);
+}
+
+static bool upload(double* dev, const std::vector<double>& v) {
+  return cudaMemcpy(dev, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+}
+// Even columns of a folded table to P, odd ones to Q, split into bf16 hi / lo
+// rows of `half` elements.
+static bool upload_split(const FoldTables& t, const std::vector<double>& F, int h, int k, int half) {
+  std::vector<bf16> b[4];
+  for (auto& v : b) v.assign((size_t)h * half, __float2bfloat16_rn(0.f));
+  for (int r = 0; r < h; ++r)
+    for (int j = 0; j < h; ++j)
+      for (int q = 0; q < 2; ++q) {
+        const double x = F[(size_t)r * k + 2 * j + q];
+        const bf16 hi = __float2bfloat16_rn((float)x);
+        b[2 * q][(size_t)r * half + j] = hi;
+        b[2 * q + 1][(size_t)r * half + j] = __float2bfloat16_rn((float)(x - (double)__bfloat162float(hi)));
+      }
+  bf16* dev[4] = {t.Ph, t.Pl, t.Qh, t.Ql};
+  for (int q = 0; q < 4; ++q)
+    if (cudaMemcpy(dev[q], b[q].data(), sizeof(bf16) * b[q].size(), cudaMemcpyHostToDevice) != cudaSuccess) return false;
+  return true;
+}
+
+// 1 / ((ey[j] + ex[i]) - lambda) rounded to FP32, 0 for a zero eigenvalue
+// (the null mode of a Neumann / periodic Poisson problem: the zero-mean
+// solution).
+__global__ void inv_eig_kernel(const double* __restrict__ ey, const double* __restrict__ ex, int ky, int kx,
+                               const double* __restrict__ lam, float* __restrict__ out) {
+  for (int row = blockIdx.x; row < ky; row += gridDim.x)
+    for (int i = threadIdx.x; i < kx; i += blockDim.x) {
+      const double d = (ey[row] + ex[i]) - lam[blockIdx.y];
+      out[((long long)blockIdx.y * ky + row) * kx + i] = d == 0.0 ? 0.f : (float)(1.0 / d);
+    }
 }
 
 extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, double dy, int batch_max,
@@ -1228,116 +1279,64 @@ extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, dou
   p->split_ok = (nx % 8 == 0) && (ny % 8 == 0);
   p->sym = kind == FVX_SPECTRAL_DST && p->split_ok && nx % (2 * SBN) == 0 && ny % (2 * SBN) == 0;
   p->cfin = kind == FVX_SPECTRAL_DST ? 4.0 / ((double)(ny + 1) * (double)(nx + 1)) : 1.0;
-  const bool dst = kind == FVX_SPECTRAL_DST;
-  const size_t plane = (size_t)ny * nx, work = plane * batch_max;
-  // half lengths and mirror indices of the folded FP64 products (dst_f64.cuh)
-  const bool per = kind == FVX_SPECTRAL_PERIODIC;
+  const bool dst = kind == FVX_SPECTRAL_DST, per = kind == FVX_SPECTRAL_PERIODIC;
   p->hx = per ? nx / 2 + 1 : (nx + 1) / 2;
   p->hy = per ? ny / 2 + 1 : (ny + 1) / 2;
   p->kx = 2 * p->hx; p->ky = 2 * p->hy;
   p->mirx = per ? nx : nx - 1; p->miry = per ? ny : ny - 1;
+  p->halfx = (p->hx + 7) / 8 * 8; p->halfy = (p->hy + 7) / 8 * 8;
   const bool want64 = want_fp64 || !p->split_ok;
   bool ok = true;
   auto A = [&](void** q, size_t bytes) { if (ok && cudaMalloc(q, bytes) != cudaSuccess) ok = false; };
   A((void**)&p->lam_dev, sizeof(double) * n_lambda);
-  A((void**)&p->inv32, sizeof(float) * plane * n_lambda);
   A((void**)&p->norms, sizeof(double) * 4);
   A((void**)&p->err, sizeof(int));
+  A((void**)&p->ex64, sizeof(double) * p->kx); A((void**)&p->ey64, sizeof(double) * p->ky);
   if (p->split_ok) {
-    A((void**)&p->Sxh, sizeof(bf16) * nx * nx); A((void**)&p->Sxl, sizeof(bf16) * nx * nx);
-    A((void**)&p->Syh, sizeof(bf16) * ny * ny); A((void**)&p->Syl, sizeof(bf16) * ny * ny);
-    if (!dst) {
-      A((void**)&p->Ixh, sizeof(bf16) * nx * nx); A((void**)&p->Ixl, sizeof(bf16) * nx * nx);
-      A((void**)&p->Iyh, sizeof(bf16) * ny * ny); A((void**)&p->Iyl, sizeof(bf16) * ny * ny);
-    }
+    const size_t work = (size_t)batch_max * std::max((size_t)p->ky * 2 * p->halfx, (size_t)p->kx * 2 * p->halfy);
+    A((void**)&p->inv32, sizeof(float) * p->ky * p->kx * n_lambda);
     A((void**)&p->W1h, sizeof(bf16) * work); A((void**)&p->W1l, sizeof(bf16) * work);
     A((void**)&p->W2h, sizeof(bf16) * work); A((void**)&p->W2l, sizeof(bf16) * work);
-  }
-  if (p->sym) {
-    const size_t hx = (size_t)(nx / 2) * (nx / 2), hy = (size_t)(ny / 2) * (ny / 2);
-    A((void**)&p->xPh, sizeof(bf16) * hx); A((void**)&p->xPl, sizeof(bf16) * hx);
-    A((void**)&p->xQh, sizeof(bf16) * hx); A((void**)&p->xQl, sizeof(bf16) * hx);
-    A((void**)&p->yPh, sizeof(bf16) * hy); A((void**)&p->yPl, sizeof(bf16) * hy);
-    A((void**)&p->yQh, sizeof(bf16) * hy); A((void**)&p->yQl, sizeof(bf16) * hy);
+    auto tables = [&](FoldTables& t, int h, int half) {
+      const size_t bytes = sizeof(bf16) * (size_t)h * half;
+      A((void**)&t.Ph, bytes); A((void**)&t.Pl, bytes); A((void**)&t.Qh, bytes); A((void**)&t.Ql, bytes);
+    };
+    tables(p->fx, p->hx, p->halfx); tables(p->fy, p->hy, p->halfy);
+    if (dst) { p->ix = p->fx; p->iy = p->fy; }
+    else { tables(p->ix, p->hx, p->halfx); tables(p->iy, p->hy, p->halfy); }
   }
   if (want64) {
-    const size_t work64 = (size_t)p->kx * p->ky * batch_max;  // kx >= nx, ky >= ny
+    const size_t work = (size_t)p->kx * p->ky * batch_max;  // kx >= nx, ky >= ny
     const size_t tx = (size_t)p->hx * p->kx, ty = (size_t)p->hy * p->ky;
-    A((void**)&p->V1, sizeof(double) * work64);
-    A((void**)&p->V2, sizeof(double) * work64);
+    A((void**)&p->V1, sizeof(double) * work);
+    A((void**)&p->V2, sizeof(double) * work);
     A((void**)&p->Fx64, sizeof(double) * tx); A((void**)&p->Fy64, sizeof(double) * ty);
     if (!dst) { A((void**)&p->Ix64, sizeof(double) * tx); A((void**)&p->Iy64, sizeof(double) * ty); }
-    A((void**)&p->ex64, sizeof(double) * p->kx); A((void**)&p->ey64, sizeof(double) * p->ky);
   }
   if (!ok) { dst_free(p); delete p; return FVX_ERR_CUDA; }
-  // host-side tables in FP64; the tensor-core products read B as [out][in]
-  // (T itself for the forward, Tinv for the inverse)
-  std::vector<double> Tx, Tix, ex, Ty, Tiy, ey;
-  transform_pair(kind, nx, dx, Tx, Tix, ex);
-  transform_pair(kind, ny, dy, Ty, Tiy, ey);
-  const std::vector<double>&Sx = Tx, &Sy = Ty;  // split operands [out][in]
-  std::vector<float> inv32(plane * n_lambda);
-  for (int l = 0; l < n_lambda; ++l)
-    for (int j = 0; j < ny; ++j)
-      for (int i = 0; i < nx; ++i) {
-        // the null mode (Neumann / periodic Poisson) gets 0: the zero-mean solution
-        const double d = (ey[j] + ex[i]) - lambdas[l];
-        inv32[(size_t)l * plane + (size_t)j * nx + i] = (float)(d == 0.0 ? 0.0 : 1.0 / d);
-      }
-  cudaMemcpy(p->lam_dev, lambdas, sizeof(double) * n_lambda, cudaMemcpyHostToDevice);
-  if (want64) {
-    upload_folded(kind, nx, p->hx, p->kx, Tx, Tix, ex, p->Fx64, p->Ix64, p->ex64);
-    upload_folded(kind, ny, p->hy, p->ky, Ty, Tiy, ey, p->Fy64, p->Iy64, p->ey64);
+  std::vector<double> F, I, e;
+  folded_tables(kind, nx, dx, p->hx, p->kx, F, I, e);
+  ok = upload(p->ex64, e);
+  if (want64) ok = ok && upload(p->Fx64, F) && (dst || upload(p->Ix64, I));
+  if (p->split_ok) ok = ok && upload_split(p->fx, F, p->hx, p->kx, p->halfx) &&
+                        (dst || upload_split(p->ix, I, p->hx, p->kx, p->halfx));
+  folded_tables(kind, ny, dy, p->hy, p->ky, F, I, e);
+  ok = ok && upload(p->ey64, e);
+  if (want64) ok = ok && upload(p->Fy64, F) && (dst || upload(p->Iy64, I));
+  if (p->split_ok) ok = ok && upload_split(p->fy, F, p->hy, p->ky, p->halfy) &&
+                        (dst || upload_split(p->iy, I, p->hy, p->ky, p->halfy));
+  ok = ok && cudaMemcpy(p->lam_dev, lambdas, sizeof(double) * n_lambda, cudaMemcpyHostToDevice) == cudaSuccess &&
+       cudaMemset(p->err, 0, sizeof(int)) == cudaSuccess;
+  for (int l = 0; ok && p->split_ok && l < n_lambda; l += 65535) {
+    const int nl = std::min(65535, n_lambda - l);
+    inv_eig_kernel<<<dim3(std::min(p->ky, 148 * 8), nl), 256>>>(p->ey64, p->ex64, p->ky, p->kx, p->lam_dev + l,
+                                                               p->inv32 + (size_t)l * p->ky * p->kx);
   }
-  cudaMemcpy(p->inv32, inv32.data(), sizeof(float) * inv32.size(), cudaMemcpyHostToDevice);
-  if (p->split_ok) {
-    auto split = [](const std::vector<double>& S, std::vector<bf16>& h, std::vector<bf16>& l) {
-      h.resize(S.size());
-      l.resize(S.size());
-      for (size_t k = 0; k < S.size(); ++k) {
-        h[k] = __float2bfloat16_rn((float)S[k]);
-        l[k] = __float2bfloat16_rn((float)(S[k] - (double)__bfloat162float(h[k])));
-      }
-    };
-    std::vector<bf16> h, l;
-    split(Sx, h, l);
-    cudaMemcpy(p->Sxh, h.data(), sizeof(bf16) * h.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(p->Sxl, l.data(), sizeof(bf16) * l.size(), cudaMemcpyHostToDevice);
-    split(Sy, h, l);
-    cudaMemcpy(p->Syh, h.data(), sizeof(bf16) * h.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(p->Syl, l.data(), sizeof(bf16) * l.size(), cudaMemcpyHostToDevice);
-    if (!dst) {
-      split(Tix, h, l);
-      cudaMemcpy(p->Ixh, h.data(), sizeof(bf16) * h.size(), cudaMemcpyHostToDevice);
-      cudaMemcpy(p->Ixl, l.data(), sizeof(bf16) * l.size(), cudaMemcpyHostToDevice);
-      split(Tiy, h, l);
-      cudaMemcpy(p->Iyh, h.data(), sizeof(bf16) * h.size(), cudaMemcpyHostToDevice);
-      cudaMemcpy(p->Iyl, l.data(), sizeof(bf16) * l.size(), cudaMemcpyHostToDevice);
-    }
-    if (p->sym) {
-      // B_P[k][j'] = S[2j'][k], B_Q[k][j'] = S[2j'+1][k] for k, j' < n/2
-      auto halves = [&](const std::vector<double>& S, int n, bf16* Ph, bf16* Pl, bf16* Qh, bf16* Ql) {
-        const int hn = n / 2;
-        std::vector<double> P((size_t)hn * hn), Q((size_t)hn * hn);
-        for (int k = 0; k < hn; ++k)
-          for (int j = 0; j < hn; ++j) {
-            P[(size_t)k * hn + j] = S[(size_t)(2 * j) * n + k];
-            Q[(size_t)k * hn + j] = S[(size_t)(2 * j + 1) * n + k];
-          }
-        std::vector<bf16> hh, ll;
-        split(P, hh, ll);
-        cudaMemcpy(Ph, hh.data(), sizeof(bf16) * hh.size(), cudaMemcpyHostToDevice);
-        cudaMemcpy(Pl, ll.data(), sizeof(bf16) * ll.size(), cudaMemcpyHostToDevice);
-        split(Q, hh, ll);
-        cudaMemcpy(Qh, hh.data(), sizeof(bf16) * hh.size(), cudaMemcpyHostToDevice);
-        cudaMemcpy(Ql, ll.data(), sizeof(bf16) * ll.size(), cudaMemcpyHostToDevice);
-      };
-      halves(Sx, nx, p->xPh, p->xPl, p->xQh, p->xQl);
-      halves(Sy, ny, p->yPh, p->yPl, p->yQh, p->yQl);
-    }
+  if (!ok || cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+    dst_free(p);
+    delete p;
+    return FVX_ERR_CUDA;
   }
-  cudaMemset(p->err, 0, sizeof(int));
-  if (cudaDeviceSynchronize() != cudaSuccess) { dst_free(p); delete p; return FVX_ERR_CUDA; }
   *out = p;
   return FVX_OK;
 }
@@ -1394,42 +1393,98 @@ static Epi make_epi(fvx_dst_plan* p, int mode, int R, int M, int N, void* o0, vo
   return e;
 }
 
-// The split-BF16 chain on operands already split into W1 ([B][ny][nx]).
-// Output: mode EPI_F32 / EPI_F64 / EPI_F64_ACC into ``out`` with batch
-// stride ``ob`` and row pitch ``old`` (interior [B][ny][nx] view).
+// One split product of the chain, X -> the operand or output ep describes.
+// Tiles: the folded kernel's NT = 32, 64 or 128 table rows by cost, and in
+// place of NT = 128 the even/odd kernel (the same product on sizes that are
+// multiples of 256, with its staged TMA stores) where the plan has it.  Two
+// fields of 512^2 have 16 of the even/odd kernel's tiles, 64 of the 32-row
+// ones: 23.3 -> 15.0 us per product (ncu); five, 15.1 -> 12.3 on 64 rows; one
+// of 1024^2, 23.9 -> 18.5 on 32.  With more rows the larger tile loads less.
+static int split_product(fvx_dst_plan* p, const bf16* Xh, const bf16* Xl, bool along_x, bool inverse, const Epi& ep,
+                         cudaStream_t st) {
+  const int h = along_x ? p->hx : p->hy, half = along_x ? p->halfx : p->halfy;
+  const FoldTables& t = along_x ? (inverse ? p->ix : p->fx) : (inverse ? p->iy : p->fy);
+  const int M = ep.m_total;
+  const long long c32 = fold_cost(32, h, M), c64 = fold_cost(64, h, M), c128 = fold_cost(128, h, M);
+  if (p->sym && (g_sym_kernel != 0 || c128 <= std::min(c32, c64)))
+    return gemm_sym(Xh, Xl, M, 2 * h, t.Ph, t.Pl, t.Qh, t.Ql, ep, st);
+  FoldEpi fe;
+  fe.e = ep;
+  fe.nh = h;
+  fe.mir = p->kind == FVX_SPECTRAL_DST || inverse ? (along_x ? p->mirx : p->miry) : -1;
+  fe.half_out = ep.perm_r ? (along_x ? p->halfy : p->halfx) : 0;
+  if (c32 <= c64 && c32 <= c128) return launch_fold_bf16<32>(Xh, Xl, h, half, t, fe, st);
+  if (c64 <= c128) return launch_fold_bf16<64>(Xh, Xl, h, half, t, fe, st);
+  return launch_fold_bf16<128>(Xh, Xl, h, half, t, fe, st);
+}
+
+// Epilogue of the chain's product k = 0 .. 3 writing an operand (the next
+// product's, de-interleaved): along x, along y (divided by Lambda), along x
+// back.
+static Epi operand_epi(fvx_dst_plan* p, int k, int B, bf16* oh, bf16* ol) {
+  const bool along_x = k != 1;
+  const int R = along_x ? p->ky : p->kx;             // rows per batch
+  const int N = k == 2 ? p->nx : (along_x ? p->kx : p->ky);  // output rows
+  const int pitch = 2 * (along_x ? p->halfy : p->halfx);
+  Epi e = make_epi(p, EPI_SPLIT, R, B * R, N, oh, ol, (long long)N * pitch, pitch, 0, 0, 1.0, k == 1);
+  e.perm_r = 1;
+  return e;
+}
+
+// The chain's first operand: the folded layout in W1 for plans whose public
+// workspace has it (sym), else in W2, so that W1 stays the natural-order one.
+static void first_operand(fvx_dst_plan* p, bf16** h, bf16** l) {
+  *h = p->sym ? p->W1h : p->W2h;
+  *l = p->sym ? p->W1l : p->W2l;
+}
+
+// The split-BF16 chain from the first operand ([B][ky][2 halfx]).  Output:
+// mode EPI_F32 / EPI_F32_ACC / EPI_F64_ACC into ``out`` with batch stride
+// ``ob`` and row pitch ``old`` (interior [B][ny][nx] view).
 static int chain_split(fvx_dst_plan* p, int B, int out_mode, void* out, long long ob, long long old,
                        cudaStream_t st) {
-  const int ny = p->ny, nx = p->nx;
-  const double c = p->cfin;
-  const bool dst = p->kind == FVX_SPECTRAL_DST;
-  const bf16 *Ixh = dst ? p->Sxh : p->Ixh, *Ixl = dst ? p->Sxl : p->Ixl;
-  const bf16 *Iyh = dst ? p->Syh : p->Iyh, *Iyl = dst ? p->Syl : p->Iyl;
+  bf16 *ah, *al;
+  first_operand(p, &ah, &al);
+  bf16 *bh = p->sym ? p->W2h : p->W1h, *bl = p->sym ? p->W2l : p->W1l;
   int rc;
-  if (p->sym) {
-    // even/odd products; every intermediate is stored de-interleaved along
-    // the next product's contraction axis, the result in natural order
-    Epi e1 = make_epi(p, EPI_SPLIT, ny, B * ny, nx, p->W2h, p->W2l, (long long)nx * ny, ny, 0, 0, 1.0, false);
-    e1.perm_r = 1;
-    if ((rc = gemm_sym(p->W1h, p->W1l, B * ny, nx, p->xPh, p->xPl, p->xQh, p->xQl, e1, st))) return rc;
-    Epi e2 = make_epi(p, EPI_SPLIT, nx, B * nx, ny, p->W1h, p->W1l, (long long)ny * nx, nx, 0, 0, 1.0, true);
-    e2.perm_r = 1;
-    if ((rc = gemm_sym(p->W2h, p->W2l, B * nx, ny, p->yPh, p->yPl, p->yQh, p->yQl, e2, st))) return rc;
-    if ((rc = gemm_sym(p->W1h, p->W1l, B * ny, nx, p->xPh, p->xPl, p->xQh, p->xQl, e1, st))) return rc;
-    Epi e4 = make_epi(p, out_mode, nx, B * nx, ny, out, nullptr, ob, old, 0, 0, c, false);
-    return gemm_sym(p->W2h, p->W2l, B * nx, ny, p->yPh, p->yPl, p->yQh, p->yQl, e4, st);
+  if ((rc = split_product(p, ah, al, true, false, operand_epi(p, 0, B, bh, bl), st))) return rc;
+  if ((rc = split_product(p, bh, bl, false, false, operand_epi(p, 1, B, ah, al), st))) return rc;
+  if ((rc = split_product(p, ah, al, true, true, operand_epi(p, 2, B, bh, bl), st))) return rc;
+  Epi e4 = make_epi(p, out_mode, p->nx, B * p->nx, p->ny, out, nullptr, ob, old, 0, 0, p->cfin, false);
+  return split_product(p, bh, bl, false, true, e4, st);
+}
+
+// First operand from an interior view (element (b, y, x) at src[b * sbs + y *
+// sld + x]).
+template <typename T>
+static int split_in(fvx_dst_plan* p, int B, const T* src, long long sbs, long long sld, cudaStream_t st) {
+  bf16 *h, *l;
+  first_operand(p, &h, &l);
+  if (p->kind == FVX_SPECTRAL_DST) {
+    split_input_kernel<T><<<grid1d((long long)B * p->ny * p->nx), 256, 0, st>>>(src, sbs, sld, p->ny, p->nx, B, h, l,
+                                                                               2 * p->halfx, p->halfx);
+    return fvx_cuda_status();
   }
-  // 1: (Q S_x)^T -> W2 [B][nx][ny]
-  Epi e1 = make_epi(p, EPI_SPLIT, ny, B * ny, nx, p->W2h, p->W2l, (long long)nx * ny, ny, 0, 0, 1.0, false);
-  if ((rc = gemm_split(p->W1h, p->W1l, B * ny, nx, p->Sxh, p->Sxl, nx, e1, st))) return rc;
-  // 2: (S_y Q S_x) ./ Lambda -> W1 [B][ny][nx]
-  Epi e2 = make_epi(p, EPI_SPLIT, nx, B * nx, ny, p->W1h, p->W1l, (long long)ny * nx, nx, 0, 0, 1.0, true);
-  // inv_eig is indexed [n][r] = [y'][x'] = the [ny][nx] grid
-  if ((rc = gemm_split(p->W2h, p->W2l, B * nx, ny, p->Syh, p->Syl, ny, e2, st))) return rc;
-  // 3: inverse along x -> W2
-  if ((rc = gemm_split(p->W1h, p->W1l, B * ny, nx, Ixh, Ixl, nx, e1, st))) return rc;
-  // 4: inverse along y, scaled -> out [B][ny][nx]
-  Epi e4 = make_epi(p, out_mode, nx, B * nx, ny, out, nullptr, ob, old, 0, 0, c, false);
-  return gemm_split(p->W2h, p->W2l, B * nx, ny, Iyh, Iyl, ny, e4, st);
+  if (fvx_launch_pdl(fold_split_kernel<T, false>, dim3(copy_rows_grid((long long)B * p->hy)), dim3(256), 0, st, src,
+                     nullptr, sbs, sld, p->ny, p->nx, p->hy, p->hx, p->miry, p->mirx, B, 2 * p->halfx, p->halfx, h,
+                     l) != cudaSuccess)
+    return FVX_ERR_CUDA;
+  return fvx_cuda_status();
+}
+
+// First operand from the public natural-order workspace W1 (plans without
+// the folded layout there).
+static int natural_in(fvx_dst_plan* p, int B, cudaStream_t st) {
+  const long long plane = (long long)p->ny * p->nx;
+  cudaError_t e;
+  if (p->kind == FVX_SPECTRAL_DST)
+    e = fvx_launch_pdl(deinterleave_kernel, dim3(copy_rows_grid((long long)B * p->ny)), dim3(128), 0, st, p->W1h,
+                       p->W1l, (long long)B * p->ny, p->nx, 2 * p->halfx, p->halfx, p->W2h, p->W2l);
+  else
+    e = fvx_launch_pdl(fold_split_kernel<bf16, true>, dim3(copy_rows_grid((long long)B * p->hy)), dim3(256), 0, st,
+                       p->W1h, p->W1l, plane, (long long)p->nx, p->ny, p->nx, p->hy, p->hx, p->miry, p->mirx, B,
+                       2 * p->halfx, p->halfx, p->W2h, p->W2l);
+  return e == cudaSuccess ? fvx_cuda_status() : FVX_ERR_CUDA;
 }
 
 // The FP64 chain: folded products (dst_f64.cuh) from the interior view
@@ -1488,12 +1543,9 @@ extern "C" int fvx_dst_solve_f32(fvx_dst_plan* p, const float* rhs, long long rh
   if (!p || !rhs || !psi) return FVX_ERR_ARG;
   if (batch < 1 || batch > p->batch_max) return FVX_ERR_SHAPE;
   cudaStream_t st = fvx_stream(stream);
-  long long n = (long long)batch * p->ny * p->nx;
   if (!p->split_ok)  // sizes the TMA tiles cannot address: FP64 chain, FP32 output
     return chain_f64(p, batch, rhs, rhs_bstride, rhs_ld, true, psi, psi_bstride, psi_ld, st);
-  split_input_kernel<float><<<grid1d(n), 256, 0, st>>>(rhs, rhs_bstride, rhs_ld, p->ny, p->nx, batch, p->W1h,
-                                                        p->W1l, 1.0, p->sym ? 1 : 0);
-  int rc = fvx_cuda_status();
+  const int rc = split_in(p, batch, rhs, rhs_bstride, rhs_ld, st);
   if (rc) return rc;
   return chain_split(p, batch, EPI_F32, psi, psi_bstride, psi_ld, st);
 }
@@ -1504,7 +1556,12 @@ extern "C" int fvx_dst_solve_presplit_f32(fvx_dst_plan* p, float* psi, long long
                                           int batch, void* stream) {
   if (!p || !psi) return FVX_ERR_ARG;
   if (batch < 1 || batch > p->batch_max || !p->split_ok) return FVX_ERR_SHAPE;
-  return chain_split(p, batch, EPI_F32, psi, psi_bstride, psi_ld, fvx_stream(stream));
+  cudaStream_t st = fvx_stream(stream);
+  if (!p->sym) {
+    const int rc = natural_in(p, batch, st);
+    if (rc) return rc;
+  }
+  return chain_split(p, batch, EPI_F32, psi, psi_bstride, psi_ld, st);
 }
 
 // FP64-residual iterative refinement of an FP32 result: ``passes`` times,
@@ -1520,10 +1577,12 @@ extern "C" int fvx_dst_refine_f32(fvx_dst_plan* p, const float* rhs, long long r
   if (batch < 1 || batch > p->batch_max || !p->split_ok) return FVX_ERR_SHAPE;
   if (p->kind != FVX_SPECTRAL_DST) return FVX_ERR_METHOD;
   cudaStream_t st = fvx_stream(stream);
+  bf16 *rh, *rl;
+  first_operand(p, &rh, &rl);
   for (int it = 0; it < passes; ++it) {
     residual_kernel<float, float><<<residual_grid(batch * p->ny), 256, 0, st>>>(rhs, rhs_bstride, rhs_ld, psi, psi_bstride, psi_ld,
                                                               p->ny, p->nx, batch, p->dx, p->dy, p->lam_dev,
-                                                              p->n_lam, p->W1h, p->W1l, nullptr, p->sym ? 1 : 0);
+                                                              p->n_lam, rh, rl, nullptr, 2 * p->halfx, p->halfx);
     int rc = fvx_cuda_status();
     if (rc) return rc;
     if ((rc = chain_split(p, batch, EPI_F32_ACC, psi, psi_bstride, psi_ld, st))) return rc;
@@ -1588,17 +1647,18 @@ extern "C" int fvx_dst_solve_f64(fvx_dst_plan* p, const double* rhs, long long r
   for (double l : p->lam_host) lam_max = fmax(lam_max, fabs(l));
   const double anorm = 4.0 / (p->dx * p->dx) + 4.0 / (p->dy * p->dy) + lam_max;
   zero_f64_kernel<<<grid1d(n), 256, 0, st>>>(psi, psi_bstride, psi_ld, ny, nx, batch);
-  split_input_kernel<double><<<grid1d(n), 256, 0, st>>>(rhs, rhs_bstride, rhs_ld, ny, nx, batch, p->W1h, p->W1l, 1.0,
-                                                         p->sym ? 1 : 0);
   if ((rc = fvx_cuda_status())) return rc;
+  if ((rc = split_in(p, batch, rhs, rhs_bstride, rhs_ld, st))) return rc;
+  bf16 *rh, *rl;
+  first_operand(p, &rh, &rl);
   double be = 1, rr = 1;
   int it = 0;
   for (it = 1; it <= max_iter; ++it) {
     if ((rc = chain_split(p, batch, EPI_F64_ACC, psi, psi_bstride, psi_ld, st))) return rc;
     cudaMemsetAsync(p->norms, 0, sizeof(double) * 4, st);
     residual_kernel<double, double><<<residual_grid(batch * ny), 256, 0, st>>>(rhs, rhs_bstride, rhs_ld, psi, psi_bstride, psi_ld, ny, nx,
-                                                        batch, p->dx, p->dy, p->lam_dev, p->n_lam, p->W1h, p->W1l,
-                                                        p->norms, p->sym ? 1 : 0);
+                                                        batch, p->dx, p->dy, p->lam_dev, p->n_lam, rh, rl,
+                                                        p->norms, 2 * p->halfx, p->halfx);
     double h[4];
     if (cudaMemcpyAsync(h, p->norms, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
@@ -1625,25 +1685,12 @@ extern "C" int fvx_dst_kernel_config(int kind) {
 extern "C" int fvx_dst_gemm_step(fvx_dst_plan* p, int which, int batch, void* stream) {
   if (!p || !p->split_ok) return FVX_ERR_ARG;
   if (batch < 1 || batch > p->batch_max) return FVX_ERR_SHAPE;
-  const int ny = p->ny, nx = p->nx;
-  cudaStream_t st = fvx_stream(stream);
-  if (which == 0) {
-    Epi e1 = make_epi(p, EPI_SPLIT, ny, batch * ny, nx, p->W2h, p->W2l, (long long)nx * ny, ny, 0, 0, 1.0, false);
-    if (p->sym) {
-      e1.perm_r = 1;
-      return gemm_sym(p->W1h, p->W1l, batch * ny, nx, p->xPh, p->xPl, p->xQh, p->xQl, e1, st);
-    }
-    return gemm_split(p->W1h, p->W1l, batch * ny, nx, p->Sxh, p->Sxl, nx, e1, st);
-  }
-  if (which == 1) {
-    Epi e2 = make_epi(p, EPI_SPLIT, nx, batch * nx, ny, p->W1h, p->W1l, (long long)ny * nx, nx, 0, 0, 1.0, true);
-    if (p->sym) {
-      e2.perm_r = 1;
-      return gemm_sym(p->W2h, p->W2l, batch * nx, ny, p->yPh, p->yPl, p->yQh, p->yQl, e2, st);
-    }
-    return gemm_split(p->W2h, p->W2l, batch * nx, ny, p->Syh, p->Syl, ny, e2, st);
-  }
-  return FVX_ERR_ARG;
+  if (which != 0 && which != 1) return FVX_ERR_ARG;
+  bf16 *ah, *al;
+  first_operand(p, &ah, &al);
+  bf16 *bh = p->sym ? p->W2h : p->W1h, *bl = p->sym ? p->W2l : p->W1l;
+  if (which == 0) return split_product(p, ah, al, true, false, operand_epi(p, 0, batch, bh, bl), fvx_stream(stream));
+  return split_product(p, bh, bl, false, false, operand_epi(p, 1, batch, ah, al), fvx_stream(stream));
 }
 
 // ===========================================================================
@@ -1767,7 +1814,7 @@ extern "C" int fvx_dst_solve_noalloc_f32(const float* rhs, long long rhs_ld, flo
   if (cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess) return FVX_ERR_CUDA;
   const int total = nx * nx + ny * ny + ny * nx;
   noalloc_tables_kernel<<<(total + 255) / 256, 256, 0, st>>>(ny, nx, dx, dy, lambda, sxh, sxl, syh, syl, inv);
-  split_input_kernel<float><<<grid1d((long long)ny * nx), 256, 0, st>>>(rhs, 0, rhs_ld, ny, nx, 1, w1h, w1l, 1.0);
+  split_input_kernel<float><<<grid1d((long long)ny * nx), 256, 0, st>>>(rhs, 0, rhs_ld, ny, nx, 1, w1h, w1l, nx, 0);
   int rc = fvx_cuda_status();
   if (rc) return rc;
   auto epi = [&](int mode, int R, int M, int N, void* o0, void* o1, long long bs, long long ld, double alpha,

@@ -169,9 +169,8 @@ int fvx_dst_plan_destroy(fvx_dst_plan* plan);
  * computed with the real Hartley transform pair, which diagonalises the
  * same periodic 5-point operator).  Input and output are the full [ny, nx]
  * array (no ghost ring); the null mode of a Neumann / periodic Poisson
- * problem is set to zero (the zero-mean solution).  DCT-II and periodic
- * plans take the dense product path; fvx_dst_solve_f64 supports method 0
- * only for them. */
+ * problem is set to zero (the zero-mean solution).  fvx_dst_solve_f64
+ * supports method 0 only for DCT-II and periodic plans. */
 int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, double dy, int batch_max, const double* lambdas,
                              int n_lambda, int want_fp64, fvx_dst_plan** plan);
 /* Capacitance-matrix step between the two rectangular solves of a masked
