@@ -71,8 +71,7 @@ struct LayerDesc {     // psi_k = sum_m c[m] psi_mode[b[m]]
 
 // Persistent fused-stage kernel over every tile of every field.  The tile's
 // field arguments are read from shared memory: a register copy stays live
-// across the whole tile body (WENO5: 63 registers against the single-field
-// kernel's 40, four resident blocks per SM instead of six).
+// across the whole tile body and costs resident blocks.
 template <int S>
 __global__ void __launch_bounds__(qg::THREADS, 6)
 ens_stage_kernel(const FieldDesc* __restrict__ fields, int nfields, int stage, int total, unsigned* counter) {

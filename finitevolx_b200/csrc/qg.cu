@@ -24,19 +24,39 @@ static int launch_t(const StageArgs& a, cudaStream_t st) {
   static fvx_once_per_device attr;
   if (fvx_once_on_device(attr, [sm] { return fvx_set_max_smem(stage_kernel<T, S, TX, TY>, (int)sm); }))
     return FVX_ERR_CUDA;
-  const TileSplit ts = tile_split<S, TX, TY>(a.ny, a.nx);
+  const TileSplit ts = tile_split<T, S, TX, TY>(a.ny, a.nx);
   if (fvx_launch_pdl(stage_kernel<T, S, TX, TY>, dim3(ts.ntx * ts.nty), dim3(THREADS), sm, st, a, ts) !=
       cudaSuccess)
     return FVX_ERR_CUDA;
   return fvx_cuda_status();
 }
 
-// Tile configuration per (scheme, dtype), set by the autotuner.
-static int g_tile_cfg[32][2] = {};
+// Tile configuration per (scheme, dtype) as fvx_qg_tile_config set it, -1:
+// by the field's size.
+static int g_tile_cfg[32][2];
+static const bool g_tile_init = [] {
+  for (auto& c : g_tile_cfg) c[0] = c[1] = -1;
+  return true;
+}();
+
+// Rows per march by field size: long marches spread a tile's set-up and halo
+// (its first faces, its loads) over more cells, short ones give every SM
+// enough warps.  us per step with 64x32 (16 rows) / 64x16 (8) / 32x16 (4) /
+// 16x16 (2): 2048^2 FP32 440 / 448 / 468 / 500, 1024^2 FP32 254 / 212 / 201 /
+// 208, 256^2 FP32 121 / 99 / 88 / 82, 1024^2 FP64 742 / 727 / 727 / 740, 256^2
+// FP64 109 / 77 / 63 / 56.
+static int default_tile(long long cells) {
+  if (cells >= 3500000) return 3;
+  if (cells >= 1900000) return 0;
+  if (cells >= 500000) return 1;
+  return 5;
+}
 
 template <typename T, int S>
 static int launch(const StageArgs& a, cudaStream_t st) {
-  switch (g_tile_cfg[S][sizeof(T) == 8]) {
+  int cfg = g_tile_cfg[S][sizeof(T) == 8];
+  if (cfg < 0) cfg = default_tile((long long)a.ny * a.nx);
+  switch (cfg) {
     case 1: return launch_t<T, S, kTileTX[1], kTileTY[1]>(a, st);
     case 2: return launch_t<T, S, kTileTX[2], kTileTY[2]>(a, st);
     case 3: return launch_t<T, S, kTileTX[3], kTileTY[3]>(a, st);
@@ -93,8 +113,8 @@ FVX_DEF_QG(f64, double)
 
 // Tile shape of the fused stage kernel for one scheme and dtype (0 FP32, 1
 // FP64): cfg 0 = 64x16, 1 = 32x16, 2 = 128x8, 3 = 64x32, 4 = 128x16, 5 = 16x16
-// cells.  Returns the number of
-// configurations when cfg < 0 (and changes nothing).
+// cells (until the first call a tile is chosen by the field's size).  Returns
+// the number of configurations when cfg < 0 (and changes nothing).
 extern "C" int fvx_qg_tile_config(int method, int dtype, int cfg) {
   if (cfg < 0) return qg::kTileConfigs;
   if (method < 0 || method >= 32 || dtype < 0 || dtype > 1 || cfg >= qg::kTileConfigs) return FVX_ERR_ARG;

@@ -38,66 +38,97 @@ template <typename T> DEV T tabs(T x) { return x < T(0) ? -x : x; }
 template <typename T> DEV T tmax(T a, T b) { return a > b ? a : b; }
 template <typename T> DEV T tmin(T a, T b) { return a < b ? a : b; }
 
+// The reconstructions below work on the differences d of neighbouring cells:
+// a candidate is q0 plus a combination of them, the smoothness forms are
+// squares of them, and the weights 1 / s_k (s_k = (b_k + eps)^2) are brought
+// to their common denominator, prod_{j != k} s_j, so that one division
+// normalises the whole sum (a division costs 13 FP64 FMAs of throughput;
+// FP32 takes one reciprocal).  s_k >= eps^2, so no product underflows;
+// stencils whose products overflow take the form with a division per weight.
+template <typename T> DEV bool recon_finite(T den, T num) {
+  if constexpr (sizeof(T) == 8) return den < 1e308 && fabs(num) < 1e308;
+  else return den < 3e38f && fabsf(num) < 3e38f;
+}
+
 // ---- WENO3 (advection/weno.py:297-347) ------------------------------------
 // The right-biased forms (:413-459, :462-522, :597-665) are these functions on
 // the mirrored stencil; face_value() below feeds them that way.
 template <typename T> DEV T weno3(T qm, T q0, T qp) {
   const T eps = T(1e-8);
-  T qi1 = T(-0.5) * qm + T(1.5) * q0;
-  T qi2 = T(0.5) * (q0 + qp);
-  T w1 = fdiv(T(1.0 / 3.0), sq(sq(q0 - qm) + eps));
-  T w2 = fdiv(T(2.0 / 3.0), sq(sq(qp - q0) + eps));
-  return fdiv(w1 * qi1 + w2 * qi2, w1 + w2);
+  const T d1 = q0 - qm, d2 = qp - q0;
+  const T s1 = sq(d1 * d1 + eps), s2 = sq(d2 * d2 + eps);
+  // weights 1/3, 2/3 and candidates q0 + d/2: (s2 d1 + 2 s1 d2) / (2 (s2 + 2 s1))
+  const T den = s2 + T(2) * s1, num = s2 * d1 + T(2) * (s1 * d2);
+  if (recon_finite(den, num)) return q0 + T(0.5) * fdiv(num, den);
+  const T w1 = fdiv(T(1.0 / 3.0), s1), w2 = fdiv(T(2.0 / 3.0), s2);
+  return fdiv(w1 * (T(-0.5) * qm + T(1.5) * q0) + w2 * (T(0.5) * (q0 + qp)), w1 + w2);
 }
 template <typename T> DEV T wenoz3(T qm, T q0, T qp) {
   const T eps = T(1e-14);
-  T qi1 = T(-0.5) * qm + T(1.5) * q0;
-  T qi2 = T(0.5) * (q0 + qp);
-  T b1 = sq(q0 - qm), b2 = sq(qp - q0);
-  T tau = tabs(b2 - b1);
-  T w1 = T(1.0 / 3.0) * (T(1) + fdiv(tau, b1 + eps));
-  T w2 = T(2.0 / 3.0) * (T(1) + fdiv(tau, b2 + eps));
-  return fdiv(w1 * qi1 + w2 * qi2, w1 + w2);
+  const T d1 = q0 - qm, d2 = qp - q0;
+  const T b1 = d1 * d1, b2 = d2 * d2, tau = tabs(b2 - b1), t1 = b1 + eps, t2 = b2 + eps;
+  const T W1 = (t1 + tau) * t2, W2 = T(2) * ((t2 + tau) * t1);
+  const T den = W1 + W2, num = W1 * d1 + W2 * d2;
+  if (recon_finite(den, num)) return q0 + T(0.5) * fdiv(num, den);
+  const T w1 = T(1.0 / 3.0) * (T(1) + fdiv(tau, t1)), w2 = T(2.0 / 3.0) * (T(1) + fdiv(tau, t2));
+  return fdiv(w1 * (T(-0.5) * qm + T(1.5) * q0) + w2 * (T(0.5) * (q0 + qp)), w1 + w2);
 }
 // ---- WENO5 (advection/weno.py:350-410, :462-522) -------------------------
+// The form with a division per weight, on the raw values.
 template <typename T, bool Z>
-DEV T weno5_core(T qi1, T qi2, T qi3, T b1, T b2, T b3) {
+__noinline__ __device__ T weno5_divisions(T qmm, T qm, T q0, T qp, T qpp) {
+  const T k1 = T(13.0 / 12.0), k2 = T(0.25);
+  const T qi1 = T(1.0 / 3.0) * qmm - T(7.0 / 6.0) * qm + T(11.0 / 6.0) * q0;
+  const T qi2 = T(-1.0 / 6.0) * qm + T(5.0 / 6.0) * q0 + T(1.0 / 3.0) * qp;
+  const T qi3 = T(1.0 / 3.0) * q0 + T(5.0 / 6.0) * qp - T(1.0 / 6.0) * qpp;
+  const T b1 = k1 * sq(qmm - T(2) * qm + q0) + k2 * sq(qmm - T(4) * qm + T(3) * q0);
+  const T b2 = k1 * sq(qm - T(2) * q0 + qp) + k2 * sq(qm - qp);
+  const T b3 = k1 * sq(q0 - T(2) * qp + qpp) + k2 * sq(T(3) * q0 - T(4) * qp + qpp);
+  T w1, w2, w3;
   if (Z) {
-    const T eps = T(1e-16);
-    T tau5 = tabs(b1 - b3);
-    T w1 = T(0.1) * (T(1) + fdiv(tau5, b1 + eps));
-    T w2 = T(0.6) * (T(1) + fdiv(tau5, b2 + eps));
-    T w3 = T(0.3) * (T(1) + fdiv(tau5, b3 + eps));
-    return fdiv(w1 * qi1 + w2 * qi2 + w3 * qi3, w1 + w2 + w3);
+    const T eps = T(1e-16), tau5 = tabs(b1 - b3);
+    w1 = T(0.1) * (T(1) + fdiv(tau5, b1 + eps));
+    w2 = T(0.6) * (T(1) + fdiv(tau5, b2 + eps));
+    w3 = T(0.3) * (T(1) + fdiv(tau5, b3 + eps));
   } else {
     const T eps = T(1e-8);
-    if constexpr (sizeof(T) == 4) {
-      // FP32: the weights d_k / s_k (s_k = (b_k + eps)^2) times s1 s2 s3,
-      // d_k prod_{j != k} s_j, give the same normalised combination with one
-      // reciprocal instead of four.  s_k >= 1e-16, so no product underflows;
-      // the few stencils whose products overflow (|q| jumps above ~1e4) take
-      // the four-division form.
-      const float s1 = sq(b1 + eps), s2 = sq(b2 + eps), s3 = sq(b3 + eps);
-      const float W1 = 0.1f * (s2 * s3), W2 = 0.6f * (s1 * s3), W3 = 0.3f * (s1 * s2);
-      const float den = W1 + W2 + W3;
-      const float r = (W1 * qi1 + W2 * qi2 + W3 * qi3) * rcp_approx(den);
-      if (den < 3e38f && fabsf(r) < 3.4e38f) return r;
-    }
-    T w1 = fdiv(T(0.1), sq(b1 + eps));
-    T w2 = fdiv(T(0.6), sq(b2 + eps));
-    T w3 = fdiv(T(0.3), sq(b3 + eps));
-    return fdiv(w1 * qi1 + w2 * qi2 + w3 * qi3, w1 + w2 + w3);
+    w1 = fdiv(T(0.1), sq(b1 + eps));
+    w2 = fdiv(T(0.6), sq(b2 + eps));
+    w3 = fdiv(T(0.3), sq(b3 + eps));
   }
+  return fdiv(w1 * qi1 + w2 * qi2 + w3 * qi3, w1 + w2 + w3);
 }
 template <typename T, bool Z> DEV T weno5(T qmm, T qm, T q0, T qp, T qpp) {
-  const T k1 = T(13.0 / 12.0), k2 = T(0.25);
-  T qi1 = T(1.0 / 3.0) * qmm - T(7.0 / 6.0) * qm + T(11.0 / 6.0) * q0;
-  T qi2 = T(-1.0 / 6.0) * qm + T(5.0 / 6.0) * q0 + T(1.0 / 3.0) * qp;
-  T qi3 = T(1.0 / 3.0) * q0 + T(5.0 / 6.0) * qp - T(1.0 / 6.0) * qpp;
-  T b1 = k1 * sq(qmm - T(2) * qm + q0) + k2 * sq(qmm - T(4) * qm + T(3) * q0);
-  T b2 = k1 * sq(qm - T(2) * q0 + qp) + k2 * sq(qm - qp);
-  T b3 = k1 * sq(q0 - T(2) * qp + qpp) + k2 * sq(T(3) * q0 - T(4) * qp + qpp);
-  return weno5_core<T, Z>(qi1, qi2, qi3, b1, b2, b3);
+  const T d0 = qm - qmm, d1 = q0 - qm, d2 = qp - q0, d3 = qpp - qp;
+  const T a1 = d1 - d0, a2 = d2 - d1, a3 = d3 - d2;
+  const T c1 = a1 + T(2) * d1, c2 = d1 + d2, c3 = a3 - T(2) * d2;
+  const T k = T(13.0 / 3.0), eps4 = Z ? T(4e-16) : T(4e-8);
+  // t = 4 (b + eps)
+  const T t1 = c1 * c1 + (k * a1 * a1 + eps4), t2 = c2 * c2 + (k * a2 * a2 + eps4),
+          t3 = c3 * c3 + (k * a3 * a3 + eps4);
+  const T g1 = T(5.0 / 6.0) * d1 - T(1.0 / 3.0) * d0, g2 = T(1.0 / 6.0) * d1 + T(1.0 / 3.0) * d2,
+          g3 = T(2.0 / 3.0) * d2 - T(1.0 / 6.0) * d3;
+  T W1, W2, W3;
+  if constexpr (Z) {
+    const T tau = tabs(t1 - t3);
+    if constexpr (sizeof(T) == 4) {  // products of three t >= 4e-16 would underflow
+      W1 = T(0.1) * (T(1) + fdiv(tau, t1));
+      W2 = T(0.6) * (T(1) + fdiv(tau, t2));
+      W3 = T(0.3) * (T(1) + fdiv(tau, t3));
+    } else {
+      W1 = T(0.1) * ((t1 + tau) * (t2 * t3));
+      W2 = T(0.6) * ((t2 + tau) * (t1 * t3));
+      W3 = T(0.3) * ((t3 + tau) * (t1 * t2));
+    }
+  } else {
+    const T s1 = t1 * t1, s2 = t2 * t2, s3 = t3 * t3;
+    W1 = T(0.1) * (s2 * s3);
+    W2 = T(0.6) * (s1 * s3);
+    W3 = T(0.3) * (s1 * s2);
+  }
+  const T den = W1 + W2 + W3, num = W1 * g1 + W2 * g2 + W3 * g3;
+  if (recon_finite(den, num)) return q0 + fdiv(num, den);
+  return weno5_divisions<T, Z>(qmm, qm, q0, qp, qpp);
 }
 // ---- WENO7 / WENO9, generic Jiang-Shu form (advection/weno.py:268-294) ---
 template <typename T> DEV T tab_c(int R, int k, int j) {
@@ -132,12 +163,12 @@ DEV T weno_generic(const T* vin) {
   T v[2 * R - 1];
 #pragma unroll
   for (int k = 0; k < 2 * R - 1; ++k) v[k] = SHIFT ? vin[k] - s : vin[k];
-  T num = T(0), den = T(0);
+  T cand[R], st[R];
 #pragma unroll
   for (int k = 0; k < R; ++k) {
-    T cand = T(0);
+    cand[k] = T(0);
 #pragma unroll
-    for (int j = 0; j < R; ++j) cand = cand + tab_c<T>(R, k, j) * v[k + j];
+    for (int j = 0; j < R; ++j) cand[k] = cand[k] + tab_c<T>(R, k, j) * v[k + j];
     T beta = T(0);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -146,9 +177,29 @@ DEV T weno_generic(const T* vin) {
       for (int j = 0; j < R; ++j) row = row + tab_b<T>(R, k, i, j) * v[k + j];
       beta = beta + v[k + i] * row;
     }
-    T a = fdiv(tab_w<T>(R, k), sq(beta + eps));
+    st[k] = sq(beta + eps);
+  }
+  T num = T(0), den = T(0);
+  if constexpr (sizeof(T) == 8) {  // one division (in FP32 the products of three or four s_k underflow)
+    T pre[R], suf = T(1);
+    pre[0] = T(1);
+#pragma unroll
+    for (int k = 1; k < R; ++k) pre[k] = pre[k - 1] * st[k - 1];
+#pragma unroll
+    for (int k = R - 1; k >= 0; --k) {
+      const T a = tab_w<T>(R, k) * (pre[k] * suf);
+      suf *= st[k];
+      den = den + a;
+      num = num + a * cand[k];
+    }
+    if (recon_finite(den, num)) return num / den;
+    num = den = T(0);
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const T a = fdiv(tab_w<T>(R, k), st[k]);
     den = den + a;
-    num = num + a * cand;
+    num = num + a * cand[k];
   }
   return SHIFT ? s + fdiv(num, den) : num / den;
 }
@@ -159,6 +210,18 @@ template <typename T, int S> DEV T limiter(T r) {
   if (S == FVX_VAN_LEER) { T ra = tabs(r); return (r + ra) / (T(1) + ra); }
   if (S == FVX_SUPERBEE) return tmax(T(0), tmax(tmin(T(2) * r, T(1)), tmin(r, T(2))));
   return tmax(T(0), tmin(tmin((T(1) + r) / T(2), T(2) * r), T(2)));  // MC
+}
+
+// limiter(r) with r = a / b, van Leer with one division: for r > 0 its value
+// is 2a / (a + b) (no cancellation: a and b have one sign), for finite r < 0
+// it is 0; zero, overflowing and undefined ratios keep the two-division form.
+template <typename T, int S> DEV T limiter_ratio(T a, T b) {
+  if constexpr (S == FVX_VAN_LEER) {
+    const T p = a * b, big = sizeof(T) == 8 ? T(1e300) : T(1e37f);
+    if (p > T(0) && p < big) return T(2) * a / (a + b);
+    if (p < T(0) && p > -big) return T(0);
+  }
+  return limiter<T, S>(a / b);
 }
 
 template <int S> struct SchemeInfo {
@@ -194,14 +257,12 @@ DEV T face_value(const T* p, int st, int i, int N, bool pos) {
     if (pos) {
       T dfwd = at(1) - at(0);
       T dbwd = at(0) - at(-1);
-      T r = dbwd / (dfwd + T(1e-8));
-      return at(0) + T(0.5) * limiter<T, S>(r) * dfwd;
+      return at(0) + T(0.5) * limiter_ratio<T, S>(dbwd, dfwd + T(1e-8)) * dfwd;
     }
     if (i > N - 3) return at(1);
     T dn = at(0) - at(1);
     T dn2 = at(1) - at(2);
-    T r = dn2 / (dn + T(1e-8));
-    return at(1) + T(0.5) * limiter<T, S>(r) * dn;
+    return at(1) + T(0.5) * limiter_ratio<T, S>(dn2, dn + T(1e-8)) * dn;
   }
   if constexpr (SchemeInfo<S>::is_weno) {
     // Upwind-oriented stencil: e(k) is the cell k steps downstream of the
