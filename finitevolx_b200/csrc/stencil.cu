@@ -1,24 +1,10 @@
-// Stencil operators on the Arakawa C-grid: advection (all finitevolX
-// schemes, with mask-aware tier dispatch), face fluxes, C-grid differences
+// Stencil operators on the Arakawa C-grid: face fluxes (all finitevolX
+// schemes, with mask-aware tier dispatch), C-grid differences
 // and interpolations, Arakawa Jacobian, harmonic / biharmonic diffusion and
 // the periodic ghost-ring fill.  FP32 and FP64 instantiations of each.
 #include "recon.cuh"
 
 namespace fvx {
-
-// ===========================================================================
-// Advection: fused face-flux + flux divergence, one smem tile per CTA.
-// Restates Advection2D.__call__ (advection/advection.py:329-420):
-//   out[2:-2,2:-2] = -((fe[j,i]-fe[j,i-1])/dx + (fn[j,i]-fn[j-1,i])/dy),
-//   zero elsewhere, then * mask.h when a mask is given.
-// Masked dispatchable methods pick, per face, the reconstruction of the tier
-// of the upwind cell (upwind_flux, advection/flux.py:221-253).
-// ===========================================================================
-
-constexpr int ATX = 64;   // output tile width (cells)
-constexpr int ATY = 16;   // output tile height
-constexpr int AH = 5;     // halo covering WENO9 (face i reads i-4 .. i+5)
-constexpr int ATHREADS = 256;
 
 // tier byte: bits 0-1 x-tier, bits 2-3 y-tier; 0 none, 1 -> s=2, 2 -> s=4, 3 -> s=6
 template <typename T, int S4, int S6>
@@ -27,139 +13,6 @@ DEV T tiered_face(const T* p, int st, int i, int N, bool pos, int code) {
   if (code == 1) return pos ? p[0] : p[st];  // upwind1
   if (code == 3 && S6 >= 0) return face_value<T, (S6 >= 0 ? S6 : 0)>(p, st, i, N, pos);
   return face_value<T, S4>(p, st, i, N, pos);
-}
-
-// One load phase per tile: h (tile + halo), u on the tile's east faces and v
-// on its north faces land in one flat shared buffer, four loads in flight
-// per thread (eight raise the FP32 kernels' registers from 31 to 59); the
-// face fluxes then overwrite u and v in place.
-// FP64 WENO7 / WENO9 faces are evaluated through a call: inlined into the
-// face loops, the compiler hoists the schemes' ~84 table coefficients out of
-// the loop into registers (FP64 WENO7: 134 registers, or spills under a cap
-// of three CTAs per SM); behind the call they stay constant-bank operands
-// (56-60 registers, no spills).  FP32 inlined needs 39 registers and runs
-// faster than through the call.
-template <typename T, int S>
-struct AdvFaceCall {
-  static constexpr bool v = sizeof(T) == 8 && (S == FVX_WENO7 || S == FVX_WENO9);
-};
-template <typename T, int S>
-__noinline__ __device__ T face_value_call(const T* p, int st, int i, int N, bool pos) {
-  return face_value<T, S>(p, st, i, N, pos);
-}
-template <typename T, int S>
-DEV T adv_face(const T* p, int st, int i, int N, bool pos) {
-  if constexpr (AdvFaceCall<T, S>::v) return face_value_call<T, S>(p, st, i, N, pos);
-  else return face_value<T, S>(p, st, i, N, pos);
-}
-template <typename T, int S, int S4, int S6, bool MASKED>
-__global__ void __launch_bounds__(ATHREADS)
-advect_tile_kernel(const T* __restrict__ h, const T* __restrict__ u, const T* __restrict__ v,
-                   T* __restrict__ out, int ny, int nx, T dx, T dy,
-                   const uint8_t* __restrict__ tiers, const uint8_t* __restrict__ mh) {
-  constexpr int HW = ATX + 2 * AH, HH = ATY + 2 * AH;
-  constexpr int NH = HH * HW, NU = ATY * (ATX + 1), NV = (ATY + 1) * ATX, NTOT = NH + NU + NV;
-  constexpr int U = 4;
-  __shared__ T tl[NTOT];
-  __shared__ uint8_t tx_[ATY][ATX + 2];
-  __shared__ uint8_t ty_[ATY + 2][ATX];
-  T* hs = tl;             // [HH][HW], origin (y0 - AH, x0 - AH)
-  T* fe = tl + NH;        // [ATY][ATX + 1]: u on east faces, then the x flux
-  T* fn = tl + NH + NU;   // [ATY + 1][ATX]: v on north faces, then the y flux
-  const int x0 = blockIdx.x * ATX, y0 = blockIdx.y * ATY;
-  const int tid = threadIdx.x;
-  for (int k0 = tid; k0 < NTOT; k0 += U * ATHREADS) {
-    T val[U];
-#pragma unroll
-    for (int q = 0; q < U; ++q) {
-      int k = k0 + q * ATHREADS;
-      T x = T(0);
-      if (k < NH) {
-        const int ly = k / HW, lx = k - ly * HW;
-        const int gy = y0 - AH + ly, gx = x0 - AH + lx;
-        if (gy >= 0 && gy < ny && gx >= 0 && gx < nx) x = h[(size_t)gy * nx + gx];
-      } else if (k < NH + NU) {
-        k -= NH;
-        const int ly = k / (ATX + 1), lf = k - ly * (ATX + 1);
-        const int gj = y0 + ly, gi = x0 - 1 + lf;
-        if (gj >= 1 && gj <= ny - 2 && gi >= 1 && gi <= nx - 2) x = u[(size_t)gj * nx + gi];
-      } else if (k < NTOT) {
-        k -= NH + NU;
-        const int lf = k / ATX, lx = k - lf * ATX;
-        const int gj = y0 - 1 + lf, gi = x0 + lx;
-        if (gj >= 1 && gj <= ny - 2 && gi >= 1 && gi <= nx - 2) x = v[(size_t)gj * nx + gi];
-      }
-      val[q] = x;
-    }
-#pragma unroll
-    for (int q = 0; q < U; ++q)
-      if (k0 + q * ATHREADS < NTOT) tl[k0 + q * ATHREADS] = val[q];
-  }
-  if (MASKED) {
-    for (int k = tid; k < ATY * (ATX + 2); k += ATHREADS) {
-      int ly = k / (ATX + 2), lx = k % (ATX + 2);
-      int gy = y0 + ly, gx = x0 - 1 + lx;
-      tx_[ly][lx] = (gy < ny && gx >= 0 && gx < nx) ? (tiers[(size_t)gy * nx + gx] & 3) : 0;
-    }
-    for (int k = tid; k < (ATY + 2) * ATX; k += ATHREADS) {
-      int ly = k / ATX, lx = k % ATX;
-      int gy = y0 - 1 + ly, gx = x0 + lx;
-      ty_[ly][lx] = (gy >= 0 && gy < ny && gx < nx) ? ((tiers[(size_t)gy * nx + gx] >> 2) & 3) : 0;
-    }
-  }
-  __syncthreads();
-  // Face fluxes, overwriting u / v in place.  East face (ly, lf) is the
-  // face between cells x0-2+lf and x0-1+lf of row y0+ly; north face (lf, lx)
-  // the one between rows y0-2+lf and y0-1+lf of column x0+lx.  Each trip of
-  // the first loop takes cell (y0+ly, x0+lx)'s east and north faces (two
-  // independent reconstructions; ATY x ATX / ATHREADS whole trips), the
-  // second the tile's west-most east faces and south-most north faces.
-  auto east = [&](int ly, int lf) -> T {
-    const int gj = y0 + ly, gi = x0 - 1 + lf;
-    if (!(gj >= 1 && gj <= ny - 2 && gi >= 1 && gi <= nx - 2)) return T(0);
-    const T uu = fe[ly * (ATX + 1) + lf];
-    const bool pos = uu >= T(0);
-    const T* p = &hs[(ly + AH) * HW + lf - 1 + AH];
-    T hf;
-    if (MASKED) hf = tiered_face<T, S4, S6>(p, 1, gi, nx, pos, pos ? tx_[ly][lf] : tx_[ly][lf + 1]);
-    else hf = adv_face<T, S>(p, 1, gi, nx, pos);
-    return hf * uu;
-  };
-  auto north = [&](int lf, int lx) -> T {
-    const int gj = y0 - 1 + lf, gi = x0 + lx;
-    if (!(gj >= 1 && gj <= ny - 2 && gi >= 1 && gi <= nx - 2)) return T(0);
-    const T vv = fn[lf * ATX + lx];
-    const bool pos = vv >= T(0);
-    const T* p = &hs[(lf - 1 + AH) * HW + lx + AH];
-    T hf;
-    if (MASKED) hf = tiered_face<T, S4, S6>(p, HW, gj, ny, pos, pos ? ty_[lf][lx] : ty_[lf + 1][lx]);
-    else hf = adv_face<T, S>(p, HW, gj, ny, pos);
-    return hf * vv;
-  };
-  static_assert((ATY * ATX) % ATHREADS == 0, "whole trips over the tile's cells");
-#pragma unroll 1
-  for (int k = tid; k < ATY * ATX; k += ATHREADS) {
-    const int ly = k / ATX, lx = k - ly * ATX;
-    const T a = east(ly, lx + 1), b = north(ly + 1, lx);
-    fe[ly * (ATX + 1) + lx + 1] = a;
-    fn[(ly + 1) * ATX + lx] = b;
-  }
-  for (int k = tid; k < ATY + ATX; k += ATHREADS) {
-    if (k < ATY) fe[k * (ATX + 1)] = east(k, 0);
-    else fn[k - ATY] = north(0, k - ATY);
-  }
-  __syncthreads();
-  for (int k = tid; k < ATY * ATX; k += ATHREADS) {
-    int ly = k / ATX, lx = k % ATX;
-    int gj = y0 + ly, gi = x0 + lx;
-    if (gj >= ny || gi >= nx) continue;
-    T r = T(0);
-    if (gj >= 2 && gj <= ny - 3 && gi >= 2 && gi <= nx - 3)
-      r = -((fe[ly * (ATX + 1) + lx + 1] - fe[ly * (ATX + 1) + lx]) / dx +
-            (fn[(ly + 1) * ATX + lx] - fn[ly * ATX + lx]) / dy);
-    if (MASKED || mh != nullptr) r = r * T(mh[(size_t)gj * nx + gi]);
-    out[(size_t)gj * nx + gi] = r;
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -517,19 +370,6 @@ __global__ void upwind_blend_kernel(BlendArgs<T> A, const T* __restrict__ u, T* 
 // ===========================================================================
 // Host dispatch
 // ===========================================================================
-template <typename T, int S>
-static void launch_advect_unmasked(const T* h, const T* u, const T* v, T* out, int ny, int nx, T dx, T dy,
-                                   const uint8_t* mh, cudaStream_t st) {
-  dim3 g((nx + ATX - 1) / ATX, (ny + ATY - 1) / ATY);
-  advect_tile_kernel<T, S, 0, -1, false><<<g, ATHREADS, 0, st>>>(h, u, v, out, ny, nx, dx, dy, nullptr, mh);
-}
-template <typename T, int S4, int S6>
-static void launch_advect_masked(const T* h, const T* u, const T* v, T* out, int ny, int nx, T dx, T dy,
-                                 const uint8_t* tiers, const uint8_t* mh, cudaStream_t st) {
-  dim3 g((nx + ATX - 1) / ATX, (ny + ATY - 1) / ATY);
-  advect_tile_kernel<T, 0, S4, S6, true><<<g, ATHREADS, 0, st>>>(h, u, v, out, ny, nx, dx, dy, tiers, mh);
-}
-
 // Minimum line length each scheme's boundary ladder is defined for.
 static int min_len(int m) {
   switch (m) {
@@ -538,39 +378,6 @@ static int min_len(int m) {
     case FVX_WENO5: case FVX_WENOZ5: return 4;
     default: return 3;
   }
-}
-
-template <typename T>
-static int advect2d(const T* h, const T* u, const T* v, T* out, int ny, int nx, double dx, double dy,
-                    int method, const uint8_t* tiers, const uint8_t* mh, cudaStream_t st) {
-  if (!h || !u || !v || !out) return FVX_ERR_ARG;
-  if (method < 0 || method >= FVX_WENOZ3) return FVX_ERR_METHOD;
-  if (ny < min_len(method) || nx < min_len(method)) return FVX_ERR_SHAPE;
-  T tdx = T(dx), tdy = T(dy);
-  if (tiers) {
-    if (!mh) return FVX_ERR_ARG;
-    switch (method) {
-      case FVX_WENO5: launch_advect_masked<T, FVX_WENO3, FVX_WENO5>(h, u, v, out, ny, nx, tdx, tdy, tiers, mh, st); break;
-      case FVX_WENOZ5: launch_advect_masked<T, FVX_WENOZ3, FVX_WENOZ5>(h, u, v, out, ny, nx, tdx, tdy, tiers, mh, st); break;
-      case FVX_WENO3: launch_advect_masked<T, FVX_WENO3, -1>(h, u, v, out, ny, nx, tdx, tdy, tiers, mh, st); break;
-      case FVX_MINMOD: launch_advect_masked<T, FVX_MINMOD, -1>(h, u, v, out, ny, nx, tdx, tdy, tiers, mh, st); break;
-      case FVX_VAN_LEER: launch_advect_masked<T, FVX_VAN_LEER, -1>(h, u, v, out, ny, nx, tdx, tdy, tiers, mh, st); break;
-      case FVX_SUPERBEE: launch_advect_masked<T, FVX_SUPERBEE, -1>(h, u, v, out, ny, nx, tdx, tdy, tiers, mh, st); break;
-      case FVX_MC: launch_advect_masked<T, FVX_MC, -1>(h, u, v, out, ny, nx, tdx, tdy, tiers, mh, st); break;
-      default: return FVX_ERR_METHOD;
-    }
-    return fvx_cuda_status();
-  }
-  switch (method) {
-#define FVX_CASE(M) case M: launch_advect_unmasked<T, M>(h, u, v, out, ny, nx, tdx, tdy, mh, st); break;
-    FVX_CASE(FVX_NAIVE) FVX_CASE(FVX_UPWIND1) FVX_CASE(FVX_UPWIND2) FVX_CASE(FVX_UPWIND3)
-    FVX_CASE(FVX_WENO3) FVX_CASE(FVX_WENO5) FVX_CASE(FVX_WENOZ5) FVX_CASE(FVX_WENO7)
-    FVX_CASE(FVX_WENO9) FVX_CASE(FVX_MINMOD) FVX_CASE(FVX_VAN_LEER) FVX_CASE(FVX_SUPERBEE)
-    FVX_CASE(FVX_MC)
-#undef FVX_CASE
-    default: return FVX_ERR_METHOD;
-  }
-  return fvx_cuda_status();
 }
 
 template <typename T, int S, int S4, int S6, bool MK>
@@ -620,12 +427,7 @@ using namespace fvx;
 // ===========================================================================
 #define FVX_DTYPES(X) X(f32, float) X(f64, double)
 
-#define FVX_DEF_ADVECT(SFX, T)                                                                       \
-  extern "C" int fvx_advect2d_##SFX(const T* h, const T* u, const T* v, T* out, int ny, int nx,      \
-                                    double dx, double dy, int method, const uint8_t* tiers,          \
-                                    const uint8_t* mask_h, void* stream) {                           \
-    return advect2d<T>(h, u, v, out, ny, nx, dx, dy, method, tiers, mask_h, fvx_stream(stream));      \
-  }                                                                                                  \
+#define FVX_DEF_STENCIL(SFX, T)                                                                       \
   extern "C" int fvx_face_flux2d_##SFX(const T* h, const T* u, const T* v, T* fe, T* fn, int ny,     \
                                        int nx, int method, const uint8_t* tiers, void* stream) {     \
     return face_flux2d<T>(h, u, v, fe, fn, ny, nx, method, tiers, fvx_stream(stream));               \
@@ -698,7 +500,7 @@ using namespace fvx;
     return fvx_cuda_status();                                                                        \
   }
 
-FVX_DTYPES(FVX_DEF_ADVECT)
+FVX_DTYPES(FVX_DEF_STENCIL)
 
 #define FVX_DEF_MISC(SFX, T)                                                                          \
   extern "C" int fvx_lincomb_##SFX(int64_t n, double a, const T* x, double b, const T* y, double c,   \
