@@ -134,19 +134,22 @@ __global__ void cgrid_op_kernel(int op, const T* __restrict__ a, const T* __rest
 // ===========================================================================
 // Arakawa Jacobian (operators/jacobian.py:106-131): out [B, Ny-2, Nx-2].
 // ===========================================================================
-// A thread per output column walking kJacRows rows with a 3 x 3 window of f
+// A thread per output column walking `rows` rows with a 3 x 3 window of f
 // and g in registers (three new values of each per row instead of eight):
 // the warp's loads of a row are consecutive columns.  Each output keeps the
-// reference's three-form expression and operand order.
-constexpr int kJacCols = 128, kJacRows = 16;
+// reference's three-form expression and operand order.  rows: 16 where that
+// still gives every SM four blocks, else 4 (130 x 98 FP64: 9 blocks and 11.4
+// us at 16 rows, all of it one column's chain of loads).
+constexpr int kJacCols = 128;
 template <typename T>
 __global__ void __launch_bounds__(kJacCols)
-jacobian_kernel(const T* __restrict__ f, const T* __restrict__ g, T* __restrict__ out, int ny, int nx, T scale) {
+jacobian_kernel(const T* __restrict__ f, const T* __restrict__ g, T* __restrict__ out, int ny, int nx, T scale,
+                int rows) {
   const int i = blockIdx.x * kJacCols + threadIdx.x;  // output column 0..nx-3
-  const int j0 = blockIdx.y * kJacRows;               // first output row
+  const int j0 = blockIdx.y * rows;                   // first output row
   const int b = blockIdx.z;
   if (i >= nx - 2 || j0 >= ny - 2) return;
-  const int j1 = min(j0 + kJacRows, ny - 2);
+  const int j1 = min(j0 + rows, ny - 2);
   // padded row j0 + r, columns i .. i + 2: window rows a (top), m (middle), c (bottom)
   const T* F = f + (size_t)b * ny * nx + (size_t)j0 * nx + i;
   const T* G = g + (size_t)b * ny * nx + (size_t)j0 * nx + i;
@@ -459,8 +462,10 @@ using namespace fvx;
                                             int nx, double dx, double dy, void* stream) {            \
     if (!f || !g || !out) return FVX_ERR_ARG;                                                        \
     if (ny < 3 || nx < 3 || batch < 1 || batch > 65535) return FVX_ERR_SHAPE;                        \
-    dim3 gr((nx - 2 + kJacCols - 1) / kJacCols, (ny - 2 + kJacRows - 1) / kJacRows, batch);              \
-    jacobian_kernel<T><<<gr, kJacCols, 0, fvx_stream(stream)>>>(f, g, out, ny, nx, T(1.0 / (12.0 * dx * dy))); \
+    const int gx = (nx - 2 + kJacCols - 1) / kJacCols;                                                \
+    const int rows = (long long)gx * ((ny + 13) / 16) * batch >= 4 * 148 || (ny + 1) / 4 > 65535 ? 16 : 4; \
+    dim3 gr(gx, (ny - 2 + rows - 1) / rows, batch);                                                  \
+    jacobian_kernel<T><<<gr, kJacCols, 0, fvx_stream(stream)>>>(f, g, out, ny, nx, T(1.0 / (12.0 * dx * dy)), rows); \
     return fvx_cuda_status();                                                                        \
   }                                                                                                  \
   extern "C" int fvx_diffusion2d_##SFX(const T* h, const T* kappa_field, double kappa, T* out,       \
