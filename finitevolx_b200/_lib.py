@@ -69,7 +69,11 @@ def require_cuda() -> torch.device:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Handle of the current device's current stream."""
+    if not torch.cuda.is_initialized():
+        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle itself, without building a Stream object (~1.5 us a call)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def P(t) -> ctypes.c_void_p:
@@ -81,6 +85,11 @@ def P(t) -> ctypes.c_void_p:
 
 def as_field(x, dtype=None, device=None) -> torch.Tensor:
     """Bring an array-like onto the CUDA device as a contiguous tensor."""
+    # a tensor that is already there, of the wanted type: no availability
+    # query and no device objects (4-5 us per argument of a small call)
+    if (device is None and isinstance(x, torch.Tensor) and x.is_cuda and (dtype is None or x.dtype == dtype)
+            and x.get_device() == torch._C._cuda_getDevice()):
+        return x.contiguous()
     dev = device or require_cuda()
     if isinstance(x, torch.Tensor):
         t = x

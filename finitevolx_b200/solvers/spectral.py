@@ -24,7 +24,7 @@ same linear map as the FFT solve on real data.
 from __future__ import annotations
 
 import ctypes
-from dataclasses import dataclass
+import math
 
 import numpy as np
 import torch
@@ -81,7 +81,7 @@ class DSTHelmholtzPlan:
     def _views(self, rhs):
         if rhs.shape[-2:] != (self.ny, self.nx):
             raise ValueError(f"rhs interior shape {tuple(rhs.shape[-2:])} != plan {(self.ny, self.nx)}")
-        b = int(np.prod(rhs.shape[:-2])) if rhs.ndim > 2 else 1
+        b = math.prod(rhs.shape[:-2])
         if b > self.batch_max:
             raise ValueError(f"batch {b} exceeds the plan's batch_max {self.batch_max}")
         return b
@@ -141,8 +141,17 @@ _CACHE: dict = {}
 SpectralHelmholtzPlan = DSTHelmholtzPlan
 
 
+def _lambda_tuple(lam) -> tuple:
+    """The lambda values as a tuple of floats (one for a scalar)."""
+    if isinstance(lam, (float, int)):
+        return (float(lam),)
+    if isinstance(lam, torch.Tensor):
+        lam = lam.cpu()
+    return tuple(np.atleast_1d(np.asarray(lam, dtype=np.float64)).tolist())
+
+
 def get_plan(ny, nx, dx, dy, lambdas, batch, fp64=True, bc: str = "dst") -> DSTHelmholtzPlan:
-    lam = tuple(np.atleast_1d(np.asarray(lambdas, dtype=np.float64)).tolist())
+    lam = _lambda_tuple(lambdas)
     key = (bc, ny, nx, float(dx), float(dy), lam, torch.cuda.current_device())
     p = _CACHE.get(key)
     if p is None or p.batch_max < batch:
@@ -155,12 +164,11 @@ def _solve(rhs, dx, dy, lambda_, method, bc):
     rhs = L.as_field(rhs)
     if rhs.ndim < 2:
         raise ValueError("rhs must be at least 2-D")
-    lam = np.atleast_1d(np.asarray(lambda_.cpu() if isinstance(lambda_, torch.Tensor) else lambda_,
-                                   dtype=np.float64))
-    if lam.size > 1 and (rhs.ndim < 3 or rhs.shape[-3] != lam.size):
-        raise ValueError(f"rhs.shape[-3] must match the {lam.size} lambda values")
+    lam = _lambda_tuple(lambda_)
+    if len(lam) > 1 and (rhs.ndim < 3 or rhs.shape[-3] != len(lam)):
+        raise ValueError(f"rhs.shape[-3] must match the {len(lam)} lambda values")
     ny, nx = rhs.shape[-2:]
-    b = int(np.prod(rhs.shape[:-2])) if rhs.ndim > 2 else 1
+    b = math.prod(rhs.shape[:-2])
     return get_plan(ny, nx, dx, dy, lam, b, bc=bc).solve(rhs, method=method)
 
 
@@ -211,16 +219,7 @@ def fft_eigenvalues(n: int, d: float) -> np.ndarray:
 
 def solve_helmholtz_dst(rhs, dx: float, dy: float, lambda_=0.0, method: str = "fp64") -> torch.Tensor:
     """(nabla^2 - lambda) psi = rhs with psi = 0 outside the interior array."""
-    rhs = L.as_field(rhs)
-    if rhs.ndim < 2:
-        raise ValueError("rhs must be at least 2-D")
-    lam = np.atleast_1d(np.asarray(lambda_.cpu() if isinstance(lambda_, torch.Tensor) else lambda_,
-                                   dtype=np.float64))
-    if lam.size > 1 and (rhs.ndim < 3 or rhs.shape[-3] != lam.size):
-        raise ValueError(f"rhs.shape[-3] must match the {lam.size} lambda values")
-    ny, nx = rhs.shape[-2:]
-    b = int(np.prod(rhs.shape[:-2])) if rhs.ndim > 2 else 1
-    return get_plan(ny, nx, dx, dy, lam, b).solve(rhs, method=method)
+    return _solve(rhs, dx, dy, lambda_, method, "dst")
 
 
 def solve_poisson_dst(rhs, dx: float, dy: float) -> torch.Tensor:
