@@ -818,23 +818,92 @@ gemm_sym_pair_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_const
 // half > 0: de-interleaved rows (even x first, odd x from element half on,
 // the folded products' operand layout); pitch: elements per output row.
 template <typename T>
-__global__ void split_input_kernel(const T* __restrict__ in, long long bstride, long long ld, int ny, int nx,
+__global__ void split_input_kernel(const T* in, long long bstride, long long ld, int ny, int nx,
                                    int batch, bf16* __restrict__ hi, bf16* __restrict__ lo, int pitch,
                                    int half) {
   // rows of the [batch][ny][nx] input over the grid, (even, odd) pairs of a
-  // row over the threads: no 64-bit divisions, and the two halves
-  // of the de-interleaved row are written by consecutive threads
+  // row over the threads, no 64-bit divisions.  De-interleaved: eight
+  // elements per thread from 16-byte loads where the rows allow (bound by
+  // memory; a pair of 4-byte loads and 2-byte stores per thread kept too few
+  // bytes in flight, 35 us at 16 x 1024^2 FP32, now 20), else two
+  // neighbouring lanes swap an element so that one stores both even elements
+  // as a word and the other both odd ones.  Launched as a programmatic
+  // dependent: the input is the previous kernel's output, read after the wait.
+  grid_dep_wait();
   const int rows = batch * ny, pairs = (nx + 1) >> 1;
+  if (half && (nx & 7) == 0 && (pitch & 7) == 0 && (half & 3) == 0 && ((uintptr_t)in & 15) == 0 &&
+      (ld * sizeof(T)) % 16 == 0 && (bstride * sizeof(T)) % 16 == 0) {
+    const unsigned g8 = (unsigned)nx >> 3, n = (unsigned)rows * g8;
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+      const unsigned r = k / g8, g = k - r * g8;
+      const unsigned b = r / (unsigned)ny, y = r - b * ny;
+      const T* src = in + (long long)b * bstride + (long long)y * ld + 8 * g;
+      float v[8];
+      if constexpr (sizeof(T) == 4) {
+        const float4 a = __ldcg((const float4*)src), c = __ldcg((const float4*)src + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const double2 a = __ldcg((const double2*)src + q);
+          v[2 * q] = (float)a.x;
+          v[2 * q + 1] = (float)a.y;
+        }
+      }
+      uint32_t wh[2][2], wl[2][2];  // [even / odd][two words of two elements]
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float x = v[4 * q + e], z = v[4 * q + 2 + e];
+          const __nv_bfloat162 h2 = __floats2bfloat162_rn(x, z);
+          const __nv_bfloat162 l2 = __floats2bfloat162_rn(x - __low2float(h2), z - __high2float(h2));
+          wh[e][q] = *(const uint32_t*)&h2;
+          wl[e][q] = *(const uint32_t*)&l2;
+        }
+      const long long o = (long long)r * pitch + 4 * g;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        *(uint2*)(hi + o + e * half) = make_uint2(wh[e][0], wh[e][1]);
+        *(uint2*)(lo + o + e * half) = make_uint2(wl[e][0], wl[e][1]);
+      }
+    }
+    grid_dep_launch();
+    return;
+  }
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     const int b = r / ny, y = r - b * ny;
     const T* src = in + (long long)b * bstride + (long long)y * ld;
     const long long o = (long long)r * pitch;
+    if (half && (nx & 3) == 0) {  // pairs come in twos, rows and halves on whole words
+      for (int p0 = 0; p0 < pairs; p0 += blockDim.x) {
+        const int p = p0 + threadIdx.x;
+        const bool ok = p < pairs;
+        uint32_t e[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float v = ok ? (float)__ldcg(src + 2 * p + k) : 0.f;
+          const bf16 h = __float2bfloat16_rn(v);
+          const bf16 l = __float2bfloat16_rn(v - __bfloat162float(h));
+          e[k] = (uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(l) << 16);
+        }
+        const bool odd = p & 1;
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? e[0] : e[1], 1);
+        if (ok) {
+          const uint32_t x0 = odd ? got : e[0], x1 = odd ? e[1] : got;  // elements p & ~1 and p | 1 of this half
+          const long long d = o + (odd ? half : 0) + (p & ~1);
+          *(uint32_t*)(hi + d) = (x0 & 0xffffu) | (x1 << 16);
+          *(uint32_t*)(lo + d) = (x0 >> 16) | (x1 & 0xffff0000u);
+        }
+      }
+      continue;
+    }
     for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int x = 2 * p + e;
         if (x >= nx) break;
-        const float v = (float)src[x];
+        const float v = (float)__ldcg(src + x);
         const bf16 h = __float2bfloat16_rn(v);
         const long long d = o + (half ? (e ? half + p : p) : x);
         hi[d] = h;
@@ -842,6 +911,7 @@ __global__ void split_input_kernel(const T* __restrict__ in, long long bstride, 
       }
     }
   }
+  grid_dep_launch();
 }
 
 template <typename T>
@@ -1461,8 +1531,9 @@ static int split_in(fvx_dst_plan* p, int B, const T* src, long long sbs, long lo
   bf16 *h, *l;
   first_operand(p, &h, &l);
   if (p->kind == FVX_SPECTRAL_DST) {
-    split_input_kernel<T><<<grid1d((long long)B * p->ny * p->nx), 256, 0, st>>>(src, sbs, sld, p->ny, p->nx, B, h, l,
-                                                                               2 * p->halfx, p->halfx);
+    if (fvx_launch_pdl(split_input_kernel<T>, dim3(copy_rows_grid((long long)B * p->ny)), dim3(256), 0, st, src, sbs,
+                       sld, p->ny, p->nx, B, h, l, 2 * p->halfx, p->halfx) != cudaSuccess)
+      return FVX_ERR_CUDA;
     return fvx_cuda_status();
   }
   if (fvx_launch_pdl(fold_split_kernel<T, false>, dim3(copy_rows_grid((long long)B * p->hy)), dim3(256), 0, st, src,
