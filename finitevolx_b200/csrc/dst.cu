@@ -25,6 +25,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <cstdio>
@@ -422,6 +423,12 @@ DEV void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
+DEV void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(taddr));
+}
 DEV void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Epilogue of the even/odd product, run by the 16 epilogue warps of a CTA
@@ -812,6 +819,241 @@ gemm_sym_pair_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_const
   }
 }
 
+// The even/odd product where there are more tiles than SMs (batched solves):
+// one CTA per SM walks tiles t, t + grid, ... with two P/Q accumulators (all
+// 512 TMEM columns), so that a tile's epilogue runs under the next tile's
+// MMAs and the operand ring runs across tiles.  The tiles, their order of
+// accumulation and their stores are those of gemm_sym_bf16_kernel.  The ring
+// keeps its three 64 KiB stages; the epilogue's staging gets the remaining
+// 32 KiB, 8 columns per group and step, waiting for the stores before.  With
+// at most one tile per SM nothing overlaps and the other form's larger
+// staging ends sooner.
+constexpr int T_STAGES = 3, T_COLS = 8, kSMs = 148;
+constexpr int T_STG = 2 * 2 * 2 * T_COLS * 64 * 2;  // per group: 8 KiB, split boxes or FP32 boxes
+constexpr int T_SMEM = T_STAGES * SymCfg<64>::STAGE + EPI_GROUPS * T_STG + 1024 + 256;
+static_assert(T_STG == 2 * T_COLS * 128 * 4, "the FP32 boxes fill the same space");
+static_assert(T_SMEM <= 227 * 1024, "shared memory of a CTA");
+
+DEV void mbar_arrive(uint32_t a) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
+}
+
+__global__ void __launch_bounds__(S_THREADS, 1)
+gemm_sym_tiles_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
+                      const __grid_constant__ CUtensorMap mPh, const __grid_constant__ CUtensorMap mPl,
+                      const __grid_constant__ CUtensorMap mQh, const __grid_constant__ CUtensorMap mQl,
+                      const __grid_constant__ CUtensorMap mO0, const __grid_constant__ CUtensorMap mO1, int K,
+                      int ntn, int ntiles, Epi ep) {
+  using C = SymCfg<64>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* stg = smem + T_STAGES * C::STAGE;
+  uint64_t* bars = (uint64_t*)(stg + EPI_GROUPS * T_STG);  // full[S], empty[S], acc full[2], acc empty[2], done
+  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * T_STAGES + 5);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int KH = K >> 1, KT = K / BK;  // P and Q blocks alternate
+  auto full = [&](int s) { return smem_u32(&bars[s]); };
+  auto empty = [&](int s) { return smem_u32(&bars[T_STAGES + s]); };
+  auto accf = [&](int u) { return smem_u32(&bars[2 * T_STAGES + u]); };
+  auto acce = [&](int u) { return smem_u32(&bars[2 * T_STAGES + 2 + u]); };
+  const uint32_t done = smem_u32(&bars[2 * T_STAGES + 4]);
+  // tile t: columns n0 = 128 (t % ntn), rows 128 (t / ntn); its staggered start
+  auto shift = [&](int t) { return 2 * (int)(((unsigned)(t % ntn) * 5u + (unsigned)(t / ntn) * 3u) % (unsigned)(KT / 2)); };
+
+  if (threadIdx.x == 0) {
+    prefetch_map(&mAh); prefetch_map(&mAl); prefetch_map(&mPh);
+    prefetch_map(&mPl); prefetch_map(&mQh); prefetch_map(&mQl);
+    prefetch_map(&mO0); prefetch_map(&mO1);
+    for (int s = 0; s < T_STAGES; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+    for (int u = 0; u < 2; ++u) { mbar_init(accf(u), 1); mbar_init(acce(u), 4 * EPI_GROUPS); }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(4 * SBN));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0 && lane == 0) {
+    auto load_b = [&](int s, int kt, int n0) {
+      mbar_expect_tx(full(s), C::STAGE);
+      const uint32_t base = smem_u32(smem + s * C::STAGE);
+      const bool odd = kt & 1;
+      tma_load_2d(base + 2 * C::A_T, odd ? &mQh : &mPh, full(s), (kt >> 1) * BK, n0);
+      tma_load_2d(base + 2 * C::A_T + C::B_T, odd ? &mQl : &mPl, full(s), (kt >> 1) * BK, n0);
+    };
+    const int first = (int)blockIdx.x;
+    const int fill = ep.stall ? 0 : T_STAGES;  // K >= 256: at least four blocks per tile
+    for (int k = 0; k < fill; ++k) load_b(k, (k + shift(first)) % KT, (first % ntn) * SBN);
+    grid_dep_wait();
+    int s = 0, g = 0;
+    bool ok = !ep.stall;
+    for (int t = first; t < ntiles && ok; t += gridDim.x) {
+      const int n0 = (t % ntn) * SBN, m0 = (t / ntn) * BM, ks = shift(t);
+      for (int kt0 = 0; kt0 < KT; ++kt0, ++g) {
+        const int kt = (kt0 + ks) % KT;
+        if (g >= T_STAGES) {
+          ok = mbar_wait(empty(s), ((g / T_STAGES) - 1) & 1, abort_flag, ep.err, ep.wait_cycles);
+          if (!ok) break;
+          load_b(s, kt, n0);
+        }
+        const uint32_t base = smem_u32(smem + s * C::STAGE);
+        const int ac = ((kt & 1) ? KH : 0) + (kt >> 1) * BK;
+        tma_load_2d(base, &mAh, full(s), ac, m0);
+        tma_load_2d(base + C::A_T, &mAl, full(s), ac, m0);
+        s = s + 1 == T_STAGES ? 0 : s + 1;
+      }
+    }
+    drain_ring(full(0), T_STAGES, g);
+  } else if (warp == 1 && lane == 0) {
+    bool ok = true;
+    int s = 0, g = 0, i = 0;
+    for (int t = (int)blockIdx.x; t < ntiles && ok; t += gridDim.x, ++i) {
+      const int u = i & 1, ks = shift(t);
+      if (i >= 2) {
+        ok = mbar_wait(acce(u), ((i >> 1) - 1) & 1, abort_flag, ep.err, ep.wait_cycles);
+        if (!ok) break;
+      }
+      for (int kt0 = 0; kt0 < KT; ++kt0, ++g) {
+        ok = mbar_wait(full(s), (g / T_STAGES) & 1, abort_flag, ep.err, ep.wait_cycles);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t base = smem_u32(smem + s * C::STAGE);
+        const uint64_t ah = sdesc_sw128(base), al = sdesc_sw128(base + C::A_T);
+        const uint64_t bh = sdesc_sw128(base + 2 * C::A_T), bl = sdesc_sw128(base + 2 * C::A_T + C::B_T);
+        const uint32_t d = tmem + (uint32_t)(u * 2 * SBN) + (((kt0 + ks) & 1) ? (uint32_t)SBN : 0u);
+        const bool first = kt0 < 2;  // the first P block and the first Q block overwrite
+#pragma unroll
+        for (int kk = 0; kk < BK / 16; ++kk) {
+          const uint64_t o = (uint64_t)(kk * 32 >> 4);
+          umma_bf16<COLL_FILL>(d, ah + o, bh + o, kIdesc128, !(first && kk == 0));
+          umma_bf16<COLL_LASTUSE>(d, ah + o, bl + o, kIdesc128, 1u);
+          umma_bf16(d, al + o, bh + o, kIdesc128, 1u);
+        }
+        umma_commit(empty(s));
+        s = s + 1 == T_STAGES ? 0 : s + 1;
+      }
+      if (ok) umma_commit(accf(u));
+    }
+    umma_commit(done);
+  } else if (warp >= 2) {
+    const int wq = warp & 3, grp = (warp - 2) >> 2, cbeg = grp * EPI_COLS;
+    const int row = wq * 32 + lane, half = row & 1, rl = row >> 1;
+    const int R = ep.rows_per_batch;
+    const float alpha = (float)ep.alpha;
+    const bool scaled = ep.alpha != 1.0;
+    const bool issuer = lane == 0 && wq == 2;
+    uint8_t* box8 = stg + grp * T_STG;
+    const uint32_t sb = smem_u32(box8);
+    int i = 0;
+    // After an abort every wait returns at once and the loop runs out with
+    // its barriers, so that no warp is left waiting for another.
+    for (int t = (int)blockIdx.x; t < ntiles; t += gridDim.x, ++i) {
+      const int n0 = (t % ntn) * SBN, m0 = (t / ntn) * BM, u = i & 1;
+      const int bb = m0 / R, r0 = m0 - bb * R;
+      const float* ie = ep.inv_eig ? ep.inv_eig + (long long)(bb % ep.n_eig) * ep.n_cols * R + (r0 + row) : nullptr;
+      float ivp[T_COLS], ivm[T_COLS];  // 1/Lambda of a step, loaded a step ahead
+      auto load_iv = [&](int c0) {
+#pragma unroll
+        for (int j = 0; j < T_COLS; ++j) {
+          const int k = n0 + c0 + j;
+          ivp[j] = __ldg(ie + (long long)k * R);
+          ivm[j] = __ldg(ie + (long long)(K - 1 - k) * R);
+        }
+      };
+      if (ie) load_iv(cbeg);
+      bool ok = mbar_wait(accf(u), (i >> 1) & 1, abort_flag, ep.err, ep.wait_cycles);
+      ok = __all_sync(0xffffffffu, ok && !*abort_flag);
+      tc_fence_after();
+      if (t + (int)gridDim.x >= ntiles) grid_dep_launch();  // the last tile
+      const uint32_t acc = tmem + (uint32_t)(u * 2 * SBN) + ((uint32_t)(wq * 32) << 16);
+#pragma unroll 1
+      for (int sc = 0; sc < EPI_COLS; sc += T_COLS) {
+        const int c0 = cbeg + sc;
+        float xp[T_COLS], xm[T_COLS];
+        if (ok) {
+          uint32_t vp[T_COLS], vq[T_COLS];
+          tmem_ld8(acc + (uint32_t)c0, vp);
+          tmem_ld8(acc + (uint32_t)(SBN + c0), vq);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < T_COLS; ++j) {
+            const float P = __uint_as_float(vp[j]), Q = __uint_as_float(vq[j]);
+            xp[j] = P + Q;
+            xm[j] = P - Q;
+            if (scaled) { xp[j] *= alpha; xm[j] *= alpha; }
+            if (ie) { xp[j] *= ivp[j]; xm[j] *= ivm[j]; }
+          }
+          if (ie && sc + T_COLS < EPI_COLS) load_iv(c0 + T_COLS);
+        }
+        if (sc + T_COLS >= EPI_COLS) {  // this warp's part of the accumulator is read
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acce(u));
+        }
+        if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");  // the boxes are free
+        if (ok) {
+          if (ep.mode == EPI_SPLIT) {
+            bf16* box = (bf16*)box8;  // [which][half][hi/lo][8 n][64 r]
+            constexpr int BX = T_COLS * 64;
+#pragma unroll
+            for (int j = 0; j < T_COLS; ++j) {
+              const __nv_bfloat162 h2 = __floats2bfloat162_rn(xp[j], xm[j]);
+              const __nv_bfloat162 l2 = __floats2bfloat162_rn(xp[j] - __low2float(h2), xm[j] - __high2float(h2));
+              const int op = j * 64 + rl, om = (T_COLS - 1 - j) * 64 + rl;
+              box[((0 * 2 + half) * 2 + 0) * BX + op] = h2.x;
+              box[((0 * 2 + half) * 2 + 1) * BX + op] = l2.x;
+              box[((1 * 2 + half) * 2 + 0) * BX + om] = h2.y;
+              box[((1 * 2 + half) * 2 + 1) * BX + om] = l2.y;
+            }
+          } else {
+            float* box = (float*)box8;  // [which][8 n][128 r]
+#pragma unroll
+            for (int j = 0; j < T_COLS; ++j) {
+              box[j * 128 + row] = xp[j];
+              box[T_COLS * 128 + (T_COLS - 1 - j) * 128 + row] = xm[j];
+            }
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+        if (ok && issuer) {
+          const int ym = K - n0 - c0 - T_COLS;  // first mirrored column
+          if (ep.mode == EPI_SPLIT) {
+            for (int which = 0; which < 2; ++which)
+              for (int hf = 0; hf < 2; ++hf)
+                for (int hl = 0; hl < 2; ++hl)
+                  tma_store_3d(hl ? &mO1 : &mO0, sb + (uint32_t)(((which * 2 + hf) * 2 + hl) * T_COLS * 64 * 2),
+                               (hf ? (R >> 1) : 0) + (r0 >> 1), which ? ym : n0 + c0, bb);
+          } else {
+            tma_store_3d(&mO0, sb, r0, n0 + c0, bb);
+            tma_store_3d(&mO0, sb + (uint32_t)(T_COLS * 128 * 4), r0, ym, bb);
+          }
+          tma_store_commit();
+        }
+      }
+    }
+    // shared memory stays allocated until the stores have read it
+    if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    if (lane == 0) mbar_drain(done, 0);  // the MMAs issued before an abort have completed
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(4 * SBN));
+  }
+}
+
 #include "dst_fold.cuh"
 
 // ---- input split / copy / residual kernels ---------------------------------
@@ -1052,7 +1294,7 @@ static int gemm_split(const bf16* Xh, const bf16* Xl, int M, int K, const bf16* 
 // 3-D tensor map over an epilogue output [B][N][R] (R innermost, row pitch
 // ld, batch pitch bs, in elements), box {box_r, 128, 1}, no swizzle.
 static bool make_out_map(CUtensorMap* map, void* base, bool f32, uint64_t R, uint64_t N, uint64_t B, long long ld,
-                         long long bs, uint32_t box_r) {
+                         long long bs, uint32_t box_r, uint32_t box_n = 16) {
   auto enc = encode_fn();
   if (!enc) return false;
   const uint64_t es = f32 ? 4 : 2;
@@ -1060,7 +1302,7 @@ static bool make_out_map(CUtensorMap* map, void* base, bool f32, uint64_t R, uin
     return false;
   cuuint64_t dims[3] = {R, N, B};
   cuuint64_t strides[2] = {(cuuint64_t)ld * es, (cuuint64_t)(B > 1 ? bs : ld * (long long)N) * es};
-  cuuint32_t box[3] = {box_r, 16, 1};  // one 16-column step of an epilogue group
+  cuuint32_t box[3] = {box_r, box_n, 1};  // one step of an epilogue group
   cuuint32_t estr[3] = {1, 1, 1};
   return enc(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides,
              box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
@@ -1097,14 +1339,30 @@ static int gemm_sym(const bf16* Xh, const bf16* Xl, int M, int K, const bf16* Ph
   memset(&o1, 0, sizeof(o1));
   ep.tma_out = 0;
   const int R = ep.rows_per_batch;
+  // More tiles than SMs: the form that runs a tile's epilogue under the next
+  // tile's MMAs.  A batch of 16 solves of 1024^2 (512 tiles, 3.5 per SM)
+  // takes 279 us against 330 with a CTA per tile, 4 of 2048^2 451 against
+  // 505.  Up to one tile per SM nothing overlaps (16 of 512^2, 128 tiles).
+  const long long tiles = (long long)(KH / SBN) * ((M + BM - 1) / BM);
+  bool walk = g_sym_kernel == 0 && tiles > kSMs && tiles <= INT_MAX;
+  const uint32_t box_n = walk ? T_COLS : 16;
   if ((ep.mode == EPI_SPLIT || ep.mode == EPI_F32) && R % BM == 0 && M % R == 0 && ep.off_n == 0 &&
       ep.off_r == 0 && ep.n_cols == K && (ep.mode == EPI_F32 || ep.perm_r)) {
     const uint64_t B = (uint64_t)(M / R);
     bool okm = ep.mode == EPI_SPLIT
-                   ? make_out_map(&o0, ep.out0, false, R, K, B, ep.ld, ep.batch_stride, 64) &&
-                         make_out_map(&o1, ep.out1, false, R, K, B, ep.ld, ep.batch_stride, 64)
-                   : make_out_map(&o0, ep.out0, true, R, K, B, ep.ld, ep.batch_stride, 128);
+                   ? make_out_map(&o0, ep.out0, false, R, K, B, ep.ld, ep.batch_stride, 64, box_n) &&
+                         make_out_map(&o1, ep.out1, false, R, K, B, ep.ld, ep.batch_stride, 64, box_n)
+                   : make_out_map(&o0, ep.out0, true, R, K, B, ep.ld, ep.batch_stride, 128, box_n);
     ep.tma_out = okm ? 1 : 0;
+  }
+  if (walk && ep.tma_out) {
+    static fvx_once_per_device tattr;
+    if (fvx_once_on_device(tattr, [] { return fvx_set_max_smem(gemm_sym_tiles_kernel, T_SMEM); }))
+      return FVX_ERR_CUDA;
+    if (fvx_launch_pdl(gemm_sym_tiles_kernel, dim3(kSMs), dim3(S_THREADS), T_SMEM, st, a_h, a_l, p_h, p_l, q_h, q_l, o0,
+                       o1, K, KH / SBN, (int)tiles, ep) != cudaSuccess)
+      return FVX_ERR_CUDA;
+    return fvx_cuda_status();
   }
   if (M % (2 * BM) == 0 && g_sym_kernel == 1) {
     // CTA pairs: B blocks of 64 table rows per CTA
