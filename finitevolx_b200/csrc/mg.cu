@@ -776,6 +776,262 @@ up_leg_kernel(Lev<T> L, const T* f, const T* u_pre, Lev<T> C, const T* ec, int k
   }
 }
 
+// ---------------------------------------------------------------------------
+// The coarse part of a V-cycle in one CTA, resident in shared memory: levels
+// l0 .. nl-1 entered with f[l0] set and a zero initial guess, u[l0] left with
+// the result.  Every level's arrays (padded by a ring of zeros, so that no
+// neighbour needs a test) are loaded before the wait for the kernel that
+// wrote f; a sweep then costs a barrier, shared reads of the neighbours and
+// register arithmetic.  A chain of dependent sweeps bounds it: 24 FP32 sweeps
+// over global memory took 11 us of a 512^2 problem's coarse part, the 50
+// coarsest ones 10.5.  With R rows per thread an FP32 plan takes the levels
+// up to 64 x 64, whose two legs cost more than the 12 sweeps here.  A 512^2
+// FP32 V-cycle took 98.0 us and takes 82.5.  The arithmetic of every cell is
+// the legs' (jac_v), the coarsest sweeps run in E.
+// ---------------------------------------------------------------------------
+template <typename T> struct CoarseRows { static constexpr int R = sizeof(T) == 4 ? 4 : 1; };
+constexpr size_t kResidentSmem = 224 * 1024;
+
+__host__ __device__ inline size_t padded_cells(int ny, int nx) { return (size_t)(ny + 2) * (nx + 2); }
+// Rows per thread of an ny x nx level (columns on consecutive threads).
+__host__ __device__ inline int coarse_rows(int ny, int nx) {
+  const int nseg = kCoarseThreads / nx;
+  return nseg > 0 ? (ny + nseg - 1) / nseg : 1 << 20;
+}
+
+template <typename T> struct ResLev {
+  T *u, *v, *f, *w, *cx, *cy, *m;
+};
+template <typename T> DEV ResLev<T> res_lev(T* base, size_t P) {
+  return ResLev<T>{base, base + P, base + 2 * P, base + 3 * P, base + 4 * P, base + 5 * P, base + 6 * P};
+}
+
+// k sweeps of a level from the values in A (and s.u); the thread owns rows
+// r0 .. of column c, its first cell at p.  Returns the buffer of the result.
+template <typename T, int R> struct ResCells {
+  T u[R], f[R], w[R], cx[R], cxw[R], cy[R], cys0;
+};
+template <typename T, int R>
+DEV void res_load(const ResLev<T>& V, const T* A, ResCells<T, R>& s, int p, int pitch, int rows) {
+  s.cys0 = rows > 0 ? V.cy[p - pitch] : T(0);
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int q = i < rows ? p + i * pitch : 0;  // cell 0 is on the ring of zeros
+    s.u[i] = A[q];
+    s.f[i] = V.f[q];
+    s.w[i] = V.w[q];
+    s.cx[i] = V.cx[q];
+    s.cxw[i] = i < rows ? V.cx[q - 1] : T(0);
+    s.cy[i] = V.cy[q];
+  }
+}
+template <typename T, int R>
+DEV T* res_sweeps(const Lev<T>& L, ResCells<T, R>& s, T* A, T* B, int k, int p, int pitch, int rows) {
+  for (int sw = 0; sw < k; ++sw) {
+    if (rows > 0) {
+      T us = A[p - pitch], cys = s.cys0;
+      const T top = A[p + rows * pitch];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        if (i < rows) {
+          const int q = p + i * pitch;
+          const T um = s.u[i], un = i + 1 < rows ? s.u[i + 1 < R ? i + 1 : i] : top;
+          const T nv = jac_v(um, A[q + 1], A[q - 1], un, us, s.cx[i], s.cxw[i], s.cy[i], cys, s.f[i], s.w[i], L.dx2,
+                             L.rdx2, L.dy2, L.rdy2, L.lam);
+          us = um;
+          cys = s.cy[i];
+          s.u[i] = nv;
+          B[q] = nv;
+        }
+      }
+    }
+    __syncthreads();
+    T* t = A;
+    A = B;
+    B = t;
+  }
+  return A;
+}
+
+template <typename T, typename E, int R>
+__global__ void __launch_bounds__(kCoarseThreads)
+coarse_resident_kernel(LevArray<T> G, Lev<E> D, int l0, int nl, int n_pre, int n_post, int n_coarse, T omega) {
+  __shared__ Lev<T> S[kMaxLevels];
+  extern __shared__ __align__(16) unsigned char res_raw[];
+  const int tid = threadIdx.x;
+  if (tid < nl) S[tid] = G.L[tid];
+  const int last = nl - 1;
+  // the coarsest solve's arrays first (E is the wider type), then the levels
+  E* e0 = (E*)res_raw;
+  const size_t PE = padded_cells(D.ny, D.nx);
+  E *ea = e0, *eb = e0 + PE, *ecx = e0 + 2 * PE, *ecy = e0 + 3 * PE, *ew = e0 + 4 * PE;
+  T* lev0 = (T*)(e0 + 5 * PE);
+  __syncthreads();
+  for (int q = tid; q < (int)PE; q += kCoarseThreads) {
+    const int pitch = D.nx + 2, j = q / pitch - 1, i = q - (j + 1) * pitch - 1;
+    const bool in = j >= 0 && j < D.ny && i >= 0 && i < D.nx;
+    const size_t c = in ? (size_t)j * D.nx + i : 0;
+    ea[q] = E(0);
+    eb[q] = E(0);
+    ecx[q] = in ? D.cx[c] : E(0);
+    ecy[q] = in ? D.cy[c] : E(0);
+    ew[q] = in ? (E)omega * D.inv[c] : E(0);
+  }
+  {
+    T* base = lev0;
+    for (int l = l0; l < nl; ++l) {
+      const Lev<T> L = S[l];
+      const size_t P = padded_cells(L.ny, L.nx);
+      const ResLev<T> V = res_lev(base, P);
+      const int pitch = L.nx + 2;
+#pragma unroll 2
+      for (int q = tid; q < (int)P; q += kCoarseThreads) {
+        const int j = q / pitch - 1, i = q - (j + 1) * pitch - 1;
+        const bool in = j >= 0 && j < L.ny && i >= 0 && i < L.nx;
+        const size_t c = in ? (size_t)j * L.nx + i : 0;
+        const T m = in ? L.mask[c] : T(0), cx = in ? L.cx[c] : T(0), cy = in ? L.cy[c] : T(0),
+                w = in ? L.inv[c] : T(0);
+        V.u[q] = T(0);
+        V.v[q] = T(0);
+        V.f[q] = T(0);
+        V.w[q] = omega * w;
+        V.cx[q] = cx;
+        V.cy[q] = cy;
+        V.m[q] = m;
+      }
+      base += 7 * P;
+    }
+  }
+  grid_dep_wait();
+  __syncthreads();
+  // the thread's cells of a level: rows r0 .. r0 + rows - 1 of column c
+  auto own = [&](const Lev<T>& L, int& c, int& r0, int& rows) {
+    const int LR = coarse_rows(L.ny, L.nx), seg = tid / L.nx;
+    c = tid - seg * L.nx;
+    r0 = seg * LR;
+    rows = r0 >= L.ny ? 0 : (L.ny - r0 < LR ? L.ny - r0 : LR);
+  };
+  {  // f of the first level
+    const Lev<T> L = S[l0];
+    const ResLev<T> V = res_lev(lev0, padded_cells(L.ny, L.nx));
+    int c, r0, rows;
+    own(L, c, r0, rows);
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (i < rows) V.f[(r0 + i + 1) * (L.nx + 2) + c + 1] = __ldcg(L.f + (size_t)(r0 + i) * L.nx + c);
+  }
+  grid_dep_launch();
+  __syncthreads();
+  T* base = lev0;
+  for (int l = l0; l < last; ++l) {
+    const Lev<T> L = S[l];
+    const size_t P = padded_cells(L.ny, L.nx);
+    const ResLev<T> V = res_lev(base, P);
+    const int pitch = L.nx + 2;
+    int c, r0, rows;
+    own(L, c, r0, rows);
+    const int p = (r0 + 1) * pitch + c + 1;
+    ResCells<T, R> s;
+    res_load<T, R>(V, V.u, s, p, pitch, rows);
+    T* A = res_sweeps<T, R>(L, s, V.u, V.v, n_pre, p, pitch, rows);
+    T* B = A == V.u ? V.v : V.u;
+    // r * mask into B (the legs' form), then the restricted residual
+    if (rows > 0) {
+      T us = A[p - pitch], cys = s.cys0;
+      const T top = A[p + rows * pitch];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        if (i < rows) {
+          const int q = p + i * pitch;
+          const T um = s.u[i], un = i + 1 < rows ? s.u[i + 1 < R ? i + 1 : i] : top;
+          const T ue = A[q + 1], uw = A[q - 1], mc = V.m[q];
+          const T lap = divd(s.cx[i] * (ue - um) - s.cxw[i] * (um - uw), L.dx2, L.rdx2) +
+                        divd(s.cy[i] * (un - um) - cys * (um - us), L.dy2, L.rdy2);
+          B[q] = ((s.f[i] - (lap - L.lam * um) * mc) * mc) * mc;
+          us = um;
+          cys = s.cy[i];
+        }
+      }
+    }
+    __syncthreads();
+    base += 7 * P;
+    const Lev<T> C = S[l + 1];
+    const ResLev<T> W = res_lev(base, padded_cells(C.ny, C.nx));
+    for (int q = tid; q < C.ny * C.nx; q += kCoarseThreads) {
+      const int J = q / C.nx, I = q - J * C.nx;
+      const int k = (2 * J + 1) * pitch + 2 * I + 1, kc = (J + 1) * (C.nx + 2) + I + 1;
+      const T sum4 = ((B[k] + B[k + pitch]) + B[k + 1]) + B[k + pitch + 1];
+      const T cnt = ((V.m[k] + V.m[k + pitch]) + V.m[k + 1]) + V.m[k + pitch + 1];
+      W.f[kc] = (sum4 / (cnt > T(1) ? cnt : T(1))) * W.m[kc];
+    }
+    __syncthreads();
+  }
+  {  // the coarsest solve: one cell per thread of the warps that hold any
+    const int nx = D.nx, cells = D.ny * nx, pitch = nx + 2;
+    const ResLev<T> V = res_lev(base, padded_cells(D.ny, nx));
+    const int nthr = (cells + 31) & ~31;
+    if (tid < nthr) {
+      const bool live = tid < cells;
+      const int j = live ? tid / nx : 0, i = live ? tid - j * nx : 0, q = (j + 1) * pitch + i + 1;
+      const E cx = ecx[q], cxw = ecx[q - 1], cy = ecy[q], cys = ecy[q - pitch], w = ew[q], f = (E)V.f[q];
+      E um = E(0);
+      E *a = ea, *b = eb;
+      for (int sw = 0; sw < n_coarse; ++sw) {
+        um = jac_v(um, a[q + 1], a[q - 1], a[q + pitch], a[q - pitch], cx, cxw, cy, cys, f, w, D.dx2, D.rdx2, D.dy2,
+                   D.rdy2, D.lam);
+        if (live) b[q] = um;
+        asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+        E* t = a;
+        a = b;
+        b = t;
+      }
+      if (live) V.u[q] = (T)um;
+    }
+    __syncthreads();
+  }
+  const T* ec = res_lev(base, padded_cells(D.ny, D.nx)).u;
+  for (int l = last - 1; l >= l0; --l) {
+    const Lev<T> L = S[l], C = S[l + 1];
+    const ResLev<T> W = res_lev(base, padded_cells(C.ny, C.nx));
+    const size_t P = padded_cells(L.ny, L.nx);
+    base -= 7 * P;
+    const ResLev<T> V = res_lev(base, P);
+    const int pitch = L.nx + 2, cp = C.nx + 2;
+    int c, r0, rows;
+    own(L, c, r0, rows);
+    const int p = (r0 + 1) * pitch + c + 1;
+    T* A = (n_pre & 1) ? V.v : V.u;
+    ResCells<T, R> s;
+    res_load<T, R>(V, A, s, p, pitch, rows);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (i < rows) {
+        const int r = r0 + i, sj = (2 * (r & 1) - 1) * cp, si = 2 * (c & 1) - 1;
+        const int k = ((r >> 1) + 1) * cp + (c >> 1) + 1;
+        auto val = [&](int kk) -> T { return ec[kk] * W.m[kk]; };
+        const T ws = ((T(9) * val(k) + T(3) * val(k + si)) + T(3) * val(k + sj)) + T(1) * val(k + sj + si);
+        const T ds = ((T(9) * W.m[k] + T(3) * W.m[k + si]) + T(3) * W.m[k + sj]) + T(1) * W.m[k + sj + si];
+        const T mf = V.m[p + i * pitch];
+        const T e = (ws / (ds > T(1) ? ds : T(1))) * mf;
+        s.u[i] = (s.u[i] + e) * mf;
+        A[p + i * pitch] = s.u[i];
+      }
+    }
+    __syncthreads();
+    ec = res_sweeps<T, R>(L, s, A, A == V.u ? V.v : V.u, n_post, p, pitch, rows);
+    if (l == l0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (i < rows) L.u[(size_t)(r0 + i) * L.nx + c] = s.u[i];
+    }
+  }
+  if (l0 == last)
+    for (int q = tid; q < D.ny * D.nx; q += kCoarseThreads) {
+      const int j = q / D.nx, i = q - j * D.nx;
+      S[l0].u[q] = ec[(j + 1) * (D.nx + 2) + i + 1];
+    }
+}
+
 // masked_laplacian (iterative.py:144-191): periodic roll, (lap - lam psi_m) * m
 template <typename T>
 __global__ void masked_laplacian_kernel(const T* psi, const T* m, T* out, int ny, int nx, T dx, T dy, T lam) {
@@ -806,6 +1062,7 @@ struct fvx_mg {
   int nl = 0, lc = 0, n_pre = 6, n_post = 6, n_coarse = 50, dtype = 0;
   double* omega_scratch = nullptr;  // [2 * kOmegaBlocks partials, omega], ticket after it
   double omega = 0.95, lam = 0.0;
+  bool mask01 = true;  // the caller's mask is 0 / 1 (the coarser ones always are)
   std::vector<void*> allocs;
   LevArray<float> A32;
   LevArray<double> A64;  // FP64 plans: every level; FP32 plans: the coarsest level only
@@ -929,6 +1186,8 @@ extern "C" int fvx_mg_create(const double* mask, const double* coeff, int ny, in
   fvx_mg* g = new fvx_mg();
   g->nl = n_levels; g->n_pre = n_pre; g->n_post = n_post; g->n_coarse = n_coarse;
   g->omega = omega; g->lam = lambda; g->dtype = dtype;
+  for (size_t c = 0; c < n0; ++c)
+    if (mask[c] != 0.0 && mask[c] != 1.0) g->mask01 = false;
   g->lc = n_levels - 1;
   while (g->lc > 0 && (size_t)H[g->lc - 1].ny * H[g->lc - 1].nx <= (size_t)kCoarseCells) --g->lc;
   int rc = dtype == 0 ? upload_levels<float>(g, H) : upload_levels<double>(g, H);
@@ -1021,9 +1280,46 @@ static int leg_attr() {
   });
 }
 
-// The single-CTA coarse V-cycle from level l (FP32 plans: in FP64).
+// Shared memory of coarse_resident_kernel over levels l .. nl-1, 0 where it
+// does not take them.
+template <typename T>
+static size_t resident_smem(fvx_mg* g, int l) {
+  const LevArray<T>& A = levs<T>(g);
+  const Lev<T>& last = A.L[g->nl - 1];
+  if (last.ny * (long long)last.nx > kCoarseThreads || (l == 0 && !g->mask01)) return 0;
+  size_t bytes = 5 * padded_cells(last.ny, last.nx) * sizeof(double);
+  for (int k = l; k < g->nl; ++k) {
+    if (k < g->nl - 1 && coarse_rows(A.L[k].ny, A.L[k].nx) > CoarseRows<T>::R) return 0;
+    bytes += 7 * padded_cells(A.L[k].ny, A.L[k].nx) * sizeof(T);
+  }
+  return bytes <= kResidentSmem ? bytes : 0;
+}
+// First level (>= 1) that the V-cycle's single CTA starts at: the resident
+// form reaches further up than kCoarseCells where its registers and shared
+// memory allow.
+template <typename T>
+static int resident_first(fvx_mg* g) {
+  int l = g->lc;
+  while (l > 1 && resident_smem<T>(g, l - 1)) --l;
+  return l;
+}
+
+// The single-CTA coarse V-cycle from level l (FP32 plans: in FP64).  Levels
+// that do not fit shared memory (a large coarsest grid) run over global memory.
 template <typename T>
 static int coarse_vcycle(fvx_mg* g, int l, cudaStream_t st) {
+  if (const size_t bytes = resident_smem<T>(g, l)) {
+    constexpr int R = CoarseRows<T>::R;
+    static fvx_once_per_device attr;
+    if (fvx_once_on_device(attr, [] {
+          return fvx_set_max_smem(coarse_resident_kernel<T, double, R>, (int)kResidentSmem);
+        }))
+      return FVX_ERR_CUDA;
+    if (fvx_launch_pdl(coarse_resident_kernel<T, double, R>, dim3(1), dim3(kCoarseThreads), bytes, st, levs<T>(g),
+                       g->A64.L[g->nl - 1], l, g->nl, g->n_pre, g->n_post, g->n_coarse, (T)g->omega) != cudaSuccess)
+      return FVX_ERR_CUDA;
+    return fvx_cuda_status();
+  }
   if constexpr (sizeof(T) == 4)
     coarse_vcycle_f64_kernel<<<1, kCoarseThreads, 0, st>>>(g->A32, g->A64.L[g->nl - 1], l, g->nl, g->n_pre,
                                                            g->n_post, g->n_coarse, (float)g->omega);
@@ -1097,7 +1393,7 @@ template <typename T>
 static int vcycle_levels(fvx_mg* g, int l, T** result, cudaStream_t st) {
   LevArray<T>& A = levs<T>(g);
   const T om = (T)g->omega;
-  if (l >= g->lc) {
+  if (l >= resident_first<T>(g)) {
     *result = A.L[l].u;
     return coarse_vcycle<T>(g, l, st);
   }
