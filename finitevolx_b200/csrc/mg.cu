@@ -81,8 +81,22 @@ DEV bool pcg_last_block(unsigned* ticket) {
   return last;
 }
 
+// a / d for a divisor whose correctly rounded reciprocal r is at hand: the
+// quotient estimate a r corrected twice by its exact remainder, which rounds
+// correctly (Markstein's theorem, IBM J. Res. Dev. 34 (1990) 111: a quotient
+// within one unit in the last place plus remainder times RN(1/d)).  Zero
+// numerators (masked cells) take it too; the built-in division sends their
+// whole warp through its slow path.  Exponents outside +-400, where a
+// remainder could underflow, and non-finite values divide plainly.
+DEV double div_by(double a, double d, double r) {
+  const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, ed = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+  if ((ea - 623u > 800u && a != 0.0) || ed - 623u > 800u) return a / d;
+  const double q0 = a * r;
+  const double q1 = __fma_rn(__fma_rn(-q0, d, a), r, q0);
+  return __fma_rn(__fma_rn(-q1, d, a), r, q1);
+}
 template <typename T> DEV T divd(T a, T d2, T rd2) {
-  if constexpr (sizeof(T) == 8) return a / d2;
+  if constexpr (sizeof(T) == 8) return div_by(a, d2, rd2);
   else return a * rd2;
 }
 

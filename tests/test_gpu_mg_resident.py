@@ -56,3 +56,17 @@ def test_fractional_mask_small_grid(cuda_ok):
     ref = O.mg_vcycle(O.mg_build(m, 1.0, 1.0, lambda_=0.1), np.zeros_like(f), f)
     got = MultigridSolver(m, 1.0, 1.0, lambda_=0.1).v_cycle(None, torch.tensor(f, device="cuda")).cpu().numpy()
     assert np.linalg.norm(got - ref) <= 1e-11 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("k", [-600, -360, 360, 600])
+def test_fp64_quotients_scale_exactly(cuda_ok, k):
+    # the operator is linear, so a right-hand side scaled by a power of two
+    # scales every intermediate exactly: quotients formed by multiplication
+    # and remainder (exponents within +-400) and plainly divided ones (beyond)
+    # have to agree to the last bit
+    m, c, f = problem(128, 128)
+    mg = MultigridSolver(m, 1.3, 0.9, lambda_=0.02, coeff=c)
+    fd = torch.tensor(f, device="cuda")
+    scale = 2.0 ** k
+    assert torch.equal(mg.v_cycle(None, fd * scale), mg.v_cycle(None, fd) * scale)
+    assert torch.equal(mg.apply(fd * scale), mg.apply(fd) * scale)
