@@ -10,8 +10,8 @@
 // solve_cg (iterative.py:48-136).
 //
 // Device layout per level: mask, cx, cy, inv_diag, u, f, tmp (T = float or
-// double, row-major [ny, nx]).  Levels at or below kCoarseCells cells run
-// inside one CTA (one launch for the whole coarse part of the V-cycle);
+// double, row-major [ny, nx]).  The coarse levels (FP32: up to
+// 64 x 64) run inside one CTA, one launch for the V-cycle's whole coarse part;
 // finer levels use one launch per leg (all of its sweeps and the transfer).
 #include "fvx_common.cuh"
 
@@ -87,7 +87,9 @@ DEV bool pcg_last_block(unsigned* ticket) {
 // within one unit in the last place plus remainder times RN(1/d)).  Zero
 // numerators (masked cells) take it too; the built-in division sends their
 // whole warp through its slow path.  Exponents outside +-400, where a
-// remainder could underflow, and non-finite values divide plainly.
+// remainder could underflow, and non-finite values divide plainly.  An FP64
+// V-cycle at 512^2 took 213 us with built-in divisions and 160 with these, a
+// coarsest sweep over a masked grid 0.52 us and 0.18.
 DEV double div_by(double a, double d, double r) {
   const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu, ed = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
   if ((ea - 623u > 800u && a != 0.0) || ed - 623u > 800u) return a / d;
@@ -472,9 +474,16 @@ constexpr int kOmegaBlocks = 64;
 constexpr int kLegMaxSweeps = 16;
 constexpr int kLegFewTiles = 148;  // legs with fewer tiles use more threads per CTA
 
-template <typename T> struct LegTile;
-template <> struct LegTile<float> { static constexpr int TX = 64, TY = 32; };
-template <> struct LegTile<double> { static constexpr int TX = 32, TY = 16; };
+// V = 0: the throughput tile; V = 1: a quarter of it, for levels with so few
+// tiles that most SMs idle (kLegQuarter): the halo is recomputed more often,
+// but each CTA's sweeps are half as long.  FP32 V-cycle at 512^2 (quarters on
+// 256^2 and 128^2): 83 us without, 74 with; FP64 (down to 64^2): 160 and 143.
+template <typename T, int V> struct LegTile;
+template <> struct LegTile<float, 0> { static constexpr int TX = 64, TY = 32; };
+template <> struct LegTile<float, 1> { static constexpr int TX = 32, TY = 16; };
+template <> struct LegTile<double, 0> { static constexpr int TX = 32, TY = 16; };
+template <> struct LegTile<double, 1> { static constexpr int TX = 16, TY = 8; };
+constexpr int kLegQuarter = 37;  // tiles at most: their quarters are one per SM
 
 // One weighted-Jacobi update of a cell from its own and its neighbours'
 // values: jacobi_at's arithmetic with the multiplications by the 0/1 mask
@@ -494,11 +503,11 @@ DEV T jac_v(T um, T ue, T uw, T un, T us, T cx, T cxw, T cy, T cys, T f, T winv,
 struct LegShape {
   int RW, RH, RN, LR;  // LR: rows per thread
 };
-template <typename T>
+template <typename T, int V>
 __host__ __device__ inline LegShape leg_shape(int H, int nt) {
   LegShape g;
-  g.RW = LegTile<T>::TX + 2 * H;
-  g.RH = LegTile<T>::TY + 2 * H;
+  g.RW = LegTile<T, V>::TX + 2 * H;
+  g.RH = LegTile<T, V>::TY + 2 * H;
   g.RN = g.RW * g.RH;
   const int nseg = nt / g.RW;
   g.LR = nseg > 0 ? (g.RH + nseg - 1) / nseg : 1 << 20;
@@ -520,9 +529,9 @@ __host__ __device__ inline CoarseWin coarse_win(int x0, int y0, int RW, int RH) 
 
 // Shared memory of a leg with k sweeps (both kinds): cx and two u buffers
 // over the halo-(k + 1) region, and the up leg's coarse window (twice).
-template <typename T>
+template <typename T, int V>
 static size_t leg_smem(int k) {
-  const LegShape g = leg_shape<T>(k + 1, 1);
+  const LegShape g = leg_shape<T, V>(k + 1, 1);
   const size_t CN = (size_t)((g.RW + 1) / 2 + 3) * ((g.RH + 1) / 2 + 3);
   return (3 * (size_t)g.RN + 2 * CN) * sizeof(T);
 }
@@ -608,12 +617,12 @@ DEV T* leg_sweeps(const Lev<T>& L, LegCells<T, R>& s, T* A, T* B, const T* scx, 
 // u_pre, ec, ec_scale) is read only after grid_dep_wait, through L2
 // (ld.global.cg), from pointers not marked __restrict__ -- a restrict-const
 // load may be served by the read-only path or moved above the wait.
-template <typename T, int NT, int R>
+template <typename T, int V, int NT, int R>
 __global__ void __launch_bounds__(NT)
 down_leg_kernel(Lev<T> L, const T* f, const T* u_init, int k, T omega, Lev<T> C) {
-  constexpr int TX = LegTile<T>::TX, TY = LegTile<T>::TY;
+  constexpr int TX = LegTile<T, V>::TX, TY = LegTile<T, V>::TY;
   const int H = k + 1;
-  const LegShape g = leg_shape<T>(H, NT);
+  const LegShape g = leg_shape<T, V>(H, NT);
   const int RW = g.RW, RH = g.RH, LR = g.LR;
   extern __shared__ __align__(16) unsigned char leg_raw[];
   T* scx = (T*)leg_raw;
@@ -714,16 +723,16 @@ down_leg_kernel(Lev<T> L, const T* f, const T* u_init, int k, T omega, Lev<T> C)
 // out (tile) <- k sweeps from u_pre + P ec.  Halo k.
 // ec_scale (may be null): the coarse correction is read as ec * (T)*ec_scale
 // (the hybrid cycle's energy-optimal scaling, applied as the window loads).
-template <typename T, int NT, int R>
+template <typename T, int V, int NT, int R>
 __global__ void __launch_bounds__(NT)
 up_leg_kernel(Lev<T> L, const T* f, const T* u_pre, Lev<T> C, const T* ec, int k, T omega, T* __restrict__ out,
               const double* ec_scale) {
-  constexpr int TX = LegTile<T>::TX, TY = LegTile<T>::TY;
+  constexpr int TX = LegTile<T, V>::TX, TY = LegTile<T, V>::TY;
   const int H = k;
-  const LegShape g = leg_shape<T>(H, NT);
+  const LegShape g = leg_shape<T, V>(H, NT);
   const int RW = g.RW, RH = g.RH, LR = g.LR;
   // the buffer layout of leg_smem(k) (sized for halo k + 1)
-  const int RNmax = leg_shape<T>(k + 1, 1).RN;
+  const int RNmax = leg_shape<T, V>(k + 1, 1).RN;
   extern __shared__ __align__(16) unsigned char leg_raw[];
   T* scx = (T*)leg_raw;
   T* A = scx + RNmax;
@@ -770,9 +779,9 @@ up_leg_kernel(Lev<T> L, const T* f, const T* u_pre, Lev<T> C, const T* ec, int k
     T u = T(0);
     if (in) {
       const int J = gy >> 1, I = gx >> 1, sj = 2 * (gy & 1) - 1, si = 2 * (gx & 1) - 1;
-      auto V = [&](int jj, int ii) -> T { return sv[(jj - cw.CY0) * cw.CW + (ii - cw.CX0)]; };
+      auto val = [&](int jj, int ii) -> T { return sv[(jj - cw.CY0) * cw.CW + (ii - cw.CX0)]; };
       auto M = [&](int jj, int ii) -> T { return scm[(jj - cw.CY0) * cw.CW + (ii - cw.CX0)]; };
-      const T ws = ((T(9) * V(J, I) + T(3) * V(J, I + si)) + T(3) * V(J + sj, I)) + T(1) * V(J + sj, I + si);
+      const T ws = ((T(9) * val(J, I) + T(3) * val(J, I + si)) + T(3) * val(J + sj, I)) + T(1) * val(J + sj, I + si);
       const T ds = ((T(9) * M(J, I) + T(3) * M(J, I + si)) + T(3) * M(J + sj, I)) + T(1) * M(J + sj, I + si);
       const T e = (ws / (ds > T(1) ? ds : T(1))) * mf;
       u = (up[i] + e) * mf;
@@ -1269,29 +1278,69 @@ extern "C" int fvx_mg_num_levels(fvx_mg* g) { return g ? g->nl : -1; }
 // one CTA of 32 warps per SM); FP64 prefers 512 x 4 (1024 x 4 would spill),
 // except on levels with fewer tiles than SMs, where more threads per tile
 // shorten each CTA's sweeps.
-constexpr int kLegNT[4] = {512, 512, 1024, 1024}, kLegR[4] = {4, 8, 4, 8};
+// Quarter tiles take 1024 x 2 (4), or 1024 x 4 (5) with many sweeps.
+constexpr int kLegNT[6] = {512, 512, 1024, 1024, 1024, 1024}, kLegR[6] = {4, 8, 4, 8, 2, 4};
 template <typename T>
-static int leg_config(int H, bool few) {
+static int leg_config(int H, bool few, bool quarter) {
+  if (quarter) {
+    for (int i = 4; i < 6; ++i)
+      if (leg_shape<T, 1>(H, kLegNT[i]).LR <= kLegR[i]) return i;
+  }
   static constexpr int order32[4] = {2, 3, 1, 0}, order64[4] = {0, 1, 2, 3}, order_few[4] = {2, 3, 0, 1};
   const int* order = few ? order_few : (sizeof(T) == 4 ? order32 : order64);
   for (int j = 0; j < 4; ++j) {
     const int i = order[j];
-    if (leg_shape<T>(H, kLegNT[i]).LR <= kLegR[i]) return i;
+    if (leg_shape<T, 0>(H, kLegNT[i]).LR <= kLegR[i]) return i;
   }
   return -1;
 }
 
-template <typename T>
-static int leg_attr() {
+// Launches of one configuration, as programmatic dependents: the constants
+// load while the kernel before finishes (the kernels wait before reading f
+// and u).  Attributes are set on first use, so that only the configurations
+// that run are loaded.
+template <typename T, int V, int NT, int R>
+static int launch_down(dim3 gr, size_t sm, cudaStream_t st, const Lev<T>& L, const T* f, const T* u_init, int k, T om,
+                       const Lev<T>& C) {
   static fvx_once_per_device attr;
-  return fvx_once_on_device(attr, [] {
-    const int bytes = (int)leg_smem<T>(kLegMaxSweeps);
-    return fvx_set_max_smem(down_leg_kernel<T, 512, 4>, bytes) && fvx_set_max_smem(down_leg_kernel<T, 512, 8>, bytes) &&
-           fvx_set_max_smem(down_leg_kernel<T, 1024, 4>, bytes) &&
-           fvx_set_max_smem(down_leg_kernel<T, 1024, 8>, bytes) && fvx_set_max_smem(up_leg_kernel<T, 512, 4>, bytes) &&
-           fvx_set_max_smem(up_leg_kernel<T, 512, 8>, bytes) && fvx_set_max_smem(up_leg_kernel<T, 1024, 4>, bytes) &&
-           fvx_set_max_smem(up_leg_kernel<T, 1024, 8>, bytes);
-  });
+  if (fvx_once_on_device(attr, [] {
+        return fvx_set_max_smem(down_leg_kernel<T, V, NT, R>, (int)leg_smem<T, V>(kLegMaxSweeps));
+      }))
+    return FVX_ERR_CUDA;
+  if (fvx_launch_pdl(down_leg_kernel<T, V, NT, R>, gr, dim3(NT), sm, st, L, f, u_init, k, om, C) != cudaSuccess)
+    return FVX_ERR_CUDA;
+  return fvx_cuda_status();
+}
+template <typename T, int V, int NT, int R>
+static int launch_up(dim3 gr, size_t sm, cudaStream_t st, const Lev<T>& L, const T* f, const T* up, const Lev<T>& C,
+                     const T* ec, int k, T om, T* out, const double* ec_scale) {
+  static fvx_once_per_device attr;
+  if (fvx_once_on_device(attr, [] {
+        return fvx_set_max_smem(up_leg_kernel<T, V, NT, R>, (int)leg_smem<T, V>(kLegMaxSweeps));
+      }))
+    return FVX_ERR_CUDA;
+  if (fvx_launch_pdl(up_leg_kernel<T, V, NT, R>, gr, dim3(NT), sm, st, L, f, up, C, ec, k, om, out, ec_scale) !=
+      cudaSuccess)
+    return FVX_ERR_CUDA;
+  return fvx_cuda_status();
+}
+
+// Configuration, grid and shared memory of the legs of level L with k sweeps.
+struct LegPlan {
+  int cfg;
+  dim3 grid;
+  size_t smem;
+};
+template <typename T>
+static LegPlan leg_plan(const Lev<T>& L, int k) {
+  auto tiles = [&](int tx, int ty) { return dim3((L.nx + tx - 1) / tx, (L.ny + ty - 1) / ty); };
+  LegPlan p;
+  p.grid = tiles(LegTile<T, 0>::TX, LegTile<T, 0>::TY);
+  const size_t n = (size_t)p.grid.x * p.grid.y;
+  p.cfg = leg_config<T>(k + 1, n < (size_t)kLegFewTiles, n <= (size_t)kLegQuarter);
+  p.smem = p.cfg < 4 ? leg_smem<T, 0>(k) : leg_smem<T, 1>(k);
+  if (p.cfg >= 4) p.grid = tiles(LegTile<T, 1>::TX, LegTile<T, 1>::TY);
+  return p;
 }
 
 // Shared memory of coarse_resident_kernel over levels l .. nl-1, 0 where it
@@ -1348,28 +1397,22 @@ static int coarse_vcycle(fvx_mg* g, int l, cudaStream_t st) {
 template <typename T>
 static int leg_down(fvx_mg* g, int l, const T* f, const T* u_init, int k, cudaStream_t st) {
   if (k > kLegMaxSweeps) return FVX_ERR_ARG;
-  int rc = leg_attr<T>();
-  if (rc) return rc;
   LevArray<T>& A = levs<T>(g);
   Lev<T>& L = A.L[l];
-  constexpr int TX = LegTile<T>::TX, TY = LegTile<T>::TY;
-  dim3 gr((L.nx + TX - 1) / TX, (L.ny + TY - 1) / TY);
-  // programmatic launch: the constants load while the kernel before
-  // finishes (the kernel waits before reading f and u_init)
-  const int cfg = leg_config<T>(k + 1, (size_t)gr.x * gr.y < (size_t)kLegFewTiles);
-  const size_t sm = leg_smem<T>(k);
+  const LegPlan pl = leg_plan<T>(L, k);
+  const dim3 gr = pl.grid;
+  const size_t sm = pl.smem;
   const Lev<T>& C = A.L[l + 1];
   const T om = (T)g->omega;
-  cudaError_t e = cudaErrorInvalidValue;
-  switch (cfg) {
-    case 0: e = fvx_launch_pdl(down_leg_kernel<T, 512, 4>, gr, dim3(512), sm, st, L, f, u_init, k, om, C); break;
-    case 1: e = fvx_launch_pdl(down_leg_kernel<T, 512, 8>, gr, dim3(512), sm, st, L, f, u_init, k, om, C); break;
-    case 2: e = fvx_launch_pdl(down_leg_kernel<T, 1024, 4>, gr, dim3(1024), sm, st, L, f, u_init, k, om, C); break;
-    case 3: e = fvx_launch_pdl(down_leg_kernel<T, 1024, 8>, gr, dim3(1024), sm, st, L, f, u_init, k, om, C); break;
+  switch (pl.cfg) {
+    case 0: return launch_down<T, 0, 512, 4>(gr, sm, st, L, f, u_init, k, om, C);
+    case 1: return launch_down<T, 0, 512, 8>(gr, sm, st, L, f, u_init, k, om, C);
+    case 2: return launch_down<T, 0, 1024, 4>(gr, sm, st, L, f, u_init, k, om, C);
+    case 3: return launch_down<T, 0, 1024, 8>(gr, sm, st, L, f, u_init, k, om, C);
+    case 4: return launch_down<T, 1, 1024, 2>(gr, sm, st, L, f, u_init, k, om, C);
+    case 5: return launch_down<T, 1, 1024, 4>(gr, sm, st, L, f, u_init, k, om, C);
     default: return FVX_ERR_ARG;
   }
-  if (e != cudaSuccess) return FVX_ERR_CUDA;
-  return fvx_cuda_status();
 }
 
 // Upward leg at host-driven level l: out <- k sweeps on f from L.u + P ec.
@@ -1377,27 +1420,23 @@ template <typename T>
 static int leg_up(fvx_mg* g, int l, const T* f, const T* ec, int k, T* out, cudaStream_t st,
                   const double* ec_scale = nullptr) {
   if (k > kLegMaxSweeps) return FVX_ERR_ARG;
-  int rc = leg_attr<T>();
-  if (rc) return rc;
   LevArray<T>& A = levs<T>(g);
   Lev<T>& L = A.L[l];
-  constexpr int TX = LegTile<T>::TX, TY = LegTile<T>::TY;
-  dim3 gr((L.nx + TX - 1) / TX, (L.ny + TY - 1) / TY);
-  const int cfg = leg_config<T>(k + 1, (size_t)gr.x * gr.y < (size_t)kLegFewTiles);
-  const size_t sm = leg_smem<T>(k);
+  const LegPlan pl = leg_plan<T>(L, k);
+  const dim3 gr = pl.grid;
+  const size_t sm = pl.smem;
   const Lev<T>& C = A.L[l + 1];
   const T om = (T)g->omega;
   const T* up = L.u;
-  cudaError_t e = cudaErrorInvalidValue;
-  switch (cfg) {
-    case 0: e = fvx_launch_pdl(up_leg_kernel<T, 512, 4>, gr, dim3(512), sm, st, L, f, up, C, ec, k, om, out, ec_scale); break;
-    case 1: e = fvx_launch_pdl(up_leg_kernel<T, 512, 8>, gr, dim3(512), sm, st, L, f, up, C, ec, k, om, out, ec_scale); break;
-    case 2: e = fvx_launch_pdl(up_leg_kernel<T, 1024, 4>, gr, dim3(1024), sm, st, L, f, up, C, ec, k, om, out, ec_scale); break;
-    case 3: e = fvx_launch_pdl(up_leg_kernel<T, 1024, 8>, gr, dim3(1024), sm, st, L, f, up, C, ec, k, om, out, ec_scale); break;
+  switch (pl.cfg) {
+    case 0: return launch_up<T, 0, 512, 4>(gr, sm, st, L, f, up, C, ec, k, om, out, ec_scale);
+    case 1: return launch_up<T, 0, 512, 8>(gr, sm, st, L, f, up, C, ec, k, om, out, ec_scale);
+    case 2: return launch_up<T, 0, 1024, 4>(gr, sm, st, L, f, up, C, ec, k, om, out, ec_scale);
+    case 3: return launch_up<T, 0, 1024, 8>(gr, sm, st, L, f, up, C, ec, k, om, out, ec_scale);
+    case 4: return launch_up<T, 1, 1024, 2>(gr, sm, st, L, f, up, C, ec, k, om, out, ec_scale);
+    case 5: return launch_up<T, 1, 1024, 4>(gr, sm, st, L, f, up, C, ec, k, om, out, ec_scale);
     default: return FVX_ERR_ARG;
   }
-  if (e != cudaSuccess) return FVX_ERR_CUDA;
-  return fvx_cuda_status();
 }
 
 // V-cycle below the finest level of a host-driven cycle: entered with
