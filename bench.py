@@ -330,7 +330,7 @@ def fp64_metric_section(method, steps, flush, n=256):
     ms = _time_graphs(graphs, steps, flush)
     return {"workload": f"qg1.5_rk3ssp_{method}_dst_{n}x{n}", "dtype": "f64", "steps": steps,
             "ms_per_step": ms / steps, "value": n * n * steps / (ms * 1e-3) / 1e6, "unit": UNIT,
-            "launches_per_step": per_step, "dst": "FP64 SIMT transform-matrix chain", "stage_tile": tile,
+            "launches_per_step": per_step, "dst": "FP64 transform-matrix chain", "stage_tile": tile,
             "parity": {"rel_err_vs_fp64_oracle": err, "bar": 1e-12},
             "cpu_oracle": {"value": n * n * len(times) / sum(times) / 1e6, "unit": UNIT, "cores": cores}}
 
