@@ -808,8 +808,14 @@ up_leg_kernel(Lev<T> L, const T* f, const T* u_pre, Lev<T> C, const T* ec, int k
 // register arithmetic.  A chain of dependent sweeps bounds it: 24 FP32 sweeps
 // over global memory took 11 us of a 512^2 problem's coarse part, the 50
 // coarsest ones 10.5.  With R rows per thread an FP32 plan takes the levels
-// up to 64 x 64, whose two legs cost more than the 12 sweeps here.  A 512^2
-// FP32 V-cycle took 98.0 us and takes 82.5.  The arithmetic of every cell is
+// up to 64 x 64, whose two legs cost more than the 12 sweeps here.  The phases
+// between the sweeps run once each and are mostly cold code and index
+// arithmetic: rows by a float reciprocal instead of divisions, all levels'
+// loads in flight together, levels of one row per thread in their own code
+// with only their warps at the barriers (a 16 x 16 sweep 340 cycles with four
+// predicated rows and all warps).  A 512^2 FP32 V-cycle took 98.0 us over
+// global memory, 82.5 resident; 74 and 68 without and with the measures of
+// the last sentence, on quarter tiles above.  The arithmetic of every cell is
 // the legs' (jac_v), the coarsest sweeps run in E.
 // ---------------------------------------------------------------------------
 template <typename T> struct CoarseRows { static constexpr int R = sizeof(T) == 4 ? 4 : 1; };
@@ -849,7 +855,7 @@ DEV void res_load(const ResLev<T>& V, const T* A, ResCells<T, R>& s, int p, int 
   }
 }
 template <typename T, int R>
-DEV T* res_sweeps(const Lev<T>& L, ResCells<T, R>& s, T* A, T* B, int k, int p, int pitch, int rows) {
+DEV T* res_sweeps(const Lev<T>& L, ResCells<T, R>& s, T* A, T* B, int k, int p, int pitch, int rows, int nthr) {
   for (int sw = 0; sw < k; ++sw) {
     if (rows > 0) {
       T us = A[p - pitch], cys = s.cys0;
@@ -868,7 +874,7 @@ DEV T* res_sweeps(const Lev<T>& L, ResCells<T, R>& s, T* A, T* B, int k, int p, 
         }
       }
     }
-    __syncthreads();
+    asm volatile("bar.sync 2, %0;" ::"r"(nthr) : "memory");
     T* t = A;
     A = B;
     B = t;
@@ -876,113 +882,194 @@ DEV T* res_sweeps(const Lev<T>& L, ResCells<T, R>& s, T* A, T* B, int k, int p, 
   return A;
 }
 
+// Where a level lies: 1 / nx, rows per thread, threads of the warps that own
+// cells, first cell in the walk over all levels, first value of its arrays.
+struct ResGeo {
+  float rnx;
+  int LR, nthr, cell0, base;
+};
+// c / nx for c < 8192 (the half keeps the product off the integers)
+DEV int res_row(int c, float rnx) { return (int)(((float)c + 0.5f) * rnx); }
+// The thread's cells of a level: rows r0 .. r0 + rows - 1 of column c.
+template <typename T>
+DEV void res_own(const Lev<T>& L, const ResGeo& g, int& c, int& r0, int& rows) {
+  const int seg = res_row(threadIdx.x, g.rnx);
+  c = (int)threadIdx.x - seg * L.nx;
+  r0 = seg * g.LR;
+  rows = r0 >= L.ny ? 0 : (L.ny - r0 < g.LR ? L.ny - r0 : g.LR);
+}
+
+// Down a level: n_pre sweeps from zero, then r * mask (the legs' form) into
+// the other buffer.  Run by the level's warps.
+template <typename T, int R>
+DEV void res_down(const Lev<T>& L, const ResGeo& g, const ResLev<T>& V, int n_pre) {
+  const int pitch = L.nx + 2;
+  int c, r0, rows;
+  res_own(L, g, c, r0, rows);
+  const int p = (r0 + 1) * pitch + c + 1;
+  ResCells<T, R> s;
+  res_load<T, R>(V, V.u, s, p, pitch, rows);
+  const T* A = res_sweeps<T, R>(L, s, V.u, V.v, n_pre, p, pitch, rows, g.nthr);
+  T* B = A == V.u ? V.v : V.u;
+  if (rows > 0) {
+    T us = A[p - pitch], cys = s.cys0;
+    const T top = A[p + rows * pitch];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (i < rows) {
+        const int q = p + i * pitch;
+        const T um = s.u[i], un = i + 1 < rows ? s.u[i + 1 < R ? i + 1 : i] : top;
+        const T ue = A[q + 1], uw = A[q - 1], mc = V.m[q];
+        const T lap = divd(s.cx[i] * (ue - um) - s.cxw[i] * (um - uw), L.dx2, L.rdx2) +
+                      divd(s.cy[i] * (un - um) - cys * (um - us), L.dy2, L.rdy2);
+        B[q] = ((s.f[i] - (lap - L.lam * um) * mc) * mc) * mc;
+        us = um;
+        cys = s.cy[i];
+      }
+    }
+  }
+}
+
+// Up a level: the prolonged correction ec (masked by W.m) added, then n_post
+// sweeps.  out (may be null): the result in global memory.
+template <typename T, int R>
+DEV void res_up(const Lev<T>& L, const ResGeo& g, const ResLev<T>& V, const ResLev<T>& W, const T* ec, int cp, int n_pre,
+                int n_post, T* out) {
+  const int pitch = L.nx + 2;
+  int c, r0, rows;
+  res_own(L, g, c, r0, rows);
+  const int p = (r0 + 1) * pitch + c + 1;
+  T* A = (n_pre & 1) ? V.v : V.u;
+  ResCells<T, R> s;
+  res_load<T, R>(V, A, s, p, pitch, rows);
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    if (i < rows) {
+      const int r = r0 + i, sj = (2 * (r & 1) - 1) * cp, si = 2 * (c & 1) - 1;
+      const int k = ((r >> 1) + 1) * cp + (c >> 1) + 1;
+      auto val = [&](int kk) -> T { return ec[kk] * W.m[kk]; };
+      const T ws = ((T(9) * val(k) + T(3) * val(k + si)) + T(3) * val(k + sj)) + T(1) * val(k + sj + si);
+      const T ds = ((T(9) * W.m[k] + T(3) * W.m[k + si]) + T(3) * W.m[k + sj]) + T(1) * W.m[k + sj + si];
+      const T mf = V.m[p + i * pitch];
+      const T e = (ws / (ds > T(1) ? ds : T(1))) * mf;
+      s.u[i] = (s.u[i] + e) * mf;
+      A[p + i * pitch] = s.u[i];
+    }
+  }
+  asm volatile("bar.sync 2, %0;" ::"r"(g.nthr) : "memory");
+  res_sweeps<T, R>(L, s, A, A == V.u ? V.v : V.u, n_post, p, pitch, rows, g.nthr);
+  if (out) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (i < rows) out[(size_t)(r0 + i) * L.nx + c] = s.u[i];
+  }
+}
+
 template <typename T, typename E, int R>
 __global__ void __launch_bounds__(kCoarseThreads)
-coarse_resident_kernel(LevArray<T> G, Lev<E> D, int l0, int nl, int n_pre, int n_post, int n_coarse, T omega) {
+coarse_resident_kernel(LevArray<T> G, Lev<E> D, int l0, int nl, int n_pre, int n_post, int n_coarse, T omega,
+                       int smem16) {
   __shared__ Lev<T> S[kMaxLevels];
+  __shared__ ResGeo geo[kMaxLevels + 1];
   extern __shared__ __align__(16) unsigned char res_raw[];
   const int tid = threadIdx.x;
-  if (tid < nl) S[tid] = G.L[tid];
   const int last = nl - 1;
   // the coarsest solve's arrays first (E is the wider type), then the levels
   E* e0 = (E*)res_raw;
-  const size_t PE = padded_cells(D.ny, D.nx);
+  const int PE = (int)padded_cells(D.ny, D.nx);
   E *ea = e0, *eb = e0 + PE, *ecx = e0 + 2 * PE, *ecy = e0 + 3 * PE, *ew = e0 + 4 * PE;
   T* lev0 = (T*)(e0 + 5 * PE);
-  __syncthreads();
-  for (int q = tid; q < (int)PE; q += kCoarseThreads) {
-    const int pitch = D.nx + 2, j = q / pitch - 1, i = q - (j + 1) * pitch - 1;
-    const bool in = j >= 0 && j < D.ny && i >= 0 && i < D.nx;
-    const size_t c = in ? (size_t)j * D.nx + i : 0;
-    ea[q] = E(0);
-    eb[q] = E(0);
-    ecx[q] = in ? D.cx[c] : E(0);
-    ecy[q] = in ? D.cy[c] : E(0);
-    ew[q] = in ? (E)omega * D.inv[c] : E(0);
+  if (tid >= l0 && tid <= nl) {
+    ResGeo g{0.f, 1, 0, 0, 0};
+    for (int l = l0; l < tid; ++l) {
+      g.cell0 += G.L[l].ny * G.L[l].nx;
+      g.base += 7 * (int)padded_cells(G.L[l].ny, G.L[l].nx);
+    }
+    if (tid < nl) {
+      const Lev<T>& L = G.L[tid];
+      g.rnx = 1.f / (float)L.nx;
+      g.LR = tid < last ? coarse_rows(L.ny, L.nx) : 1;
+      g.nthr = ((L.ny + g.LR - 1) / g.LR * L.nx + 31) & ~31;
+      S[tid] = L;
+    }
+    geo[tid] = g;
   }
+  __syncthreads();
+  // Every level's constants: all loads of a thread's cells in flight while
+  // the arrays and their rings are set to zero.
+  constexpr int NC = R == 1 ? 2 : 6;  // cells of all levels <= 4 / 3 of R x the threads
   {
-    T* base = lev0;
-    for (int l = l0; l < nl; ++l) {
-      const Lev<T> L = S[l];
-      const size_t P = padded_cells(L.ny, L.nx);
-      const ResLev<T> V = res_lev(base, P);
-      const int pitch = L.nx + 2;
-#pragma unroll 2
-      for (int q = tid; q < (int)P; q += kCoarseThreads) {
-        const int j = q / pitch - 1, i = q - (j + 1) * pitch - 1;
-        const bool in = j >= 0 && j < L.ny && i >= 0 && i < L.nx;
-        const size_t c = in ? (size_t)j * L.nx + i : 0;
-        const T m = in ? L.mask[c] : T(0), cx = in ? L.cx[c] : T(0), cy = in ? L.cy[c] : T(0),
-                w = in ? L.inv[c] : T(0);
-        V.u[q] = T(0);
-        V.v[q] = T(0);
-        V.f[q] = T(0);
-        V.w[q] = omega * w;
-        V.cx[q] = cx;
-        V.cy[q] = cy;
-        V.m[q] = m;
-      }
-      base += 7 * P;
+    T m[NC], cx[NC], cy[NC], w[NC];
+    int pos[NC], P[NC];
+#pragma unroll
+    for (int u = 0; u < NC; ++u) {
+      const int k = tid + u * kCoarseThreads;
+      pos[u] = -1;
+      if (k >= geo[nl].cell0) continue;
+      int l = l0;
+      while (k >= geo[l + 1].cell0) ++l;
+      const int c = k - geo[l].cell0, nx = S[l].nx, j = res_row(c, geo[l].rnx);
+      P[u] = (S[l].ny + 2) * (nx + 2);
+      pos[u] = geo[l].base + (j + 1) * (nx + 2) + (c - j * nx) + 1;
+      m[u] = S[l].mask[c];
+      cx[u] = S[l].cx[c];
+      cy[u] = S[l].cy[c];
+      w[u] = S[l].inv[c];
+    }
+    E dx = E(0), dy = E(0), dw = E(0);
+    const bool ecell = tid < D.ny * D.nx;
+    if (ecell) { dx = D.cx[tid]; dy = D.cy[tid]; dw = D.inv[tid]; }
+    for (int q = tid; q < smem16; q += kCoarseThreads) ((uint4*)res_raw)[q] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < NC; ++u) {
+      if (pos[u] < 0) continue;
+      T* v = lev0 + pos[u];
+      v[3 * P[u]] = omega * w[u];
+      v[4 * P[u]] = cx[u];
+      v[5 * P[u]] = cy[u];
+      v[6 * P[u]] = m[u];
+    }
+    if (ecell) {
+      const int j = res_row(tid, geo[last].rnx), q = (j + 1) * (D.nx + 2) + (tid - j * D.nx) + 1;
+      ecx[q] = dx;
+      ecy[q] = dy;
+      ew[q] = (E)omega * dw;
     }
   }
   grid_dep_wait();
-  __syncthreads();
-  // the thread's cells of a level: rows r0 .. r0 + rows - 1 of column c
-  auto own = [&](const Lev<T>& L, int& c, int& r0, int& rows) {
-    const int LR = coarse_rows(L.ny, L.nx), seg = tid / L.nx;
-    c = tid - seg * L.nx;
-    r0 = seg * LR;
-    rows = r0 >= L.ny ? 0 : (L.ny - r0 < LR ? L.ny - r0 : LR);
-  };
   {  // f of the first level
-    const Lev<T> L = S[l0];
-    const ResLev<T> V = res_lev(lev0, padded_cells(L.ny, L.nx));
-    int c, r0, rows;
-    own(L, c, r0, rows);
+    const int nx = S[l0].nx, cells = S[l0].ny * nx;
+    T* f = lev0 + 2 * padded_cells(S[l0].ny, nx);
+    T v[R];
 #pragma unroll
-    for (int i = 0; i < R; ++i)
-      if (i < rows) V.f[(r0 + i + 1) * (L.nx + 2) + c + 1] = __ldcg(L.f + (size_t)(r0 + i) * L.nx + c);
+    for (int u = 0; u < R; ++u) {
+      const int c = tid + u * kCoarseThreads;
+      if (c < cells) v[u] = __ldcg(S[l0].f + c);
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const int c = tid + u * kCoarseThreads, j = res_row(c, geo[l0].rnx);
+      if (c < cells) f[(j + 1) * (nx + 2) + (c - j * nx) + 1] = v[u];
+    }
   }
   grid_dep_launch();
   __syncthreads();
-  T* base = lev0;
+  auto view = [&](int l) { return res_lev(lev0 + geo[l].base, padded_cells(S[l].ny, S[l].nx)); };
   for (int l = l0; l < last; ++l) {
     const Lev<T> L = S[l];
-    const size_t P = padded_cells(L.ny, L.nx);
-    const ResLev<T> V = res_lev(base, P);
-    const int pitch = L.nx + 2;
-    int c, r0, rows;
-    own(L, c, r0, rows);
-    const int p = (r0 + 1) * pitch + c + 1;
-    ResCells<T, R> s;
-    res_load<T, R>(V, V.u, s, p, pitch, rows);
-    T* A = res_sweeps<T, R>(L, s, V.u, V.v, n_pre, p, pitch, rows);
-    T* B = A == V.u ? V.v : V.u;
-    // r * mask into B (the legs' form), then the restricted residual
-    if (rows > 0) {
-      T us = A[p - pitch], cys = s.cys0;
-      const T top = A[p + rows * pitch];
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        if (i < rows) {
-          const int q = p + i * pitch;
-          const T um = s.u[i], un = i + 1 < rows ? s.u[i + 1 < R ? i + 1 : i] : top;
-          const T ue = A[q + 1], uw = A[q - 1], mc = V.m[q];
-          const T lap = divd(s.cx[i] * (ue - um) - s.cxw[i] * (um - uw), L.dx2, L.rdx2) +
-                        divd(s.cy[i] * (un - um) - cys * (um - us), L.dy2, L.rdy2);
-          B[q] = ((s.f[i] - (lap - L.lam * um) * mc) * mc) * mc;
-          us = um;
-          cys = s.cy[i];
-        }
-      }
+    const ResGeo g = geo[l];
+    const ResLev<T> V = view(l), W = view(l + 1);
+    if (tid < g.nthr) {
+      if (g.LR == 1) res_down<T, 1>(L, g, V, n_pre);
+      else res_down<T, R>(L, g, V, n_pre);
     }
     __syncthreads();
-    base += 7 * P;
-    const Lev<T> C = S[l + 1];
-    const ResLev<T> W = res_lev(base, padded_cells(C.ny, C.nx));
-    for (int q = tid; q < C.ny * C.nx; q += kCoarseThreads) {
-      const int J = q / C.nx, I = q - J * C.nx;
-      const int k = (2 * J + 1) * pitch + 2 * I + 1, kc = (J + 1) * (C.nx + 2) + I + 1;
+    const T* B = (n_pre & 1) ? V.u : V.v;  // r * mask
+    const int pitch = L.nx + 2, cnx = S[l + 1].nx, cells = S[l + 1].ny * cnx;
+    if (tid < cells) {  // a quarter of the level's cells, at most one per thread
+      const int J = res_row(tid, geo[l + 1].rnx), I = tid - J * cnx;
+      const int k = (2 * J + 1) * pitch + 2 * I + 1, kc = (J + 1) * (cnx + 2) + I + 1;
       const T sum4 = ((B[k] + B[k + pitch]) + B[k + 1]) + B[k + pitch + 1];
       const T cnt = ((V.m[k] + V.m[k + pitch]) + V.m[k + 1]) + V.m[k + pitch + 1];
       W.f[kc] = (sum4 / (cnt > T(1) ? cnt : T(1))) * W.m[kc];
@@ -991,11 +1078,11 @@ coarse_resident_kernel(LevArray<T> G, Lev<E> D, int l0, int nl, int n_pre, int n
   }
   {  // the coarsest solve: one cell per thread of the warps that hold any
     const int nx = D.nx, cells = D.ny * nx, pitch = nx + 2;
-    const ResLev<T> V = res_lev(base, padded_cells(D.ny, nx));
-    const int nthr = (cells + 31) & ~31;
+    const ResLev<T> V = view(last);
+    const int nthr = geo[last].nthr;
     if (tid < nthr) {
       const bool live = tid < cells;
-      const int j = live ? tid / nx : 0, i = live ? tid - j * nx : 0, q = (j + 1) * pitch + i + 1;
+      const int j = live ? res_row(tid, geo[last].rnx) : 0, i = live ? tid - j * nx : 0, q = (j + 1) * pitch + i + 1;
       const E cx = ecx[q], cxw = ecx[q - 1], cy = ecy[q], cys = ecy[q - pitch], w = ew[q], f = (E)V.f[q];
       E um = E(0);
       E *a = ea, *b = eb;
@@ -1008,51 +1095,27 @@ coarse_resident_kernel(LevArray<T> G, Lev<E> D, int l0, int nl, int n_pre, int n
         a = b;
         b = t;
       }
-      if (live) V.u[q] = (T)um;
-    }
-    __syncthreads();
-  }
-  const T* ec = res_lev(base, padded_cells(D.ny, D.nx)).u;
-  for (int l = last - 1; l >= l0; --l) {
-    const Lev<T> L = S[l], C = S[l + 1];
-    const ResLev<T> W = res_lev(base, padded_cells(C.ny, C.nx));
-    const size_t P = padded_cells(L.ny, L.nx);
-    base -= 7 * P;
-    const ResLev<T> V = res_lev(base, P);
-    const int pitch = L.nx + 2, cp = C.nx + 2;
-    int c, r0, rows;
-    own(L, c, r0, rows);
-    const int p = (r0 + 1) * pitch + c + 1;
-    T* A = (n_pre & 1) ? V.v : V.u;
-    ResCells<T, R> s;
-    res_load<T, R>(V, A, s, p, pitch, rows);
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      if (i < rows) {
-        const int r = r0 + i, sj = (2 * (r & 1) - 1) * cp, si = 2 * (c & 1) - 1;
-        const int k = ((r >> 1) + 1) * cp + (c >> 1) + 1;
-        auto val = [&](int kk) -> T { return ec[kk] * W.m[kk]; };
-        const T ws = ((T(9) * val(k) + T(3) * val(k + si)) + T(3) * val(k + sj)) + T(1) * val(k + sj + si);
-        const T ds = ((T(9) * W.m[k] + T(3) * W.m[k + si]) + T(3) * W.m[k + sj]) + T(1) * W.m[k + sj + si];
-        const T mf = V.m[p + i * pitch];
-        const T e = (ws / (ds > T(1) ? ds : T(1))) * mf;
-        s.u[i] = (s.u[i] + e) * mf;
-        A[p + i * pitch] = s.u[i];
+      if (live) {
+        V.u[q] = (T)um;
+        if (l0 == last) S[l0].u[tid] = (T)um;
       }
     }
     __syncthreads();
-    ec = res_sweeps<T, R>(L, s, A, A == V.u ? V.v : V.u, n_post, p, pitch, rows);
-    if (l == l0) {
-#pragma unroll
-      for (int i = 0; i < R; ++i)
-        if (i < rows) L.u[(size_t)(r0 + i) * L.nx + c] = s.u[i];
-    }
   }
-  if (l0 == last)
-    for (int q = tid; q < D.ny * D.nx; q += kCoarseThreads) {
-      const int j = q / D.nx, i = q - j * D.nx;
-      S[l0].u[q] = ec[(j + 1) * (D.nx + 2) + i + 1];
+  for (int l = last - 1; l >= l0; --l) {
+    const Lev<T> L = S[l];
+    const ResGeo g = geo[l];
+    const ResLev<T> V = view(l), W = view(l + 1);
+    // the coarser result: the coarsest solve leaves it in u, a level in the
+    // buffer its n_pre + n_post sweeps end in
+    const T* ec = (l + 1 < last && ((n_pre + n_post) & 1)) ? W.v : W.u;
+    T* out = l == l0 ? L.u : nullptr;
+    if (tid < g.nthr) {
+      if (g.LR == 1) res_up<T, 1>(L, g, V, W, ec, S[l + 1].nx + 2, n_pre, n_post, out);
+      else res_up<T, R>(L, g, V, W, ec, S[l + 1].nx + 2, n_pre, n_post, out);
     }
+    __syncthreads();
+  }
 }
 
 // masked_laplacian (iterative.py:144-191): periodic roll, (lap - lam psi_m) * m
@@ -1355,6 +1418,7 @@ static size_t resident_smem(fvx_mg* g, int l) {
     if (k < g->nl - 1 && coarse_rows(A.L[k].ny, A.L[k].nx) > CoarseRows<T>::R) return 0;
     bytes += 7 * padded_cells(A.L[k].ny, A.L[k].nx) * sizeof(T);
   }
+  bytes = (bytes + 15) & ~(size_t)15;
   return bytes <= kResidentSmem ? bytes : 0;
 }
 // First level (>= 1) that the V-cycle's single CTA starts at: the resident
@@ -1379,7 +1443,8 @@ static int coarse_vcycle(fvx_mg* g, int l, cudaStream_t st) {
         }))
       return FVX_ERR_CUDA;
     if (fvx_launch_pdl(coarse_resident_kernel<T, double, R>, dim3(1), dim3(kCoarseThreads), bytes, st, levs<T>(g),
-                       g->A64.L[g->nl - 1], l, g->nl, g->n_pre, g->n_post, g->n_coarse, (T)g->omega) != cudaSuccess)
+                       g->A64.L[g->nl - 1], l, g->nl, g->n_pre, g->n_post, g->n_coarse, (T)g->omega,
+                       (int)(bytes / 16)) != cudaSuccess)
       return FVX_ERR_CUDA;
     return fvx_cuda_status();
   }
