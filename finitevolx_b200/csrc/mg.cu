@@ -618,8 +618,14 @@ DEV T* leg_sweeps(const Lev<T>& L, LegCells<T, R>& s, T* A, T* B, const T* scx, 
 // u_pre, ec, ec_scale) is read only after grid_dep_wait, through L2
 // (ld.global.cg), from pointers not marked __restrict__ -- a restrict-const
 // load may be served by the read-only path or moved above the wait.
+// Blocks per SM asked of the compiler: two FP64 blocks of 512 threads on 64
+// registers each (a few spilled bytes) hide each other's chains where one on
+// 85 did not: FP64 V-cycle at 512^2 142 us with one, 124 with two, at 384^2
+// 97 and 88.
+template <typename T> constexpr int leg_blocks(int nt, int r) { return sizeof(T) == 8 && nt == 512 && r == 4 ? 2 : 1; }
+
 template <typename T, int V, int NT, int R>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, leg_blocks<T>(NT, R))
 down_leg_kernel(Lev<T> L, const T* f, const T* u_init, int k, T omega, Lev<T> C) {
   constexpr int TX = LegTile<T, V>::TX, TY = LegTile<T, V>::TY;
   const int H = k + 1;
@@ -725,7 +731,7 @@ down_leg_kernel(Lev<T> L, const T* f, const T* u_init, int k, T omega, Lev<T> C)
 // ec_scale (may be null): the coarse correction is read as ec * (T)*ec_scale
 // (the hybrid cycle's energy-optimal scaling, applied as the window loads).
 template <typename T, int V, int NT, int R>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, leg_blocks<T>(NT, R))
 up_leg_kernel(Lev<T> L, const T* f, const T* u_pre, Lev<T> C, const T* ec, int k, T omega, T* __restrict__ out,
               const double* ec_scale) {
   constexpr int TX = LegTile<T, V>::TX, TY = LegTile<T, V>::TY;
