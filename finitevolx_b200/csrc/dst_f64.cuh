@@ -338,23 +338,25 @@ constexpr FoldTile kFoldTiles[4] = {{16, 16, 2, {0, 4.5f, 9.4f}},
                                     {32, 32, 3, {0, 17.5f, 28.f, 33.f}},
                                     {32, 64, 4, {0, 32.f, 53.f, 62.f, 81.f}}};
 
-// One folded product on the tile with the least work on the fullest SM (e.g.
-// us per product, 16 x 16 / 32 x 16 / 32 x 32 / 32 x 64: 256^2 3.3 / 4.2 / 6.5
-// / 11, 512^2 11.5 / 8.7 / 10.9 / 18.6, 896^2 45 / 39 / 32 / 46, 2048^2 - / -
-// / 323 / 280).  The result does not depend on the tile.
+// One folded product on the tile with the least work on the fullest SM, of
+// those whose rows fit the grid's 65535 blocks in y (e.g. us per product, 16 x
+// 16 / 32 x 16 / 32 x 32 / 32 x 64: 256^2 3.3 / 4.2 / 6.5 / 11, 512^2 11.5 /
+// 8.7 / 10.9 / 18.6, 896^2 45 / 39 / 32 / 46, 2048^2 - / - / 323 / 280).  The
+// result does not depend on the tile.
 static int gemm_f64_fold(FoldArgs a, cudaStream_t st) {
   // 16-byte loads of X need even row and batch pitches and an aligned base
   const bool xv = ((uintptr_t)a.X & 15) == 0 && a.xld % 2 == 0 && a.xbs % 2 == 0;
   const uintptr_t oa = a.out_f32 ? 8 : 16;
   a.vec = a.R % 2 == 0 && ((uintptr_t)a.out & (oa - 1)) == 0 && a.old % 2 == 0 && a.obs % 2 == 0;
-  int best = 0;
+  int best = -1;
   double least = 0;
   for (int k = 0; k < 4; ++k) {
     const FoldTile& t = kFoldTiles[k];
+    if ((a.M + t.tm - 1) / t.tm > 65535) continue;
     const long long tiles = (long long)((a.NH + t.tn - 1) / t.tn) * ((a.M + t.tm - 1) / t.tm);
     const long long c = (tiles + 147) / 148;
     const double cost = (double)(c / t.r) * t.g[t.r] + t.g[c % t.r];
-    if (k == 0 || cost < least) { best = k; least = cost; }
+    if (best < 0 || cost < least) { best = k; least = cost; }
   }
   switch (best) {
     case 0: return launch_fold<16, 16, 64, 5, false>(a, xv, st);
