@@ -180,14 +180,15 @@ sw_kernel(Fields<T> F, int RW, T* __restrict__ o1, T* __restrict__ o2) {
 
 // 16 rows per march on large fields (the two rows around the march cost 1/8
 // more loads), fewer on small ones, where a march's chain of rows is the
-// kernel's time.  Coriolis plus Arakawa-Lamb momentum, FP64, masked, before ->
-// now: 2400^2 382 -> 127 us, 1020 x 764 52.9 -> 19.3, 130 x 98 7.9 -> 4.2.
+// kernel's time, and more where the marches would not fit the grid's y.
+// Coriolis plus Arakawa-Lamb momentum, FP64, masked, before -> now: 2400^2 382
+// -> 127 us, 1020 x 764 52.9 -> 19.3, 130 x 98 7.9 -> 4.2.
 template <typename T, int OP>
 static int launch(const Fields<T>& F, T* o1, T* o2, cudaStream_t st) {
   const long long cells = (long long)F.ny * F.nx;
-  const int RW = cells >= 2000000 ? 16 : (cells >= 400000 ? 8 : (cells >= 100000 ? 4 : 1));
-  const dim3 g((F.nx + kWarps * kCols - 1) / (kWarps * kCols), (F.ny + RW - 1) / RW);
-  if (g.y > 65535) return FVX_ERR_SHAPE;
+  int RW = cells >= 2000000 ? 16 : (cells >= 400000 ? 8 : (cells >= 100000 ? 4 : 1));
+  while (F.ny > 65535LL * RW) RW *= 2;
+  const dim3 g((F.nx + kWarps * kCols - 1) / (kWarps * kCols), (unsigned)((F.ny - 1LL) / RW + 1));
   sw_kernel<T, OP><<<g, 32 * kWarps, 0, st>>>(F, RW, o1, o2);
   return fvx_cuda_status();
 }
