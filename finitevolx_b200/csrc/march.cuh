@@ -54,8 +54,8 @@ DEV float2 f2s(float c) { return make_float2(c, c); }
 // stencils at once: 38 packed operations and one reciprocal per lane for
 // WENO5 (four for WENO-Z5).  Candidates and weights are scaled by 6 and 10
 // so that most coefficients become sums (a packed constant occupies a
-// register pair).  Stencils whose products overflow go through the scalar
-// form with a division per weight.
+// register pair).  Stencils whose products leave the range go through
+// weno5_wide.
 template <bool Z>
 DEV float2 weno5_x2(float2 qmm, float2 qm, float2 q0, float2 qp, float2 qpp) {
   const float2 d0 = f2sub(qm, qmm), d1 = f2sub(q0, qm), d2 = f2sub(qp, q0), d3 = f2sub(qpp, qp);
@@ -84,12 +84,16 @@ DEV float2 weno5_x2(float2 qmm, float2 qm, float2 q0, float2 qp, float2 qpp) {
   W3 = f2mul(f2s(3.f), W3);
   const float2 num = f2fma(W3, g3, f2fma(W2, g2, f2mul(W1, g1)));
   const float2 den = f2add(f2add(W1, W2), W3);
-  if (recon_finite(den.x, num.x) && recon_finite(den.y, num.y)) {
+  bool ok = recon_finite(den.x, num.x) && recon_finite(den.y, num.y);
+  if (Z) {
+    const float2 t = f2add(f2add(t1, t2), t3);
+    ok = ok && t.x < 8e37f && t.y < 8e37f;
+  }
+  if (ok) {
     const float s = 1.f / 6.f;
     return make_float2(fmaf(num.x * s, rcp_approx(den.x), q0.x), fmaf(num.y * s, rcp_approx(den.y), q0.y));
   }
-  return make_float2(weno5_divisions<float, Z>(qmm.x, qm.x, q0.x, qp.x, qpp.x),
-                     weno5_divisions<float, Z>(qmm.y, qm.y, q0.y, qp.y, qpp.y));
+  return make_float2(weno5_wide<Z>(qmm.x, qm.x, q0.x, qp.x, qpp.x), weno5_wide<Z>(qmm.y, qm.y, q0.y, qp.y, qpp.y));
 }
 
 // Window of a scheme: cells i - R .. i + R + 1 around face i at w[0 .. 2R+1].

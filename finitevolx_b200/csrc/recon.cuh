@@ -43,67 +43,107 @@ template <typename T> DEV T tmin(T a, T b) { return a < b ? a : b; }
 // squares of them, and the weights 1 / s_k (s_k = (b_k + eps)^2) are brought
 // to their common denominator, prod_{j != k} s_j, so that one division
 // normalises the whole sum (a division costs 13 FP64 FMAs of throughput;
-// FP32 takes one reciprocal).  s_k >= eps^2, so no product underflows;
+// FP32 takes one reciprocal).  In FP64 no such product underflows, and
 // stencils whose products overflow take the form with a division per weight.
+// In FP32 stencils whose products leave the range of the type or of the
+// reciprocal (2^126, beyond which it is flushed to 0) are scaled first, by a
+// call (weno3_wide, weno5_wide).
 template <typename T> DEV bool recon_finite(T den, T num) {
   if constexpr (sizeof(T) == 8) return den < 1e308 && fabs(num) < 1e308;
-  else return den < 3e38f && fabsf(num) < 3e38f;
+  else return den < 8e37f && fabsf(num) < 3e38f;
+}
+// Power-of-two scale for differences of at most m, to c m in [1, 4), with its
+// inverse ic.  A form is homogeneous in (d, sqrt(eps)); eps c^2 is kept within
+// [1e-18, 1e8], beyond which it changes a weight by less than 1e-8 (or decides
+// between differences 1e9 times smaller than m).
+DEV void recon_scale(float m, float eps, float& c, float& ic, float& epsc) {
+  const int e = min(max((int)(__float_as_uint(m) >> 23), 1), 253);
+  ic = __uint_as_float((unsigned)e << 23);
+  c = __uint_as_float((unsigned)(254 - e) << 23);
+  epsc = fminf(fmaxf(eps * c * c, 1e-18f), 1e8f);
 }
 
 // ---- WENO3 (advection/weno.py:297-347) ------------------------------------
 // The right-biased forms (:413-459, :462-522, :597-665) are these functions on
 // the mirrored stencil; face_value() below feeds them that way.
-template <typename T> DEV T weno3(T qm, T q0, T qp) {
-  const T eps = T(1e-8);
-  const T d1 = q0 - qm, d2 = qp - q0;
-  const T s1 = sq(d1 * d1 + eps), s2 = sq(d2 * d2 + eps);
-  // weights 1/3, 2/3 and candidates q0 + d/2: (s2 d1 + 2 s1 d2) / (2 (s2 + 2 s1))
-  const T den = s2 + T(2) * s1, num = s2 * d1 + T(2) * (s1 * d2);
-  if (recon_finite(den, num)) return q0 + T(0.5) * fdiv(num, den);
-  const T w1 = fdiv(T(1.0 / 3.0), s1), w2 = fdiv(T(2.0 / 3.0), s2);
-  return fdiv(w1 * (T(-0.5) * qm + T(1.5) * q0) + w2 * (T(0.5) * (q0 + qp)), w1 + w2);
-}
-template <typename T> DEV T wenoz3(T qm, T q0, T qp) {
-  const T eps = T(1e-14);
-  const T d1 = q0 - qm, d2 = qp - q0;
-  const T b1 = d1 * d1, b2 = d2 * d2, tau = tabs(b2 - b1), t1 = b1 + eps, t2 = b2 + eps;
-  const T W1 = (t1 + tau) * t2, W2 = T(2) * ((t2 + tau) * t1);
-  const T den = W1 + W2, num = W1 * d1 + W2 * d2;
-  if (recon_finite(den, num)) return q0 + T(0.5) * fdiv(num, den);
-  const T w1 = T(1.0 / 3.0) * (T(1) + fdiv(tau, t1)), w2 = T(2.0 / 3.0) * (T(1) + fdiv(tau, t2));
-  return fdiv(w1 * (T(-0.5) * qm + T(1.5) * q0) + w2 * (T(0.5) * (q0 + qp)), w1 + w2);
-}
-// ---- WENO5 (advection/weno.py:350-410, :462-522) -------------------------
-// The form with a division per weight, on the raw values.
-template <typename T, bool Z>
-__noinline__ __device__ T weno5_divisions(T qmm, T qm, T q0, T qp, T qpp) {
-  const T k1 = T(13.0 / 12.0), k2 = T(0.25);
-  const T qi1 = T(1.0 / 3.0) * qmm - T(7.0 / 6.0) * qm + T(11.0 / 6.0) * q0;
-  const T qi2 = T(-1.0 / 6.0) * qm + T(5.0 / 6.0) * q0 + T(1.0 / 3.0) * qp;
-  const T qi3 = T(1.0 / 3.0) * q0 + T(5.0 / 6.0) * qp - T(1.0 / 6.0) * qpp;
-  const T b1 = k1 * sq(qmm - T(2) * qm + q0) + k2 * sq(qmm - T(4) * qm + T(3) * q0);
-  const T b2 = k1 * sq(qm - T(2) * q0 + qp) + k2 * sq(qm - qp);
-  const T b3 = k1 * sq(q0 - T(2) * qp + qpp) + k2 * sq(T(3) * q0 - T(4) * qp + qpp);
-  T w1, w2, w3;
-  if (Z) {
-    const T eps = T(1e-16), tau5 = tabs(b1 - b3);
-    w1 = T(0.1) * (T(1) + fdiv(tau5, b1 + eps));
-    w2 = T(0.6) * (T(1) + fdiv(tau5, b2 + eps));
-    w3 = T(0.3) * (T(1) + fdiv(tau5, b3 + eps));
+// Numerator and denominator of 2 (face - q0): weights 1/3, 2/3 (WENO-Z3: times
+// 1 + tau / (b + eps)) and candidates q0 + d/2.
+template <typename T, bool Z> DEV void weno3_sums(T d1, T d2, T eps, T& num, T& den) {
+  if constexpr (Z) {
+    const T b1 = d1 * d1, b2 = d2 * d2, tau = tabs(b2 - b1), t1 = b1 + eps, t2 = b2 + eps;
+    const T W1 = (t1 + tau) * t2, W2 = T(2) * ((t2 + tau) * t1);
+    den = W1 + W2;
+    num = W1 * d1 + W2 * d2;
   } else {
-    const T eps = T(1e-8);
-    w1 = fdiv(T(0.1), sq(b1 + eps));
-    w2 = fdiv(T(0.6), sq(b2 + eps));
-    w3 = fdiv(T(0.3), sq(b3 + eps));
+    const T s1 = sq(d1 * d1 + eps), s2 = sq(d2 * d2 + eps);
+    den = s2 + T(2) * s1;
+    num = s2 * d1 + T(2) * (s1 * d2);
   }
-  return fdiv(w1 * qi1 + w2 * qi2 + w3 * qi3, w1 + w2 + w3);
 }
-template <typename T, bool Z> DEV T weno5(T qmm, T qm, T q0, T qp, T qpp) {
-  const T d0 = qm - qmm, d1 = q0 - qm, d2 = qp - q0, d3 = qpp - qp;
+// FP32, out of the products' range.
+template <bool Z>
+__noinline__ __device__ float weno3_wide(float qm, float q0, float qp) {
+  const float d1 = q0 - qm, d2 = qp - q0;
+  float c, ic, eps, num, den;
+  recon_scale(fmaxf(fabsf(d1), fabsf(d2)), Z ? 1e-14f : 1e-8f, c, ic, eps);
+  weno3_sums<float, Z>(d1 * c, d2 * c, eps, num, den);
+  return q0 + (0.5f * fdiv(num, den)) * ic;
+}
+// FP64, products that overflow: a division per weight.
+template <bool Z>
+DEV double weno3_divisions(double qm, double q0, double qp) {
+  const double b1 = sq(q0 - qm), b2 = sq(qp - q0);
+  double w1, w2;
+  if (Z) {
+    const double tau = tabs(b2 - b1);
+    w1 = 1.0 / 3.0 * (1.0 + tau / (b1 + 1e-14));
+    w2 = 2.0 / 3.0 * (1.0 + tau / (b2 + 1e-14));
+  } else {
+    w1 = 1.0 / 3.0 / sq(b1 + 1e-8);
+    w2 = 2.0 / 3.0 / sq(b2 + 1e-8);
+  }
+  return (w1 * (-0.5 * qm + 1.5 * q0) + w2 * (0.5 * (q0 + qp))) / (w1 + w2);
+}
+template <typename T, bool Z> DEV T weno3_form(T qm, T q0, T qp) {
+  T num, den;
+  weno3_sums<T, Z>(q0 - qm, qp - q0, Z ? T(1e-14) : T(1e-8), num, den);
+  if (recon_finite(den, num)) return q0 + T(0.5) * fdiv(num, den);
+  if constexpr (sizeof(T) == 4) return weno3_wide<Z>(qm, q0, qp);
+  else return weno3_divisions<Z>(qm, q0, qp);
+}
+template <typename T> DEV T weno3(T qm, T q0, T qp) { return weno3_form<T, false>(qm, q0, qp); }
+template <typename T> DEV T wenoz3(T qm, T q0, T qp) { return weno3_form<T, true>(qm, q0, qp); }
+// ---- WENO5 (advection/weno.py:350-410, :462-522) -------------------------
+// The form with a division per weight, on the raw values (FP64).
+template <bool Z>
+__noinline__ __device__ double weno5_divisions(double qmm, double qm, double q0, double qp, double qpp) {
+  const double k1 = 13.0 / 12.0, k2 = 0.25;
+  const double qi1 = 1.0 / 3.0 * qmm - 7.0 / 6.0 * qm + 11.0 / 6.0 * q0;
+  const double qi2 = -1.0 / 6.0 * qm + 5.0 / 6.0 * q0 + 1.0 / 3.0 * qp;
+  const double qi3 = 1.0 / 3.0 * q0 + 5.0 / 6.0 * qp - 1.0 / 6.0 * qpp;
+  const double b1 = k1 * sq(qmm - 2.0 * qm + q0) + k2 * sq(qmm - 4.0 * qm + 3.0 * q0);
+  const double b2 = k1 * sq(qm - 2.0 * q0 + qp) + k2 * sq(qm - qp);
+  const double b3 = k1 * sq(q0 - 2.0 * qp + qpp) + k2 * sq(3.0 * q0 - 4.0 * qp + qpp);
+  double w1, w2, w3;
+  if (Z) {
+    const double eps = 1e-16, tau5 = tabs(b1 - b3);
+    w1 = 0.1 * (1.0 + tau5 / (b1 + eps));
+    w2 = 0.6 * (1.0 + tau5 / (b2 + eps));
+    w3 = 0.3 * (1.0 + tau5 / (b3 + eps));
+  } else {
+    const double eps = 1e-8;
+    w1 = 0.1 / sq(b1 + eps);
+    w2 = 0.6 / sq(b2 + eps);
+    w3 = 0.3 / sq(b3 + eps);
+  }
+  return (w1 * qi1 + w2 * qi2 + w3 * qi3) / (w1 + w2 + w3);
+}
+// Numerator and denominator of face - q0 from the four differences; eps4 = 4
+// eps.  Returns the sum of the smoothness terms t = 4 (b + eps).
+template <typename T, bool Z> DEV T weno5_sums(T d0, T d1, T d2, T d3, T eps4, T& num, T& den) {
   const T a1 = d1 - d0, a2 = d2 - d1, a3 = d3 - d2;
   const T c1 = a1 + T(2) * d1, c2 = d1 + d2, c3 = a3 - T(2) * d2;
-  const T k = T(13.0 / 3.0), eps4 = Z ? T(4e-16) : T(4e-8);
-  // t = 4 (b + eps)
+  const T k = T(13.0 / 3.0);
   const T t1 = c1 * c1 + (k * a1 * a1 + eps4), t2 = c2 * c2 + (k * a2 * a2 + eps4),
           t3 = c3 * c3 + (k * a3 * a3 + eps4);
   const T g1 = T(5.0 / 6.0) * d1 - T(1.0 / 3.0) * d0, g2 = T(1.0 / 6.0) * d1 + T(1.0 / 3.0) * d2,
@@ -126,9 +166,27 @@ template <typename T, bool Z> DEV T weno5(T qmm, T qm, T q0, T qp, T qpp) {
     W2 = T(0.6) * (s1 * s3);
     W3 = T(0.3) * (s1 * s2);
   }
-  const T den = W1 + W2 + W3, num = W1 * g1 + W2 * g2 + W3 * g3;
-  if (recon_finite(den, num)) return q0 + fdiv(num, den);
-  return weno5_divisions<T, Z>(qmm, qm, q0, qp, qpp);
+  den = W1 + W2 + W3;
+  num = W1 * g1 + W2 * g2 + W3 * g3;
+  return t1 + t2 + t3;
+}
+// FP32, out of the products' range.
+template <bool Z>
+__noinline__ __device__ float weno5_wide(float qmm, float qm, float q0, float qp, float qpp) {
+  const float d0 = qm - qmm, d1 = q0 - qm, d2 = qp - q0, d3 = qpp - qp;
+  const float m = fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(d2), fabsf(d3)));
+  float c, ic, eps4, num, den;
+  recon_scale(m, Z ? 4e-16f : 4e-8f, c, ic, eps4);
+  weno5_sums<float, Z>(d0 * c, d1 * c, d2 * c, d3 * c, eps4, num, den);
+  return q0 + fdiv(num, den) * ic;
+}
+template <typename T, bool Z> DEV T weno5(T qmm, T qm, T q0, T qp, T qpp) {
+  T num, den;
+  const T t = weno5_sums<T, Z>(qm - qmm, q0 - qm, qp - q0, qpp - qp, Z ? T(4e-16) : T(4e-8), num, den);
+  // (FP32 WENO-Z5: the reciprocals of the t have to be in range as well)
+  if (recon_finite(den, num) && (!Z || sizeof(T) == 8 || t < T(8e37))) return q0 + fdiv(num, den);
+  if constexpr (sizeof(T) == 4) return weno5_wide<Z>(qmm, qm, q0, qp, qpp);
+  else return weno5_divisions<Z>(qmm, qm, q0, qp, qpp);
 }
 // ---- WENO7 / WENO9, generic Jiang-Shu form (advection/weno.py:268-294) ---
 template <typename T> DEV T tab_c(int R, int k, int j) {
