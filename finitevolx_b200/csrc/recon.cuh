@@ -47,7 +47,8 @@ template <typename T> DEV T tmin(T a, T b) { return a < b ? a : b; }
 // stencils whose products overflow take the form with a division per weight.
 // In FP32 stencils whose products leave the range of the type or of the
 // reciprocal (2^126, beyond which it is flushed to 0) are scaled first, by a
-// call (weno3_wide, weno5_wide).
+// call (weno3_wide, weno5_wide); WENO5's products of differences under 1e-9
+// are subnormal and keep an absolute error of about 1e-16.
 template <typename T> DEV bool recon_finite(T den, T num) {
   if constexpr (sizeof(T) == 8) return den < 1e308 && fabs(num) < 1e308;
   else return den < 8e37f && fabsf(num) < 3e38f;
@@ -105,9 +106,13 @@ DEV double weno3_divisions(double qm, double q0, double qp) {
   return (w1 * (-0.5 * qm + 1.5 * q0) + w2 * (0.5 * (q0 + qp))) / (w1 + w2);
 }
 template <typename T, bool Z> DEV T weno3_form(T qm, T q0, T qp) {
+  const T d1 = q0 - qm, d2 = qp - q0;
   T num, den;
-  weno3_sums<T, Z>(q0 - qm, qp - q0, Z ? T(1e-14) : T(1e-8), num, den);
-  if (recon_finite(den, num)) return q0 + T(0.5) * fdiv(num, den);
+  weno3_sums<T, Z>(d1, d2, Z ? T(1e-14) : T(1e-8), num, den);
+  // FP32: a numerator under the smallest normal number (WENO-Z3 from
+  // differences of 1e-10 down, WENO3 of 1e-22) has lost its low bits
+  const bool small = sizeof(T) == 4 && !(fabsf((float)num) > 1e-37f) && (d1 != T(0) || d2 != T(0));
+  if (recon_finite(den, num) && !small) return q0 + T(0.5) * fdiv(num, den);
   if constexpr (sizeof(T) == 4) return weno3_wide<Z>(qm, q0, qp);
   else return weno3_divisions<Z>(qm, q0, qp);
 }

@@ -54,6 +54,14 @@ def test_beyond_the_products_range(cuda_ok, scheme, amplitude):
     _check(scheme, amplitude, scheme != "wenoz3")
 
 
+# differences of 1e-10 and below put WENO-Z3's products, 1e-22 and below
+# WENO3's, under FP32's smallest normal number; WENO-Z5 uses WENO-Z3 near edges
+@pytest.mark.parametrize("scheme,amplitude", [("wenoz3", 1e-10), ("wenoz3", 1e-13), ("wenoz3", 1e-25), ("wenoz5", 1e-13),
+                                              ("weno3", 1e-23), ("weno3", 1e-28)])
+def test_small_differences(cuda_ok, scheme, amplitude):
+    _check(scheme, amplitude, scheme != "wenoz3")
+
+
 @pytest.mark.parametrize("scheme", ["weno3", "wenoz3", "weno5", "wenoz5"])
 def test_constant_field(cuda_ok, scheme):
     import torch
