@@ -1231,7 +1231,7 @@ static int upload_levels(fvx_mg* g, std::vector<HostLevel>& H, int first = 0) {
   return FVX_OK;
 }
 
-// mask: [ny, nx] float64 0/1 (host); coeff: [ny, nx] float64 or NULL.
+// mask: [ny, nx] float64 (host), 0/1 or any weights; coeff: [ny, nx] float64 or NULL.
 extern "C" int fvx_mg_create(const double* mask, const double* coeff, int ny, int nx, double dx, double dy,
                              double lambda, int n_levels, int n_pre, int n_post, int n_coarse, double omega, int dtype,
                              fvx_mg** out) {
@@ -1464,11 +1464,48 @@ static int coarse_vcycle(fvx_mg* g, int l, cudaStream_t st) {
   return fvx_cuda_status();
 }
 
+// The legs of a finest level whose mask is not 0 / 1, a launch per sweep: the
+// fused legs hold a cell's mask as one bit, these multiply by it (jacobi_at,
+// restrict_at, prolong_at).  Coarser masks always are 0 / 1.
+template <typename T>
+static void sweeps_masked(fvx_mg* g, const T* f, int k, cudaStream_t st) {
+  Lev<T>& L = levs<T>(g).L[0];
+  const size_t n = (size_t)L.ny * L.nx;
+  T *a = L.u, *b = L.tmp;
+  for (int s = 0; s < k; ++s) {
+    jacobi_kernel<T><<<grid_for(n), 256, 0, st>>>(L, a, f, b, (T)g->omega);
+    std::swap(a, b);
+  }
+  if (a != L.u) copy_kernel<T><<<grid_for(n), 256, 0, st>>>(L.u, a, n);
+}
+template <typename T>
+static int leg_down_masked(fvx_mg* g, const T* f, const T* u_init, int k, cudaStream_t st) {
+  Lev<T>&L = levs<T>(g).L[0], &C = levs<T>(g).L[1];
+  const size_t n = (size_t)L.ny * L.nx;
+  if (u_init) copy_kernel<T><<<grid_for(n), 256, 0, st>>>(L.u, u_init, n);
+  else fill_kernel<T><<<grid_for(n), 256, 0, st>>>(L.u, n, T(0));
+  sweeps_masked<T>(g, f, k, st);
+  restrict_kernel<T><<<grid_for((size_t)C.ny * C.nx), 256, 0, st>>>(L, L.u, f, C, C.f);
+  return fvx_cuda_status();
+}
+// ec_scale: ec is then level 1's u, scaled in place.
+template <typename T>
+static int leg_up_masked(fvx_mg* g, const T* f, const T* ec, int k, T* out, cudaStream_t st, const double* ec_scale) {
+  Lev<T>&L = levs<T>(g).L[0], &C = levs<T>(g).L[1];
+  const size_t n = (size_t)L.ny * L.nx, nc = (size_t)C.ny * C.nx;
+  if (ec_scale) k_scale<T><<<grid_for(nc), 256, 0, st>>>(C.u, nc, ec_scale);
+  prolong_kernel<T><<<grid_for(n), 256, 0, st>>>(L, L.u, C, ec);
+  sweeps_masked<T>(g, f, k, st);
+  copy_kernel<T><<<grid_for(n), 256, 0, st>>>(out, L.u, n);
+  return fvx_cuda_status();
+}
+
 // Downward leg at host-driven level l: L.u <- k sweeps on f from u_init
 // (NULL = 0), level l+1's f <- the restricted residual.
 template <typename T>
 static int leg_down(fvx_mg* g, int l, const T* f, const T* u_init, int k, cudaStream_t st) {
   if (k > kLegMaxSweeps) return FVX_ERR_ARG;
+  if (l == 0 && !g->mask01) return leg_down_masked<T>(g, f, u_init, k, st);
   LevArray<T>& A = levs<T>(g);
   Lev<T>& L = A.L[l];
   const LegPlan pl = leg_plan<T>(L, k);
@@ -1492,6 +1529,7 @@ template <typename T>
 static int leg_up(fvx_mg* g, int l, const T* f, const T* ec, int k, T* out, cudaStream_t st,
                   const double* ec_scale = nullptr) {
   if (k > kLegMaxSweeps) return FVX_ERR_ARG;
+  if (l == 0 && !g->mask01) return leg_up_masked<T>(g, f, ec, k, out, st, ec_scale);
   LevArray<T>& A = levs<T>(g);
   Lev<T>& L = A.L[l];
   const LegPlan pl = leg_plan<T>(L, k);
