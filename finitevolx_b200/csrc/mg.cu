@@ -1253,7 +1253,11 @@ extern "C" int fvx_mg_create(const double* mask, const double* coeff, int ny, in
   const size_t n0 = (size_t)ny * nx;
   H[0].mask.assign(mask, mask + n0);
   H[0].coeff.resize(n0);
-  for (size_t c = 0; c < n0; ++c) H[0].coeff[c] = (coeff ? coeff[c] : 1.0) * H[0].mask[c];
+  bool fractional = false;
+  for (size_t c = 0; c < n0; ++c) {
+    H[0].coeff[c] = (coeff ? coeff[c] : 1.0) * mask[c];
+    fractional |= (mask[c] != 0.0) & (mask[c] != 1.0);
+  }
   for (int l = 0; l < n_levels; ++l) {
     host_level_ops(H[l], lambda);
     if (l + 1 < n_levels) {
@@ -1279,8 +1283,7 @@ extern "C" int fvx_mg_create(const double* mask, const double* coeff, int ny, in
   fvx_mg* g = new fvx_mg();
   g->nl = n_levels; g->n_pre = n_pre; g->n_post = n_post; g->n_coarse = n_coarse;
   g->omega = omega; g->lam = lambda; g->dtype = dtype;
-  for (size_t c = 0; c < n0; ++c)
-    if (mask[c] != 0.0 && mask[c] != 1.0) g->mask01 = false;
+  g->mask01 = !fractional;
   g->lc = n_levels - 1;
   while (g->lc > 0 && (size_t)H[g->lc - 1].ny * H[g->lc - 1].nx <= (size_t)kCoarseCells) --g->lc;
   int rc = dtype == 0 ? upload_levels<float>(g, H) : upload_levels<double>(g, H);
