@@ -1434,25 +1434,31 @@ extern "C" int fvx_nn_conv_fwd(const float* in, int mode, int batch, int cin, co
   return conv_fwd(in, mode, batch, cin, w_bf16, bias, skip, out, cout, h, w, relu, fvx_stream(stream), false);
 }
 
-template <int COT>
-static bool set_wgrad_smem() {
-  return fvx_set_max_smem(conv_wgrad_kernel<COT, 16>, (int)wgrad_smem_max(COT, 16)) &&
-         fvx_set_max_smem(conv_wgrad_kernel<COT, 8>, (int)wgrad_smem_max(COT, 8)) &&
-         fvx_set_max_smem(conv_wgrad_kernel<COT, 4>, (int)wgrad_smem_max(COT, 4));
+// Attributes are set on first use, so that only the instantiations that run
+// are loaded (a network uses five of the nine).
+template <int COT, int SR, typename... A>
+static int launch_wgrad_sr(int nrows, size_t wsm, cudaStream_t st, A... a) {
+  static fvx_once_per_device attr;
+  if (fvx_once_on_device(attr, [] {
+        return fvx_set_max_smem(conv_wgrad_kernel<COT, SR>, (int)wgrad_smem_max(COT, SR));
+      }))
+    return FVX_ERR_CUDA;
+  conv_wgrad_kernel<COT, SR><<<nrows, THREADS, wsm, st>>>(a...);
+  return FVX_OK;
 }
 template <int COT, typename... A>
-static void launch_wgrad(int sr, int nrows, size_t wsm, cudaStream_t st, A... a) {
-  if (sr == 16) conv_wgrad_kernel<COT, 16><<<nrows, THREADS, wsm, st>>>(a...);
-  else if (sr == 8) conv_wgrad_kernel<COT, 8><<<nrows, THREADS, wsm, st>>>(a...);
-  else conv_wgrad_kernel<COT, 4><<<nrows, THREADS, wsm, st>>>(a...);
+static int launch_wgrad(int sr, int nrows, size_t wsm, cudaStream_t st, A... a) {
+  if (sr == 16) return launch_wgrad_sr<COT, 16>(nrows, wsm, st, a...);
+  if (sr == 8) return launch_wgrad_sr<COT, 8>(nrows, wsm, st, a...);
+  return launch_wgrad_sr<COT, 4>(nrows, wsm, st, a...);
 }
 
 // Backward of one conv layer (wb: the BF16 weights of the forward pass).
 // dy: dL/dy (post-activation); y: the layer's output (for the ReLU mask).  Writes g (scratch [B, Cout, h, w]), adds the
 // skip gradient into dskip (if non-null), adds the input gradient into
 // dsrc (if non-null; dxin scratch [B, Cin, h, w]), and writes dW, db.
-// part: scratch of nblocks * Cout * (Cin * 9 + 1) floats.
-extern "C" int fvx_nn_conv_bwd_blocks(int batch, int h, int w);
+// part: scratch of fvx_nn_conv_bwd_rows * Cout * (Cin * 9 + 1) floats.
+extern "C" int fvx_nn_conv_bwd_rows(int batch, int cin, int cout, int h, int w);
 extern "C" int fvx_nn_conv_bwd(const float* in, int mode, int batch, int cin, const void* wb, const float* dy,
                                const float* y, int cout, int h, int w, int relu, float* g, float* dskip, float* dxin,
                                float* dsrc, float* dw, float* db, float* part, void* stream) {
@@ -1464,17 +1470,13 @@ extern "C" int fvx_nn_conv_bwd(const float* in, int mode, int batch, int cin, co
   act_grad_kernel<<<blocks_for(n), 256, 0, st>>>(dy, y, g, dskip, n, relu);
   dim3 gr((w + TILE - 1) / TILE, (h + TILE - 1) / TILE, batch);
   // weight and bias gradients: P partial rows, then their fixed-order sum
-  static fvx_once_per_device attr;
-  if (fvx_once_on_device(attr, [] {
-        return set_wgrad_smem<4>() && set_wgrad_smem<2>() && set_wgrad_smem<1>();
-      }))
-    return FVX_ERR_CUDA;
   const int cot = wgrad_cot(cin, cout), sr = wgrad_strip(cin, cout, batch, h, w);
-  const int nrows = (int)std::min<long long>(kWgradRows, std::max<long long>(1, wgrad_items(batch, h, w, sr)));
+  const int nrows = fvx_nn_conv_bwd_rows(batch, cin, cout, h, w);
   const size_t wsm = wgrad_smem(cin, cout, cot, sr);
-  if (cot == 4) launch_wgrad<4>(sr, nrows, wsm, st, in, mode, cin, g, cout, h, w, batch, part);
-  else if (cot == 2) launch_wgrad<2>(sr, nrows, wsm, st, in, mode, cin, g, cout, h, w, batch, part);
-  else launch_wgrad<1>(sr, nrows, wsm, st, in, mode, cin, g, cout, h, w, batch, part);
+  const int wrc = cot == 4   ? launch_wgrad<4>(sr, nrows, wsm, st, in, mode, cin, g, cout, h, w, batch, part)
+                  : cot == 2 ? launch_wgrad<2>(sr, nrows, wsm, st, in, mode, cin, g, cout, h, w, batch, part)
+                             : launch_wgrad<1>(sr, nrows, wsm, st, in, mode, cin, g, cout, h, w, batch, part);
+  if (wrc) return wrc;
   const int len = cout * (cin * 9 + 1);
   reduce_rows_kernel<<<(len + 31) / 32, 32 * kReduceWarps, 0, st>>>(part, nrows, len, cout * cin * 9, dw, db);
   if (dsrc) {
@@ -1505,8 +1507,15 @@ extern "C" int fvx_nn_conv_bwd(const float* in, int mode, int batch, int cin, co
   return fvx_cuda_status();
 }
 
-// Number of partial rows a conv_bwd call writes at most (scratch sizing):
-// one per (sample, 4 x 16 tile) item, at most kWgradRows.
+// Number of partial rows a conv_bwd call writes: one per (sample, strip)
+// item, at most kWgradRows; -1 for sizes it refuses.
+extern "C" int fvx_nn_conv_bwd_rows(int batch, int cin, int cout, int h, int w) {
+  if (batch < 1 || cin < 1 || cin > CMAX || cout < 1 || cout > CMAX || h < 1 || w < 1) return -1;
+  const long long items = wgrad_items(batch, h, w, wgrad_strip(cin, cout, batch, h, w));
+  return (int)std::min<long long>(kWgradRows, items);
+}
+
+// An upper bound of it for any channels: one per (sample, 4 x 16 tile) item.
 extern "C" int fvx_nn_conv_bwd_blocks(int batch, int h, int w) {
   const long long items = wgrad_items(batch, h, w, 4);
   return (int)(items < kWgradRows ? (items < 1 ? 1 : items) : kWgradRows);
@@ -1977,8 +1986,8 @@ extern "C" int fvx_unet_create(int h, int w, int batch_max, fvx_unet** out) {
     const int hh = h >> L.div, ww = w >> L.div;
     gmax = std::max(gmax, (size_t)batch_max * L.cout * hh * ww);
     xmax = std::max(xmax, (size_t)batch_max * L.cin * hh * ww);
-    const size_t nblk = (size_t)fvx_nn_conv_bwd_blocks(batch_max, hh, ww);
-    pmax = std::max(pmax, nblk * L.cout * ((size_t)L.cin * 9 + 1));
+    for (int b = 1; b <= batch_max; ++b)  // (fewer samples may take shorter strips)
+      pmax = std::max(pmax, (size_t)fvx_nn_conv_bwd_rows(b, L.cin, L.cout, hh, ww) * L.cout * ((size_t)L.cin * 9 + 1));
   }
   n->g = (float*)alloc(gmax * 4);
   n->dxin = (float*)alloc(xmax * 4);

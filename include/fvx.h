@@ -408,6 +408,9 @@ int fvx_nn_conv_fwd(const float* in, int mode, int batch, int cin, const void* w
 int fvx_nn_conv_bwd(const float* in, int mode, int batch, int cin, const void* w_bf16, const float* dy,
                     const float* y, int cout, int h, int w, int relu, float* g, float* dskip, float* dxin,
                     float* dsrc, float* dw, float* db, float* part, void* stream);
+/* Rows of Cout * (Cin * 9 + 1) floats that fvx_nn_conv_bwd writes into part,
+ * and an upper bound of them for any channels. */
+int fvx_nn_conv_bwd_rows(int batch, int cin, int cout, int h, int w);
 int fvx_nn_conv_bwd_blocks(int batch, int h, int w);
 int fvx_nn_mse(const float* pred, const float* target, const float* mask, long long plane, int batch, float* dpred,
                double* loss_dev, double mask_sum, void* stream);
