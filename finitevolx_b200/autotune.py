@@ -5,8 +5,8 @@ of several launches) through the library's own entry points and applies the
 fastest:
 
 * ``tune_qg_stage``: the fused QG stage kernel's tile shape (64x16, 32x16,
-  128x8, 64x32, 128x16 cells; the halo follows the scheme) for one scheme
-  and dtype.
+  128x8, 64x32, 128x16, 16x16 cells; the halo follows the scheme) of one
+  model.
 * ``tune_qg_split``: whether the stage kernel writes the next DST operand
   split itself (fused) or a separate split pass does (unfused).
 * ``tune_dst_kernel``: the even/odd DST product on single CTAs with 64- or
@@ -106,14 +106,19 @@ def _time_graph(fn_call, reps: int = 7, warm: int = 2, batch: int = 10) -> float
     return statistics.median(ts)
 
 
-def set_stage_tile(method: str, dtype: torch.dtype, cfg: int) -> None:
-    check(fn("fvx_qg_tile_config")(I(SCHEMES[method]), I(1 if dtype == torch.float64 else 0), I(cfg)),
-          "tile config")
+def set_stage_tile(method: str, dtype: torch.dtype, cfg: int | None) -> None:
+    """Tile of every stage of a scheme and dtype whose model has none of its
+    own (``QGModel.stage_tile``); None: by the field's size, as at the start."""
+    s, d = I(SCHEMES[method]), I(1 if dtype == torch.float64 else 0)
+    if cfg is None:
+        check(fn("fvx_qg_tile_by_size")(s, d), "tile config")
+    else:
+        check(fn("fvx_qg_tile_config")(s, d, I(cfg)), "tile config")
 
 
 def tune_qg_stage(model, q, dt: float, use_cache: bool = True) -> dict:
-    """Pick the stage kernel's tile shape for ``model`` (a QGModel) on
-    state ``q``; returns {"tile": name, "ms": {name: median ms per step}}.
+    """Pick the stage kernel's tile shape for ``model`` (a QGModel; others keep
+    theirs) on state ``q``; returns {"tile": name, "ms": {name: median ms per step}}.
     Candidates are timed as whole steps (graph-replayed): inside a step the
     stage reads inputs the DST products just wrote, which the stage timed
     alone does not reproduce (at 2048^2 the two orderings of 64x16 and
@@ -123,16 +128,16 @@ def tune_qg_stage(model, q, dt: float, use_cache: bool = True) -> dict:
     if use_cache:
         hit = _load().get(key)
         if hit:
-            set_stage_tile(model.method, model.dtype, _TILES.index(hit["tile"]))
+            model.stage_tile = _TILES.index(hit["tile"])
             return hit
     n_cfg = fn("fvx_qg_tile_config")(I(0), I(0), I(-1))
     out = torch.empty_like(q)
     ms = {}
     for cfg in range(n_cfg):
-        set_stage_tile(model.method, model.dtype, cfg)
+        model.stage_tile = cfg
         ms[_TILES[cfg]] = _time_graph(lambda: model.step(q, dt, out=out), batch=4)
     best = min(ms, key=ms.get)
-    set_stage_tile(model.method, model.dtype, _TILES.index(best))
+    model.stage_tile = _TILES.index(best)
     res = {"tile": best, "ms": ms}
     _store(key, res)
     return res

@@ -72,6 +72,9 @@ class QGModel:
         # the stage kernel writes the next DST operand split (False: a
         # separate split pass per solve); finitevolx_b200.autotune picks it
         self.fuse_split = True
+        # this model's stage tile (an index of autotune's _TILES); -1: the one
+        # set for the scheme and dtype, else by the field's size
+        self.stage_tile = -1
 
     # -- pieces --------------------------------------------------------------
     def _dst_from(self, q):
@@ -114,12 +117,11 @@ class QGModel:
         hi, lo = self._w1 if split else (ctypes.c_void_p(0), ctypes.c_void_p(0))
         if split and self._fused_copy64:
             hi = self._v1  # FP64: the interior copy for the FP64 chain
-        check(fn(f"fvx_qg_stage_{sfx(qs)}")(P(qs), P(qn), P(self.psi), P(self.forcing), P(out), hi, lo,
-                                            I(self._layout if split else 0), I(g.Ny),
-                                            I(g.Nx), D(g.dx), D(g.dy), D(self.beta), D(self.drag), D(self.visc),
-                                            D(a), D(b), D(c), I(SCHEMES[self.method]),
-                                            I(1 if self.bc == "periodic" else 0), I(int(write_ghost)),
-                                            stream_ptr()), "QG stage")
+        check(fn(f"fvx_qg_stage_tile_{sfx(qs)}")(P(qs), P(qn), P(self.psi), P(self.forcing), P(out), hi, lo,
+                                                 I(self._layout if split else 0), I(g.Ny), I(g.Nx), D(g.dx),
+                                                 D(g.dy), D(self.beta), D(self.drag), D(self.visc), D(a), D(b), D(c),
+                                                 I(SCHEMES[self.method]), I(1 if self.bc == "periodic" else 0),
+                                                 I(int(write_ghost)), I(self.stage_tile), stream_ptr()), "QG stage")
         self.kernel_launches += 1
 
     # -- public --------------------------------------------------------------

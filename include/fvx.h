@@ -287,6 +287,16 @@ int fvx_qg_stage_f64(const double* q_stage, const double* q_start, const double*
                      const double* forcing, double* q_out, void* split_hi, void* split_lo, int split_layout, int ny, int nx,
                      double dx, double dy, double beta, double drag, double viscosity, double a, double b,
                      double c, int method, int periodic, int write_ghost, void* stream);
+/* The same on a tile of the caller's choice (fvx_qg_tile_config's numbers; -1:
+ * as fvx_qg_stage). */
+int fvx_qg_stage_tile_f32(const float* q_stage, const float* q_start, const float* psi_interior,
+                          const float* forcing, float* q_out, void* split_hi, void* split_lo, int split_layout,
+                          int ny, int nx, double dx, double dy, double beta, double drag, double viscosity, double a,
+                          double b, double c, int method, int periodic, int write_ghost, int tile, void* stream);
+int fvx_qg_stage_tile_f64(const double* q_stage, const double* q_start, const double* psi_interior,
+                          const double* forcing, double* q_out, void* split_hi, void* split_lo, int split_layout,
+                          int ny, int nx, double dx, double dy, double beta, double drag, double viscosity, double a,
+                          double b, double c, int method, int periodic, int write_ghost, int tile, void* stream);
 
 /* ---- masked multigrid, PCG, vertical modes -------------------------------- */
 
@@ -429,10 +439,15 @@ int fvx_qg_snapshot_pack_f64(const double* q, const double* psi, const double* u
                              const double* z, int ny, int nx, double eta_scale, double* out, void* stream);
 
 /* ---- QG fused-stage tile shape (autotuner) -------------------------------- */
-/* cfg 0 = 64x16, 1 = 32x16, 2 = 128x8, 3 = 64x32, 4 = 128x16, 5 = 16x16 cells for (method, dtype 0 FP32 / 1
- * FP64), until the first call chosen by the size of the field; cfg < 0 returns the number of configurations.  No counterpart in
- * finitevolX (launch configuration). */
+/* Tile of the stage calls that name none, per scheme and dtype (0 FP32, 1
+ * FP64): cfg 0 = 64x16, 1 = 32x16, 2 = 128x8, 3 = 64x32, 4 = 128x16, 5 = 16x16
+ * cells; cfg < 0 returns the number of configurations.  Until it is called,
+ * and after fvx_qg_tile_by_size, the field's size decides; fvx_qg_tile_for
+ * gives the tile a call would run.  No counterpart in finitevolX (launch
+ * configuration). */
 int fvx_qg_tile_config(int method, int dtype, int cfg);
+int fvx_qg_tile_by_size(int method, int dtype);
+int fvx_qg_tile_for(int method, int dtype, int ny, int nx);
 
 /* ---- ensemble of multi-layer QG members ------------------------------------ */
 /* Members (n[m]^2 interior, nl[m] <= 3 layers; l2m/m2l row-major nl x nl per

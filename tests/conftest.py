@@ -18,3 +18,17 @@ def cuda_ok():
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     return True
+
+
+@pytest.fixture(autouse=True)
+def _stage_tiles_by_size(request):
+    """A GPU test that sets a stage tile for its scheme leaves none behind."""
+    yield
+    if request.node.get_closest_marker("gpu"):
+        import torch
+        from finitevolx_b200 import autotune
+        from finitevolx_b200._lib import LIB_PATH, SCHEMES
+        if LIB_PATH.exists():
+            for method in SCHEMES:
+                for dtype in (torch.float32, torch.float64):
+                    autotune.set_stage_tile(method, dtype, None)
