@@ -9,9 +9,9 @@ fastest:
   model.
 * ``tune_qg_split``: whether the stage kernel writes the next DST operand
   split itself (fused) or a separate split pass does (unfused).
-* ``tune_dst_kernel``: the even/odd DST product on single CTAs with 64- or
-  32-element K blocks (3 or 6 ring stages) or on CTA pairs (cta_group::2,
-  each pair sharing its B blocks).
+* ``tune_dst_kernel``: one model's even/odd DST products on single CTAs with
+  64- or 32-element K blocks (3 or 6 ring stages) or on CTA pairs
+  (cta_group::2, each pair sharing its B blocks).
 * ``tune_ensemble``: the persistent work-queue grid (CTAs per SM).
 
 Results are cached in a JSON file keyed by device name and workload
@@ -170,29 +170,30 @@ DST_KERNELS = ("single64", "pair", "single32")
 
 
 def set_dst_kernel(kind) -> None:
-    """``kind``: one of DST_KERNELS (or its index)."""
+    """Product form of every plan that has none of its own; ``kind``: one of
+    DST_KERNELS (or its index)."""
     k = DST_KERNELS.index(kind) if isinstance(kind, str) else int(kind)
     check(fn("fvx_dst_kernel_config")(I(k)), "dst kernel config")
 
 
 def tune_dst_kernel(model, q, dt: float, use_cache: bool = True) -> dict:
-    """The even/odd DST product forms timed over whole QG steps of ``model``
-    (a QGModel); returns {"kernel": name, "ms": {name: median ms}}."""
+    """The even/odd DST product forms timed over whole QG steps of ``model`` (a
+    QGModel), whose plan takes the fastest (others keep theirs); returns {"kernel": name, "ms": {name: median ms}}."""
     g = model.grid
     key = f"{_device_key()}/dst_kernel/{model.dtype}/{g.Ny}x{g.Nx}"
     if use_cache:
         hit = _load().get(key)
         if hit and hit.get("kernel") in DST_KERNELS:
-            set_dst_kernel(hit["kernel"])
+            model.plan.set_kernel(DST_KERNELS.index(hit["kernel"]))
             return hit
     out = torch.empty_like(q)
 
     ms = {}
-    for name in DST_KERNELS:
-        set_dst_kernel(name)
+    for k, name in enumerate(DST_KERNELS):
+        model.plan.set_kernel(k)
         ms[name] = _time_graph(lambda: model.step(q, dt, out=out), batch=4)
     best = min(ms, key=ms.get)
-    set_dst_kernel(best)
+    model.plan.set_kernel(DST_KERNELS.index(best))
     res = {"kernel": best, "ms": ms}
     _store(key, res)
     return res

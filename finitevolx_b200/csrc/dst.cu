@@ -1309,15 +1309,17 @@ static bool make_out_map(CUtensorMap* map, void* base, bool f32, uint64_t R, uin
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Which even/odd kernel runs (fvx_dst_kernel_config): 0 = single CTAs with
-// 64-element K blocks (default), 1 = CTA pairs (row counts that are
-// multiples of 256), 2 = single CTAs with 32-element K blocks.
+// Which even/odd kernel the plans without one of their own run
+// (fvx_dst_kernel_config, fvx_dst_plan_kernel): 0 = single CTAs with 64-element
+// K blocks (default; with the folded and walking forms by size), 1 = CTA pairs
+// (row counts that are multiples of 256), 2 = single CTAs with 32-element K
+// blocks.
 static int g_sym_kernel = 0;
 
 // C[M, K] = X[M, K] S[K, K] by the even/odd product; X's columns
 // de-interleaved; P/Q: the [K/2][K/2] hi/lo tables.  Needs K % 256 == 0.
-static int gemm_sym(const bf16* Xh, const bf16* Xl, int M, int K, const bf16* Ph, const bf16* Pl, const bf16* Qh,
-                    const bf16* Ql, const Epi& ep_in, cudaStream_t st) {
+static int gemm_sym(int kind, const bf16* Xh, const bf16* Xl, int M, int K, const bf16* Ph, const bf16* Pl,
+                    const bf16* Qh, const bf16* Ql, const Epi& ep_in, cudaStream_t st) {
   Epi ep = ep_in;
   static fvx_once_per_device attr;
   if (fvx_once_on_device(attr, [] {
@@ -1327,7 +1329,7 @@ static int gemm_sym(const bf16* Xh, const bf16* Xl, int M, int K, const bf16* Ph
     return FVX_ERR_CUDA;
   if (K % (2 * SBN) != 0) return FVX_ERR_SHAPE;
   const int KH = K / 2;
-  const uint32_t bki = g_sym_kernel == 2 ? 32 : 64;  // K block of the single-CTA forms
+  const uint32_t bki = kind == 2 ? 32 : 64;  // K block of the single-CTA forms
   CUtensorMap a_h, a_l, p_h, p_l, q_h, q_l;
   if (!make_map(&a_h, Xh, K, M, BM, bki) || !make_map(&a_l, Xl, K, M, BM, bki) ||
       !make_map(&p_h, Ph, KH, KH, SBN, bki) || !make_map(&p_l, Pl, KH, KH, SBN, bki) ||
@@ -1344,7 +1346,7 @@ static int gemm_sym(const bf16* Xh, const bf16* Xl, int M, int K, const bf16* Ph
   // takes 279 us against 330 with a CTA per tile, 4 of 2048^2 451 against
   // 505.  Up to one tile per SM nothing overlaps (16 of 512^2, 128 tiles).
   const long long tiles = (long long)(KH / SBN) * ((M + BM - 1) / BM);
-  bool walk = g_sym_kernel == 0 && tiles > kSMs && tiles <= INT_MAX;
+  bool walk = kind == 0 && tiles > kSMs && tiles <= INT_MAX;
   const uint32_t box_n = walk ? T_COLS : 16;
   if ((ep.mode == EPI_SPLIT || ep.mode == EPI_F32) && R % BM == 0 && M % R == 0 && ep.off_n == 0 &&
       ep.off_r == 0 && ep.n_cols == K && (ep.mode == EPI_F32 || ep.perm_r)) {
@@ -1364,7 +1366,7 @@ static int gemm_sym(const bf16* Xh, const bf16* Xl, int M, int K, const bf16* Ph
       return FVX_ERR_CUDA;
     return fvx_cuda_status();
   }
-  if (M % (2 * BM) == 0 && g_sym_kernel == 1) {
+  if (M % (2 * BM) == 0 && kind == 1) {
     // CTA pairs: B blocks of 64 table rows per CTA
     static fvx_once_per_device pattr;
     if (fvx_once_on_device(pattr, [] { return fvx_set_max_smem(gemm_sym_pair_kernel, P_SMEM); }))
@@ -1447,6 +1449,7 @@ struct fvx_dst_plan {
   bool split_ok;
   std::vector<double> lam_host;
   double* lam_dev = nullptr;
+  int kernel = -1;   // even/odd kernel of this plan, -1: the process's
   bool sym = false;  // nx, ny multiples of 256: the workspace W1 is public in the products' layout
   // Folded transforms (dst_f64.cuh): hx, hy table rows (half lengths), kx,
   // ky folded axis lengths 2 hx, 2 hy (the spectral axes: nx, ny except for
@@ -1734,8 +1737,9 @@ static int split_product(fvx_dst_plan* p, const bf16* Xh, const bf16* Xl, bool a
   const FoldTables& t = along_x ? (inverse ? p->ix : p->fx) : (inverse ? p->iy : p->fy);
   const int M = ep.m_total;
   const long long c32 = fold_cost(32, h, M), c64 = fold_cost(64, h, M), c128 = fold_cost(128, h, M);
-  if (p->sym && (g_sym_kernel != 0 || c128 <= std::min(c32, c64)))
-    return gemm_sym(Xh, Xl, M, 2 * h, t.Ph, t.Pl, t.Qh, t.Ql, ep, st);
+  const int kind = p->kernel < 0 ? g_sym_kernel : p->kernel;
+  if (p->sym && (kind != 0 || c128 <= std::min(c32, c64)))
+    return gemm_sym(kind, Xh, Xl, M, 2 * h, t.Ph, t.Pl, t.Qh, t.Ql, ep, st);
   FoldEpi fe;
   fe.e = ep;
   fe.nh = h;
@@ -2001,16 +2005,21 @@ extern "C" int fvx_dst_solve_f64(fvx_dst_plan* p, const double* rhs, long long r
   return be <= tol ? FVX_OK : FVX_ERR_NOT_CONVERGED;
 }
 
-// One product of the split chain on the plan's workspaces, for timing the
-// tensor-core GEMM in isolation: which 0 = (W1 S_x)^T -> W2, 1 = (W2 S_y) ./
-// Lambda -> W1.  Operands are whatever the workspaces currently hold.
 extern "C" int fvx_dst_kernel_config(int kind) {
   if (kind < 0) return g_sym_kernel;
   if (kind > 2) return FVX_ERR_ARG;
   g_sym_kernel = kind;
   return FVX_OK;
 }
+extern "C" int fvx_dst_plan_kernel(fvx_dst_plan* p, int kind) {
+  if (!p || kind < -1 || kind > 2) return FVX_ERR_ARG;
+  p->kernel = kind;
+  return FVX_OK;
+}
 
+// One product of the split chain on the plan's workspaces, for timing the
+// tensor-core GEMM in isolation: which 0 = (W1 S_x)^T -> W2, 1 = (W2 S_y) ./
+// Lambda -> W1.  Operands are whatever the workspaces currently hold.
 extern "C" int fvx_dst_gemm_step(fvx_dst_plan* p, int which, int batch, void* stream) {
   if (!p || !p->split_ok) return FVX_ERR_ARG;
   if (batch < 1 || batch > p->batch_max) return FVX_ERR_SHAPE;

@@ -134,6 +134,11 @@ class DSTHelmholtzPlan:
         """Bound, in SM clock cycles, on each barrier wait of the products."""
         check(fn("fvx_dst_plan_set_wait_limit")(self._h, ctypes.c_longlong(int(cycles))), "wait limit")
 
+    def set_kernel(self, kind: int) -> None:
+        """Even/odd product kernel of this plan (an index of autotune's
+        DST_KERNELS); -1: the process's choice."""
+        check(fn("fvx_dst_plan_kernel")(self._h, I(int(kind))), "dst kernel")
+
 
 _CACHE: dict = {}
 

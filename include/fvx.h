@@ -231,13 +231,15 @@ int fvx_dst_solve_presplit_f64(fvx_dst_plan* plan, double* psi, long long psi_bs
 int fvx_dst_operand_layout(fvx_dst_plan* plan);
 /* One product of the chain on the current workspaces (timing only). */
 int fvx_dst_gemm_step(fvx_dst_plan* plan, int which, int batch, void* stream);
-/* Even/odd product kernel (process-wide, for the autotuner): 0 = one CTA
- * per 128-row tile with 64-element K blocks (3 ring stages, default), 1 =
- * CTA pairs sharing each B block (cta_group::2; row counts that are
- * multiples of 256), 2 = one CTA per tile with 32-element K blocks (6 ring
- * stages); kind < 0 returns the current choice.  No counterpart in
- * finitevolX (launch configuration). */
+/* Even/odd product kernel of the plans that have none of their own: 0 = one
+ * CTA per 128-row tile with 64-element K blocks (3 ring stages, default; by
+ * size also the folded 32- and 64-row tiles and the tile walk), 1 = CTA pairs
+ * sharing each B block (cta_group::2; row counts that are multiples of 256), 2
+ * = one CTA per tile with 32-element K blocks (6 ring stages); kind < 0
+ * returns the current choice.  fvx_dst_plan_kernel sets one plan's (-1: as the
+ * process).  No counterpart in finitevolX (launch configuration). */
 int fvx_dst_kernel_config(int kind);
+int fvx_dst_plan_kernel(fvx_dst_plan* plan, int kind);
 
 /* Allocation-free FP32 DST Helmholtz solve.  No counterpart in the
  * reference: it serves callers that cannot call cudaMalloc while they run
