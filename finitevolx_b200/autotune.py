@@ -14,20 +14,24 @@ fastest:
   (cta_group::2, each pair sharing its B blocks).
 * ``tune_ensemble``: the persistent work-queue grid (CTAs per SM).
 
-Results are cached in a JSON file keyed by device name and workload
-(``FVX_AUTOTUNE_CACHE``, default ``~/.cache/finitevolx_b200/autotune.json``)
-so later runs reuse them without timing.
+Results are cached in a JSON file keyed by device name, build of the library
+and workload (``FVX_AUTOTUNE_CACHE``, default
+``~/.cache/finitevolx_b200/autotune.json``) so later runs reuse them without
+timing; kernels that were rebuilt are timed anew.
 """
 
 from __future__ import annotations
 
+import functools
 import json
 import os
 import pathlib
 import statistics
+import zlib
 
 import torch
 
+from finitevolx_b200 import _lib
 from finitevolx_b200._lib import I, SCHEMES, check, fn
 
 _TILES = ("64x16", "32x16", "128x8", "64x32", "128x16", "16x16")
@@ -58,6 +62,20 @@ def _store(key: str, value) -> None:
 
 def _device_key() -> str:
     return torch.cuda.get_device_name(torch.cuda.current_device()).replace(" ", "_")
+
+
+@functools.lru_cache(maxsize=4)
+def _file_crc(path: str, mtime_ns: int) -> str:
+    return f"{zlib.crc32(pathlib.Path(path).read_bytes()):08x}"
+
+
+def _build_key() -> str:
+    """The library's contents: choices timed on other kernels do not apply."""
+    return _file_crc(str(_lib.LIB_PATH), _lib.LIB_PATH.stat().st_mtime_ns)
+
+
+def _key(kind: str, *parts) -> str:
+    return "/".join([_device_key(), _build_key(), kind, *map(str, parts)])
 
 
 def _time(fn_call, reps: int = 7, warm: int = 2, batch: int = 5) -> float:
@@ -124,7 +142,7 @@ def tune_qg_stage(model, q, dt: float, use_cache: bool = True) -> dict:
     alone does not reproduce (at 2048^2 the two orderings of 64x16 and
     64x32 disagree)."""
     g = model.grid
-    key = f"{_device_key()}/qg_stage/{model.method}/{model.dtype}/{g.Ny}x{g.Nx}"
+    key = _key("qg_stage", model.method, model.dtype, f"{g.Ny}x{g.Nx}")
     if use_cache:
         hit = _load().get(key)
         if hit:
@@ -148,7 +166,7 @@ def tune_qg_split(model, q, dt: float, use_cache: bool = True) -> dict:
     (a separate split pass before each DST) for whole steps; sets
     ``model.fuse_split`` and returns {"fused": bool, "ms": {...}}."""
     g = model.grid
-    key = f"{_device_key()}/qg_split/{model.method}/{model.dtype}/{g.Ny}x{g.Nx}"
+    key = _key("qg_split", model.method, model.dtype, f"{g.Ny}x{g.Nx}")
     if use_cache:
         hit = _load().get(key)
         if hit:
@@ -180,7 +198,7 @@ def tune_dst_kernel(model, q, dt: float, use_cache: bool = True) -> dict:
     """The even/odd DST product forms timed over whole QG steps of ``model`` (a
     QGModel), whose plan takes the fastest (others keep theirs); returns {"kernel": name, "ms": {name: median ms}}."""
     g = model.grid
-    key = f"{_device_key()}/dst_kernel/{model.dtype}/{g.Ny}x{g.Nx}"
+    key = _key("dst_kernel", model.dtype, f"{g.Ny}x{g.Nx}")
     if use_cache:
         hit = _load().get(key)
         if hit and hit.get("kernel") in DST_KERNELS:
@@ -202,7 +220,7 @@ def tune_dst_kernel(model, q, dt: float, use_cache: bool = True) -> dict:
 def tune_ensemble(ens, candidates=(0, 1, 2, 4), steps: int = 3, use_cache: bool = True) -> dict:
     """Persistent-grid occupancy for a QGEnsemble (0 = as many CTAs as fit)."""
     sig = ",".join(f"{n}:{nl}" for n, nl in ens.members)
-    key = f"{_device_key()}/ensemble/{ens.method}/{hash(sig) & 0xffffffff:08x}"
+    key = _key("ensemble", ens.method, f"{hash(sig) & 0xffffffff:08x}")
     if use_cache:
         hit = _load().get(key)
         if hit:
