@@ -217,10 +217,14 @@ def tune_dst_kernel(model, q, dt: float, use_cache: bool = True) -> dict:
     return res
 
 
+def _ensemble_key(ens) -> str:
+    sig = ",".join(f"{n}:{nl}" for n, nl in ens.members)
+    return _key("ensemble", ens.method, f"{zlib.crc32(sig.encode()):08x}")
+
+
 def tune_ensemble(ens, candidates=(0, 1, 2, 4), steps: int = 3, use_cache: bool = True) -> dict:
     """Persistent-grid occupancy for a QGEnsemble (0 = as many CTAs as fit)."""
-    sig = ",".join(f"{n}:{nl}" for n, nl in ens.members)
-    key = _key("ensemble", ens.method, f"{hash(sig) & 0xffffffff:08x}")
+    key = _ensemble_key(ens)
     if use_cache:
         hit = _load().get(key)
         if hit:
