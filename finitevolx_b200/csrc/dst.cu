@@ -1644,7 +1644,12 @@ extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, dou
     A((void**)&p->Fx64, sizeof(double) * tx); A((void**)&p->Fy64, sizeof(double) * ty);
     if (!dst) { A((void**)&p->Ix64, sizeof(double) * tx); A((void**)&p->Iy64, sizeof(double) * ty); }
   }
-  if (!ok) { dst_free(p); delete p; return FVX_ERR_CUDA; }
+  if (!ok) {
+    dst_free(p);
+    delete p;
+    cudaGetLastError();  // out of memory: reported here, not by the next launch
+    return FVX_ERR_CUDA;
+  }
   std::vector<double> F, I, e;
   folded_tables(kind, nx, dx, p->hx, p->kx, F, I, e);
   ok = upload(p->ex64, e);

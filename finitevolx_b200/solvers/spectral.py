@@ -25,6 +25,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
 
 import numpy as np
 import torch
@@ -45,6 +46,8 @@ class DSTHelmholtzPlan:
 
     Creating a plan allocates device memory once; ``solve`` allocates
     nothing on the device besides its output (pass ``out=`` to avoid that).
+    A plan has one set of workspaces: threads may share it on one stream, but
+    a stream of its own needs a plan of its own (as the solve_* functions have).
     """
 
     def __init__(self, ny: int, nx: int, dx: float, dy: float, lambdas=(0.0,), batch_max: int = 1,
@@ -57,6 +60,7 @@ class DSTHelmholtzPlan:
         self.bc = bc
         self.lambdas = lam
         self.batch_max = int(batch_max)
+        self._lock = threading.Lock()  # a solve's launches stay together
         self._h = ctypes.c_void_p()
         lam_c = (ctypes.c_double * len(lam))(*lam.tolist())
         check(fn("fvx_spectral_plan_create")(I(KINDS[bc]), I(self.ny), I(self.nx), D(self.dx), D(self.dy),
@@ -92,14 +96,17 @@ class DSTHelmholtzPlan:
         out = torch.empty_like(rhs) if out is None else out
         plane = self.ny * self.nx
         if rhs.dtype == torch.float32:
-            check(fn("fvx_dst_solve_f32")(self._h, P(rhs), I64(plane), I64(self.nx), P(out), I64(plane),
-                                          I64(self.nx), I(b), stream_ptr()), "solve_helmholtz_dst")
+            with self._lock:
+                st = fn("fvx_dst_solve_f32")(self._h, P(rhs), I64(plane), I64(self.nx), P(out), I64(plane),
+                                             I64(self.nx), I(b), stream_ptr())
+            check(st, "solve_helmholtz_dst")
         elif rhs.dtype == torch.float64:
             m = {"fp64": 0, "refine": 1}[method]
             info = (ctypes.c_double * 3)()
-            check(fn("fvx_dst_solve_f64")(self._h, P(rhs), I64(plane), I64(self.nx), P(out), I64(plane),
-                                          I64(self.nx), I(b), I(m), D(1e-12), I(8), info, stream_ptr()),
-                  "solve_helmholtz_dst")
+            with self._lock:
+                st = fn("fvx_dst_solve_f64")(self._h, P(rhs), I64(plane), I64(self.nx), P(out), I64(plane),
+                                             I64(self.nx), I(b), I(m), D(1e-12), I(8), info, stream_ptr())
+            check(st, "solve_helmholtz_dst")
         else:
             raise TypeError(f"unsupported dtype {rhs.dtype}")
         return out
@@ -117,8 +124,9 @@ class DSTHelmholtzPlan:
         out = torch.empty_like(rhs) if out is None else out
         plane = self.ny * self.nx
         info = (ctypes.c_double * 3)()
-        st = fn("fvx_dst_solve_f64")(self._h, P(rhs), I64(plane), I64(self.nx), P(out), I64(plane), I64(self.nx),
-                                     I(b), I(1), D(tol), I(max_iter), info, stream_ptr())
+        with self._lock:
+            st = fn("fvx_dst_solve_f64")(self._h, P(rhs), I64(plane), I64(self.nx), P(out), I64(plane), I64(self.nx),
+                                         I(b), I(1), D(tol), I(max_iter), info, stream_ptr())
         res = dict(passes=int(info[0]), backward_error=float(info[1]), rel_residual=float(info[2]),
                    converged=st == 0)
         if st not in (0, 5):
@@ -140,7 +148,47 @@ class DSTHelmholtzPlan:
         check(fn("fvx_dst_plan_kernel")(self._h, I(int(kind))), "dst kernel")
 
 
-_CACHE: dict = {}
+class _PlanPool:
+    """The plans behind ``get_plan``: one per problem and stream, because a plan's
+    workspaces serve one stream at a time, each as large as the largest batch
+    asked of it.  A problem keeps the plans of at most ``STREAMS`` streams (all
+    that PyTorch hands out, and the default one); the oldest goes first.
+
+    ``make(key, batch, fp64)`` creates a plan."""
+
+    STREAMS = 33
+
+    def __init__(self, make):
+        self._make, self._plans, self._lock = make, {}, threading.Lock()
+
+    def get(self, key, stream: int, batch: int, fp64: bool, capturing: bool):
+        p = self._plans.get((key, stream))
+        if p is not None and p.batch_max >= batch:
+            return p
+        with self._lock:
+            p = self._plans.get((key, stream))
+            if p is not None and p.batch_max >= batch:
+                return p
+            others = [k for k in self._plans if k[0] == key and k[1] != stream]
+            if capturing:  # nothing can be allocated: a plan made on another stream
+                for k in others:
+                    if self._plans[k].batch_max >= batch:
+                        return self._plans[k]
+            elif p is None and len(others) >= self.STREAMS:
+                del self._plans[others.pop(0)]
+            try:
+                p = self._make(key, batch, fp64)
+            except L.FvxError:
+                if capturing or not others:
+                    raise
+                for k in others:  # give the other streams' memory back and try again
+                    del self._plans[k]
+                p = self._make(key, batch, fp64)
+            self._plans[(key, stream)] = p
+            return p
+
+
+_POOL = _PlanPool(lambda key, batch, fp64: DSTHelmholtzPlan(*key[1:6], batch_max=max(batch, 1), fp64=fp64, bc=key[0]))
 
 
 SpectralHelmholtzPlan = DSTHelmholtzPlan
@@ -156,13 +204,11 @@ def _lambda_tuple(lam) -> tuple:
 
 
 def get_plan(ny, nx, dx, dy, lambdas, batch, fp64=True, bc: str = "dst") -> DSTHelmholtzPlan:
-    lam = _lambda_tuple(lambdas)
-    key = (bc, ny, nx, float(dx), float(dy), lam, torch.cuda.current_device())
-    p = _CACHE.get(key)
-    if p is None or p.batch_max < batch:
-        p = DSTHelmholtzPlan(ny, nx, dx, dy, lam, batch_max=max(batch, 1), fp64=fp64, bc=bc)
-        _CACHE[key] = p
-    return p
+    """The current stream's plan of a problem, for up to ``batch`` fields."""
+    dev = torch.cuda.current_device()
+    key = (bc, ny, nx, float(dx), float(dy), _lambda_tuple(lambdas), dev)
+    return _POOL.get(key, torch._C._cuda_getCurrentRawStream(dev), batch, fp64,
+                     torch.cuda.is_current_stream_capturing())
 
 
 def _solve(rhs, dx, dy, lambda_, method, bc):
