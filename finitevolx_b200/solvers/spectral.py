@@ -68,6 +68,7 @@ class DSTHelmholtzPlan:
                                              ctypes.byref(self._h)),
               "SpectralHelmholtzPlan")
         self.split_ok = (self.nx % 8 == 0) and (self.ny % 8 == 0)
+        self.fp64 = bool(fp64) or not self.split_ok  # has the FP64 chain
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -161,21 +162,27 @@ class _PlanPool:
     def __init__(self, make):
         self._make, self._plans, self._lock = make, {}, threading.Lock()
 
+    @staticmethod
+    def _serves(p, batch, fp64) -> bool:
+        return p is not None and p.batch_max >= batch and (p.fp64 or not fp64)
+
     def get(self, key, stream: int, batch: int, fp64: bool, capturing: bool):
         p = self._plans.get((key, stream))
-        if p is not None and p.batch_max >= batch:
+        if self._serves(p, batch, fp64):
             return p
         with self._lock:
             p = self._plans.get((key, stream))
-            if p is not None and p.batch_max >= batch:
+            if self._serves(p, batch, fp64):
                 return p
             others = [k for k in self._plans if k[0] == key and k[1] != stream]
             if capturing:  # nothing can be allocated: a plan made on another stream
                 for k in others:
-                    if self._plans[k].batch_max >= batch:
+                    if self._serves(self._plans[k], batch, fp64):
                         return self._plans[k]
             elif p is None and len(others) >= self.STREAMS:
                 del self._plans[others.pop(0)]
+            if p is not None:  # replaced by one that serves its callers too
+                batch, fp64 = max(batch, p.batch_max), fp64 or p.fp64
             try:
                 p = self._make(key, batch, fp64)
             except L.FvxError:

@@ -68,3 +68,12 @@ def test_capture_after_use(cuda_ok):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, ref)
+
+
+def test_fp64_after_an_fp32_only_plan(cuda_ok):
+    from finitevolx_b200.solvers.spectral import get_plan
+    f = _fields(1, torch.float64, (24, 40))[0]
+    want = solve_helmholtz_dst(f, 0.1, 0.2, 1.5)
+    get_plan(24, 40, 0.1, 0.2, (1.75,), 1, fp64=False)
+    got = get_plan(24, 40, 0.1, 0.2, (1.75,), 1).solve(f)
+    assert torch.equal(got, solve_helmholtz_dst(f, 0.1, 0.2, 1.75)) and not torch.equal(got, want)

@@ -81,3 +81,13 @@ def test_capture_uses_a_plan_made_before():
     pool = _PlanPool(Plan)
     a = pool.get("p", 0, 2, True, False)
     assert pool.get("p", 9, 2, True, True) is a
+
+
+def test_fp64_is_part_of_the_request():
+    pool = _PlanPool(Plan)
+    a = pool.get("p", 0, 4, False, False)
+    b = pool.get("p", 0, 1, True, False)
+    assert b.fp64 and b.batch_max == 4
+    assert pool.get("p", 0, 4, False, False) is b and pool.get("p", 0, 2, True, False) is b and a is not b
+    pool.get("p", 1, 1, False, False)
+    assert pool.get("p", 2, 1, True, True) is b  # a capture takes one that has it
