@@ -25,10 +25,12 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstring>
 #include <cstdio>
+#include <memory>
 #include <vector>
 
 namespace fvx {
@@ -1449,6 +1451,7 @@ struct fvx_dst_plan {
   bool split_ok;
   std::vector<double> lam_host;
   double* lam_dev = nullptr;
+  std::shared_ptr<std::atomic<int>> holds = std::make_shared<std::atomic<int>>(0);  // graphs that use the plan
   int kernel = -1;   // even/odd kernel of this plan, -1: the process's
   bool sym = false;  // nx, ny multiples of 256: the workspace W1 is public in the products' layout
   // Folded transforms (dst_f64.cuh): hx, hy table rows (half lengths), kx,
@@ -1555,12 +1558,13 @@ static void folded_tables(int kind, int n, double d, int h, int k, std::vector<d
   for (int j = 0; j < h; ++j) e[2 * j] = e[2 * j + 1] = eig(M_PI * j / (double)n);
 }
 
-static bool upload(double* dev, const std::vector<double>& v) {
-  return cudaMemcpy(dev, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+// (A copy from pageable memory returns once the source has been staged.)
+static bool upload(double* dev, const std::vector<double>& v, cudaStream_t st) {
+  return cudaMemcpyAsync(dev, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice, st) == cudaSuccess;
 }
 // Even columns of a folded table to P, odd ones to Q, split into bf16 hi / lo
 // rows of `half` elements.
-static bool upload_split(const FoldTables& t, const std::vector<double>& F, int h, int k, int half) {
+static bool upload_split(const FoldTables& t, const std::vector<double>& F, int h, int k, int half, cudaStream_t st) {
   std::vector<bf16> b[4];
   for (auto& v : b) v.assign((size_t)h * half, __float2bfloat16_rn(0.f));
   for (int r = 0; r < h; ++r)
@@ -1573,7 +1577,8 @@ static bool upload_split(const FoldTables& t, const std::vector<double>& F, int 
       }
   bf16* dev[4] = {t.Ph, t.Pl, t.Qh, t.Ql};
   for (int q = 0; q < 4; ++q)
-    if (cudaMemcpy(dev[q], b[q].data(), sizeof(bf16) * b[q].size(), cudaMemcpyHostToDevice) != cudaSuccess) return false;
+    if (cudaMemcpyAsync(dev[q], b[q].data(), sizeof(bf16) * b[q].size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
+      return false;
   return true;
 }
 
@@ -1589,6 +1594,22 @@ __global__ void inv_eig_kernel(const double* __restrict__ ey, const double* __re
     }
 }
 
+// A plan may be created while a stream of the process is being captured: its
+// set-up runs on a stream of its own, and this thread may allocate meanwhile.
+struct PlanSetup {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaStream_t st = nullptr;
+  bool ok;
+  PlanSetup() {
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess;
+  }
+  ~PlanSetup() {
+    if (ok) cudaStreamDestroy(st);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+};
+
 extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, double dy, int batch_max,
                                         const double* lambdas, int n_lambda, int want_fp64, fvx_dst_plan** out);
 
@@ -1603,6 +1624,7 @@ extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, dou
   *out = nullptr;
   if (kind != FVX_SPECTRAL_DST && kind != FVX_SPECTRAL_DCT && kind != FVX_SPECTRAL_PERIODIC) return FVX_ERR_METHOD;
   if (ny < 1 || nx < 1 || batch_max < 1 || n_lambda < 1) return FVX_ERR_SHAPE;
+  PlanSetup up;
   fvx_dst_plan* p = new fvx_dst_plan();
   p->kind = kind;
   p->ny = ny; p->nx = nx; p->dx = dx; p->dy = dy; p->batch_max = batch_max; p->n_lam = n_lambda;
@@ -1652,23 +1674,22 @@ extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, dou
   }
   std::vector<double> F, I, e;
   folded_tables(kind, nx, dx, p->hx, p->kx, F, I, e);
-  ok = upload(p->ex64, e);
-  if (want64) ok = ok && upload(p->Fx64, F) && (dst || upload(p->Ix64, I));
-  if (p->split_ok) ok = ok && upload_split(p->fx, F, p->hx, p->kx, p->halfx) &&
-                        (dst || upload_split(p->ix, I, p->hx, p->kx, p->halfx));
+  ok = up.ok && upload(p->ex64, e, up.st);
+  if (want64) ok = ok && upload(p->Fx64, F, up.st) && (dst || upload(p->Ix64, I, up.st));
+  if (p->split_ok) ok = ok && upload_split(p->fx, F, p->hx, p->kx, p->halfx, up.st) &&
+                        (dst || upload_split(p->ix, I, p->hx, p->kx, p->halfx, up.st));
   folded_tables(kind, ny, dy, p->hy, p->ky, F, I, e);
-  ok = ok && upload(p->ey64, e);
-  if (want64) ok = ok && upload(p->Fy64, F) && (dst || upload(p->Iy64, I));
-  if (p->split_ok) ok = ok && upload_split(p->fy, F, p->hy, p->ky, p->halfy) &&
-                        (dst || upload_split(p->iy, I, p->hy, p->ky, p->halfy));
-  ok = ok && cudaMemcpy(p->lam_dev, lambdas, sizeof(double) * n_lambda, cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemset(p->err, 0, sizeof(int)) == cudaSuccess;
+  ok = ok && upload(p->ey64, e, up.st);
+  if (want64) ok = ok && upload(p->Fy64, F, up.st) && (dst || upload(p->Iy64, I, up.st));
+  if (p->split_ok) ok = ok && upload_split(p->fy, F, p->hy, p->ky, p->halfy, up.st) &&
+                        (dst || upload_split(p->iy, I, p->hy, p->ky, p->halfy, up.st));
+  ok = ok && upload(p->lam_dev, p->lam_host, up.st) && cudaMemsetAsync(p->err, 0, sizeof(int), up.st) == cudaSuccess;
   for (int l = 0; ok && p->split_ok && l < n_lambda; l += 65535) {
     const int nl = std::min(65535, n_lambda - l);
-    inv_eig_kernel<<<dim3(std::min(p->ky, 148 * 8), nl), 256>>>(p->ey64, p->ex64, p->ky, p->kx, p->lam_dev + l,
-                                                               p->inv32 + (size_t)l * p->ky * p->kx);
+    inv_eig_kernel<<<dim3(std::min(p->ky, 148 * 8), nl), 256, 0, up.st>>>(p->ey64, p->ex64, p->ky, p->kx, p->lam_dev + l,
+                                                                         p->inv32 + (size_t)l * p->ky * p->kx);
   }
-  if (!ok || cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+  if (!ok || cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(up.st) != cudaSuccess) {
     dst_free(p);
     delete p;
     return FVX_ERR_CUDA;
@@ -1676,6 +1697,45 @@ extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, dou
   *out = p;
   return FVX_OK;
 }
+
+// Id of the capture that ``stream`` is in, 0 outside one.
+extern "C" int fvx_capture_id(void* stream, unsigned long long* id) {
+  cudaStreamCaptureStatus s;
+  if (!id) return FVX_ERR_ARG;
+  *id = 0;
+  if (cudaStreamGetCaptureInfo(fvx_stream(stream), &s, id) != cudaSuccess) return FVX_ERR_CUDA;
+  if (s != cudaStreamCaptureStatusActive) *id = 0;
+  return s == cudaStreamCaptureStatusInvalidated ? FVX_ERR_CUDA : FVX_OK;
+}
+
+// Counts the graph being captured on ``stream`` as a holder of the plan, until
+// the graph and all that was instantiated from it are destroyed (a user object
+// that the graph owns; its destructor makes no CUDA call).
+extern "C" int fvx_dst_plan_hold(fvx_dst_plan* p, void* stream) {
+  if (!p) return FVX_ERR_ARG;
+  cudaStreamCaptureStatus s;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(fvx_stream(stream), &s, nullptr, &graph) != cudaSuccess) return FVX_ERR_CUDA;
+  if (s != cudaStreamCaptureStatusActive || !graph) return FVX_ERR_ARG;
+  using Count = std::shared_ptr<std::atomic<int>>;
+  auto* ref = new Count(p->holds);
+  auto release = [](void* r) {
+    (*(Count*)r)->fetch_sub(1);
+    delete (Count*)r;
+  };
+  cudaUserObject_t obj;
+  if (cudaUserObjectCreate(&obj, ref, release, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    delete ref;
+    return FVX_ERR_CUDA;
+  }
+  p->holds->fetch_add(1);
+  if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    cudaUserObjectRelease(obj, 1);
+    return FVX_ERR_CUDA;
+  }
+  return FVX_OK;
+}
+extern "C" int fvx_dst_plan_holds(fvx_dst_plan* p) { return p ? p->holds->load() : -1; }
 
 extern "C" int fvx_dst_plan_destroy(fvx_dst_plan* p) {
   if (!p) return FVX_ERR_ARG;

@@ -143,6 +143,14 @@ class DSTHelmholtzPlan:
         """Bound, in SM clock cycles, on each barrier wait of the products."""
         check(fn("fvx_dst_plan_set_wait_limit")(self._h, ctypes.c_longlong(int(cycles))), "wait limit")
 
+    def hold(self, stream: int) -> None:
+        """Counts the graph being captured on ``stream`` as a holder."""
+        check(fn("fvx_dst_plan_hold")(self._h, ctypes.c_void_p(stream)), "plan in a capture")
+
+    def holds(self) -> int:
+        """Graphs that hold the plan: it has to live while there are any."""
+        return fn("fvx_dst_plan_holds")(self._h)
+
     def set_kernel(self, kind: int) -> None:
         """Even/odd product kernel of this plan (an index of autotune's
         DST_KERNELS); -1: the process's choice."""
@@ -155,18 +163,26 @@ class _PlanPool:
     asked of it.  A problem keeps the plans of at most ``STREAMS`` streams (all
     that PyTorch hands out, and the default one); the oldest goes first.
 
+    A capture gets plans of its own, made during it: its graph runs on any
+    stream, at any time, so it shares no workspace with calls outside.  They
+    live until their graph is gone, and serve the next capture after that.
+
     ``make(key, batch, fp64)`` creates a plan."""
 
     STREAMS = 33
 
     def __init__(self, make):
         self._make, self._plans, self._lock = make, {}, threading.Lock()
+        self._held: list = []  # ((key, stream, capture), plan) of graphs
 
     @staticmethod
     def _serves(p, batch, fp64) -> bool:
         return p is not None and p.batch_max >= batch and (p.fp64 or not fp64)
 
-    def get(self, key, stream: int, batch: int, fp64: bool, capturing: bool):
+    def get(self, key, stream: int, batch: int, fp64: bool, capture: int = 0):
+        """``capture``: the id of the capture ``stream`` is in, or 0."""
+        if capture:
+            return self._for_graph(key, stream, batch, fp64, capture)
         p = self._plans.get((key, stream))
         if self._serves(p, batch, fp64):
             return p
@@ -174,24 +190,42 @@ class _PlanPool:
             p = self._plans.get((key, stream))
             if self._serves(p, batch, fp64):
                 return p
+            self._held = [(k, h) for k, h in self._held if h.holds()]
             others = [k for k in self._plans if k[0] == key and k[1] != stream]
-            if capturing:  # nothing can be allocated: a plan made on another stream
-                for k in others:
-                    if self._serves(self._plans[k], batch, fp64):
-                        return self._plans[k]
-            elif p is None and len(others) >= self.STREAMS:
+            if p is None and len(others) >= self.STREAMS:
                 del self._plans[others.pop(0)]
             if p is not None:  # replaced by one that serves its callers too
                 batch, fp64 = max(batch, p.batch_max), fp64 or p.fp64
             try:
                 p = self._make(key, batch, fp64)
             except L.FvxError:
-                if capturing or not others:
+                if not others:
                     raise
                 for k in others:  # give the other streams' memory back and try again
                     del self._plans[k]
                 p = self._make(key, batch, fp64)
             self._plans[(key, stream)] = p
+            return p
+
+    def _for_graph(self, key, stream, batch, fp64, capture):
+        with self._lock:
+            for k, p in self._held:
+                if k == (key, stream, capture) and self._serves(p, batch, fp64):
+                    return p
+            free = [h for h in self._held if h[0][0] == key and not h[1].holds() and self._serves(h[1], batch, fp64)]
+            if free:
+                self._held.remove(free[0])
+                p = free[0][1]
+            else:
+                try:
+                    p = self._make(key, batch, fp64)
+                except L.FvxError:  # no memory for another: the graph takes one over
+                    k = next((k for k, e in self._plans.items() if k[0] == key and self._serves(e, batch, fp64)), None)
+                    if k is None:
+                        raise
+                    p = self._plans.pop(k)
+            p.hold(stream)
+            self._held.append(((key, stream, capture), p))
             return p
 
 
@@ -211,11 +245,16 @@ def _lambda_tuple(lam) -> tuple:
 
 
 def get_plan(ny, nx, dx, dy, lambdas, batch, fp64=True, bc: str = "dst") -> DSTHelmholtzPlan:
-    """The current stream's plan of a problem, for up to ``batch`` fields."""
+    """The current stream's plan of a problem, for up to ``batch`` fields; during
+    a capture, one that belongs to its graph."""
     dev = torch.cuda.current_device()
     key = (bc, ny, nx, float(dx), float(dy), _lambda_tuple(lambdas), dev)
-    return _POOL.get(key, torch._C._cuda_getCurrentRawStream(dev), batch, fp64,
-                     torch.cuda.is_current_stream_capturing())
+    stream, capture = torch._C._cuda_getCurrentRawStream(dev), 0
+    if torch.cuda.is_current_stream_capturing():
+        cid = ctypes.c_ulonglong()
+        check(fn("fvx_capture_id")(ctypes.c_void_p(stream), ctypes.byref(cid)), "capture")
+        capture = cid.value
+    return _POOL.get(key, stream, batch, fp64, capture)
 
 
 def _solve(rhs, dx, dy, lambda_, method, bc):

@@ -183,6 +183,15 @@ int fvx_capacitance_rhs_f32(const float* f, const float* u, const double* cinv, 
                             long long n, float* out, void* stream);
 int fvx_capacitance_rhs_f64(const double* f, const double* u, const double* cinv, const long long* idx, int nb,
                             long long n, double* out, void* stream);
+/* Plans and CUDA graphs.  A plan may be created during a capture.
+ * fvx_capture_id: id of the capture ``stream`` is in (0: none).
+ * fvx_dst_plan_hold counts the graph being captured on ``stream`` as a holder
+ * of the plan until it, and all instantiated from it, is destroyed;
+ * fvx_dst_plan_holds is the number of holders, and the plan has to live while
+ * it is not 0.  No counterpart in finitevolX. */
+int fvx_capture_id(void* stream, unsigned long long* id);
+int fvx_dst_plan_hold(fvx_dst_plan* plan, void* stream);
+int fvx_dst_plan_holds(fvx_dst_plan* plan);
 /* Reads the plan's device error flag (7 if a bounded wait gave up); syncs. */
 int fvx_dst_plan_check(fvx_dst_plan* plan, void* stream);
 /* Bound on every barrier wait inside the plan's tensor-core products, in SM

@@ -1,5 +1,6 @@
 """The pool of spectral plans (host logic, no GPU), on stand-ins for plans: no
-two streams share workspaces, batches grow, the pool is bounded."""
+two streams share workspaces, no graph shares them with anything, batches grow,
+the pool is bounded."""
 
 import threading
 import time
@@ -12,19 +13,25 @@ from finitevolx_b200.solvers.spectral import _PlanPool
 
 class Plan:
     def __init__(self, key, batch, fp64):
-        self.key, self.batch_max, self.fp64 = key, batch, fp64
+        self.key, self.batch_max, self.fp64, self.graphs = key, batch, fp64, 0
+
+    def hold(self, stream):
+        self.graphs += 1
+
+    def holds(self):
+        return self.graphs
 
 
 def test_streams_have_their_own_plans():
     pool = _PlanPool(Plan)
-    a = pool.get("p", 0, 2, True, False)
-    assert pool.get("p", 0, 1, True, False) is a
-    b = pool.get("p", 7, 2, True, False)
-    assert b is not a and pool.get("p", 7, 2, True, False) is b
-    assert pool.get("other", 0, 2, True, False) not in (a, b)
-    grown = pool.get("p", 0, 5, True, False)
-    assert grown.batch_max == 5 and pool.get("p", 0, 2, True, False) is grown
-    assert pool.get("p", 7, 2, True, False) is b
+    a = pool.get("p", 0, 2, True)
+    assert pool.get("p", 0, 1, True) is a
+    b = pool.get("p", 7, 2, True)
+    assert b is not a and pool.get("p", 7, 2, True) is b
+    assert pool.get("other", 0, 2, True) not in (a, b)
+    grown = pool.get("p", 0, 5, True)
+    assert grown.batch_max == 5 and pool.get("p", 0, 2, True) is grown
+    assert pool.get("p", 7, 2, True) is b
 
 
 def test_threads_create_one_plan():
@@ -37,7 +44,7 @@ def test_threads_create_one_plan():
 
     pool = _PlanPool(make)
     got = []
-    threads = [threading.Thread(target=lambda: got.append(pool.get("p", 0, 1, True, False))) for _ in range(8)]
+    threads = [threading.Thread(target=lambda: got.append(pool.get("p", 0, 1, True))) for _ in range(8)]
     for t in threads:
         t.start()
     for t in threads:
@@ -47,11 +54,11 @@ def test_threads_create_one_plan():
 
 def test_bounded_oldest_first():
     pool = _PlanPool(Plan)
-    plans = [pool.get("p", s, 1, True, False) for s in range(_PlanPool.STREAMS)]
-    extra = pool.get("p", 100, 1, True, False)
-    assert pool.get("p", 100, 1, True, False) is extra
-    assert all(pool.get("p", s, 1, True, False) is plans[s] for s in range(2, _PlanPool.STREAMS))
-    assert pool.get("p", 0, 1, True, False) is not plans[0]
+    plans = [pool.get("p", s, 1, True) for s in range(_PlanPool.STREAMS)]
+    extra = pool.get("p", 100, 1, True)
+    assert pool.get("p", 100, 1, True) is extra
+    assert all(pool.get("p", s, 1, True) is plans[s] for s in range(2, _PlanPool.STREAMS))
+    assert pool.get("p", 0, 1, True) is not plans[0]
 
 
 def test_memory_of_other_streams_is_given_back():
@@ -65,29 +72,66 @@ def test_memory_of_other_streams_is_given_back():
         return Plan(key, batch, fp64)
 
     pool = _PlanPool(make)
-    a, b = pool.get("p", 0, 1, True, False), pool.get("p", 1, 1, True, False)
-    c = pool.get("p", 2, 1, True, False)
-    assert pool.get("p", 2, 1, True, False) is c
-    assert pool.get("p", 0, 1, True, False) is not a
+    a, b = pool.get("p", 0, 1, True), pool.get("p", 1, 1, True)
+    c = pool.get("p", 2, 1, True)
+    assert pool.get("p", 2, 1, True) is c
+    assert pool.get("p", 0, 1, True) is not a
 
     def never(*args):
         raise FvxError("memory")
 
     with pytest.raises(FvxError):
-        _PlanPool(never).get("p", 0, 1, True, False)
-
-
-def test_capture_uses_a_plan_made_before():
-    pool = _PlanPool(Plan)
-    a = pool.get("p", 0, 2, True, False)
-    assert pool.get("p", 9, 2, True, True) is a
+        _PlanPool(never).get("p", 0, 1, True)
 
 
 def test_fp64_is_part_of_the_request():
     pool = _PlanPool(Plan)
-    a = pool.get("p", 0, 4, False, False)
-    b = pool.get("p", 0, 1, True, False)
+    a = pool.get("p", 0, 4, False)
+    b = pool.get("p", 0, 1, True)
     assert b.fp64 and b.batch_max == 4
-    assert pool.get("p", 0, 4, False, False) is b and pool.get("p", 0, 2, True, False) is b and a is not b
-    pool.get("p", 1, 1, False, False)
-    assert pool.get("p", 2, 1, True, True) is b  # a capture takes one that has it
+    assert pool.get("p", 0, 4, False) is b and pool.get("p", 0, 2, True) is b and a is not b
+
+
+def test_graphs_have_their_own_plans():
+    pool = _PlanPool(Plan)
+    eager = pool.get("p", 0, 1, True)
+    g = pool.get("p", 9, 1, True, capture=4)
+    assert g is not eager and g.graphs == 1
+    assert pool.get("p", 9, 1, True, capture=4) is g and g.graphs == 1
+    fork = pool.get("p", 8, 1, True, capture=4)  # another stream of the same capture
+    other = pool.get("p", 9, 1, True, capture=5)
+    assert len({id(p) for p in (eager, g, fork, other)}) == 4
+    # outgrown in its capture and outside: still there for the replay
+    grown = pool.get("p", 9, 3, True, capture=4)
+    assert grown is not g and pool.get("p", 0, 3, True) is not eager
+    assert {id(p) for _, p in pool._held} == {id(p) for p in (g, fork, other, grown)}
+    assert pool.get("p", 0, 1, True).graphs == 0
+
+
+def test_a_graphs_plan_goes_with_it():
+    pool = _PlanPool(Plan)
+    g, h = pool.get("p", 9, 1, True, capture=4), pool.get("p", 9, 1, True, capture=5)
+    g.graphs = 0  # destroyed: free for the next capture
+    assert pool.get("q", 9, 1, True, capture=6) is not g and pool.get("p", 9, 2, True, capture=6) is not g
+    assert pool.get("p", 9, 1, True, capture=7) is g and g.graphs == 1
+    g.graphs = 0
+    pool.get("p", 0, 1, True)  # a plan is made outside: what no graph holds goes
+    assert h in [p for _, p in pool._held] and g not in [p for _, p in pool._held]
+
+
+def test_a_graph_takes_a_plan_over_when_memory_is_short():
+    room = [1]
+
+    def make(key, batch, fp64):
+        if not room[0]:
+            raise FvxError("memory")
+        room[0] -= 1
+        return Plan(key, batch, fp64)
+
+    pool = _PlanPool(make)
+    a = pool.get("p", 0, 2, True)
+    assert pool.get("p", 9, 1, True, capture=4) is a and a.graphs == 1
+    room[0] = 1
+    assert pool.get("p", 0, 2, True) is not a
+    with pytest.raises(FvxError):
+        pool.get("p", 9, 8, True, capture=6)
