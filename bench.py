@@ -31,6 +31,9 @@ field (std 1e-5 s^-1), synthetic.
   refinement, the masked Helmholtz learned-PCG vs MG-PCG comparison and the
   ensemble of uneven members.
 
+The JSON line on stdout holds the headline keys (about 2 KB); it and the
+sections go to ``--sections`` (bench_sections.json beside this file).
+
 Multi-GPU (--gpus N under torchrun): the single-field step does not shard;
 each rank runs an independent replica ("replicas only"), value sums ranks.
 The ensemble shards by members (each rank its own members, no collective
@@ -89,8 +92,19 @@ def parse():
                     help="only U-Net training steps at batch 64 on 128^2 (seeded synthetic inputs; for ncu launch "
                          "lists and the per-step time)")
     ap.add_argument("--ens-steps", type=int, default=100)
+    ap.add_argument("--sections", default=os.path.join(ROOT, "bench_sections.json"),
+                    help="file for the whole result with the extra sections ('' for none)")
     ap.add_argument("--stage-tile", default=None, help="fix the stage tile (e.g. 64x32) instead of autotuning")
     return ap.parse_args()
+
+
+SECTIONS = ("stage_kernel", "fused_vs_unfused", "fp64_metric_config", "stencil_sweep", "dst_batched", "helmholtz",
+            "ensemble")
+
+
+def headline(res: dict) -> str:
+    """The JSON line: everything but the extra sections."""
+    return json.dumps({k: v for k, v in res.items() if k not in SECTIONS})
 
 
 def config(n, method):
@@ -190,9 +204,7 @@ def cpu_baseline(n, method, steps=3):
     first, times, cores = _oracle_steps(n, method, steps)
     t = sum(times)
     return {"value": n * n * steps / t / 1e6, "unit": UNIT, "cores": cores, "kind": "port",
-            "sample": f"{steps} rk3_ssp_steps at {n}x{n} from the bench's initial state, FP64 NumPy/SciPy oracle "
-                      f"(restatement of the reference math; finitevolX's JAX stack is not installable offline), "
-                      f"{cores} host threads (row bands + SciPy FFT workers), {t:.1f} s"}, first
+            "sample": f"{steps} steps at {n}x{n}, FP64 NumPy/SciPy oracle, {cores} host threads, {t:.1f} s"}, first
 
 
 def run_reference(args, rank):
@@ -916,11 +928,10 @@ def main():
             "warmup": args.warmup, "ms_per_step": t_max / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": dict(config(n, args.method), autotuned=tuned,
-                           helmholtz="DST-I as tensor-core transform-matrix products, 3xBF16 split, FP32 accumulate"),
+                           helmholtz="DST-I products, 3xBF16 split, FP32 accumulate"),
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": nbytes, "d2h_bytes_per_step": nbytes,
                     "ms_per_step": e2e_ms / args.steps,
-                    "form": "QGPipeline: upload of state k+1, step k (CUDA graph), download of k-1 on three "
-                            "streams; L2 flushed before every step"},
+                    "form": "QGPipeline: upload k+1, step k, download k-1 on three streams"},
             "gpu_launches": per_step_launches * args.steps,
             "roofline": {"bound": "tensor",
                          "kernel": ("gemm_sym_bf16_kernel (even/odd DST-I product, 3xBF16)" if sym
@@ -928,7 +939,7 @@ def main():
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_source": peak_src,
                          "traffic": traffic, "traffic_unit": "bytes",
-                         "traffic_source": "profiles/dst_product_traffic.json (ncu capture of this kernel)"
+                         "traffic_source": "profiles/dst_product_traffic.json (ncu)"
                                            if traffic else None,
                          "per_launch_ms": gemm_ms, "algorithmic_flops_per_launch": flops,
                          "executed_tensor_flops_per_launch": (3.0 if sym else 6.0) * n ** 3,
@@ -950,8 +961,7 @@ def main():
             if rank == 0 and np.array_equal(q0_host, initial_q(n)):
                 err = float(np.abs(q1_gpu - q1_ref).max() / np.abs(q1_ref).max())
                 res["parity"] = {"rel_err_vs_fp64_oracle": err, "bar": 1e-5, "passed": err < 1e-5,
-                                 "what": "max|q1_gpu - q1_oracle| / max|q1_oracle| after one step from the bench's "
-                                         "initial state (FP64 oracle)"}
+                                 "what": "max|q1 - q1_oracle| / max|q1_oracle| after one step"}
         if world == 1 and not args.no_fp64:
             res["fp64_metric_config"] = fp64_metric_section(args.method, args.steps, flush)
         if world == 1 and not args.no_sweep:
@@ -970,7 +980,13 @@ def main():
         if rank == 0:
             res["ensemble"] = ens
     if rank == 0:
-        print(json.dumps(res))
+        if args.sections:
+            try:
+                with open(args.sections, "w") as f:
+                    json.dump(res, f, indent=1)
+            except OSError as e:  # the line does not depend on it
+                print(f"bench: no sections file: {e}", file=sys.stderr)
+        print(headline(res))
     if world > 1:
         dist.barrier()
         del graphs
