@@ -916,7 +916,7 @@ def main():
     try:
         with open(os.path.join(ROOT, "profiles", "dst_product_traffic.json")) as f:
             tr = json.load(f)
-        if tr.get("n") == n and tr.get("kernel") == ("gemm_sym_bf16_kernel" if sym else "gemm_split_bf16_kernel"):
+        if sym and tr.get("n") == n and tr.get("kernel") == "gemm_sym_bf16_kernel":
             traffic = tr.get("dram_bytes_per_launch")
     except Exception:
         pass
@@ -934,16 +934,17 @@ def main():
                     "form": "QGPipeline: upload k+1, step k, download k-1 on three streams"},
             "gpu_launches": per_step_launches * args.steps,
             "roofline": {"bound": "tensor",
-                         "kernel": ("gemm_sym_bf16_kernel (even/odd DST-I product, 3xBF16)" if sym
-                                    else "gemm_split_bf16_kernel (DST product, 3xBF16)"),
+                         "kernel": ("gemm_sym_bf16_kernel (even/odd DST-I product, 3xBF16)" if sym and n == 2048
+                                    else "folded DST-I product, 3xBF16 (gemm_sym or gemm_fold by size)"),
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_source": peak_src,
                          "traffic": traffic, "traffic_unit": "bytes",
                          "traffic_source": "profiles/dst_product_traffic.json (ncu)"
                                            if traffic else None,
                          "per_launch_ms": gemm_ms, "algorithmic_flops_per_launch": flops,
-                         "executed_tensor_flops_per_launch": (3.0 if sym else 6.0) * n ** 3,
-                         "executed_frac": (3.0 if sym else 6.0) * n ** 3 / (gemm_ms * 1e-3) / 1e12 / peak},
+                         # two half-length products of three split passes each
+                         "executed_tensor_flops_per_launch": 3.0 * n ** 3,
+                         "executed_frac": 3.0 * n ** 3 / (gemm_ms * 1e-3) / 1e12 / peak},
             "stage_kernel": {"bound": "hbm", "kernel": f"qg stage_kernel<float, {args.method.upper()}>",
                              "per_launch_ms": stage_ms, "algorithmic_bytes_per_launch": stage_bytes,
                              "achieved": stage_bytes / (stage_ms * 1e-3) / 1e9, "unit": "GB/s",
