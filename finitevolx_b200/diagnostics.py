@@ -99,14 +99,26 @@ def qg_potential_vorticity(psi, f0: float, beta: float, dx: float, dy: float, y,
 _SUM_WORK = {}
 
 
+def _sum_work(dev):
+    """Partial sums and the ticket of the last block: one pair per stream (a
+    launch leaves the ticket at 0 for the next), a graph's in its own memory."""
+    def make():
+        return (torch.empty(296, dtype=torch.float64, device=dev), torch.zeros(1, dtype=torch.int32, device=dev))
+
+    if torch.cuda.is_current_stream_capturing():
+        return make()
+    key = (dev, torch._C._cuda_getCurrentRawStream(dev.index))
+    work = _SUM_WORK.get(key)
+    if work is None:
+        work = _SUM_WORK.setdefault(key, make())
+    return work
+
+
 def _interior_sum(a, b, scale):
     a = L.as_field(a)
     b = None if b is None else L.as_field(b, dtype=a.dtype)
     dev = a.device
-    if dev not in _SUM_WORK:
-        _SUM_WORK[dev] = (torch.empty(296, dtype=torch.float64, device=dev),
-                          torch.zeros(1, dtype=torch.int32, device=dev))
-    part, ticket = _SUM_WORK[dev]
+    part, ticket = _sum_work(dev)
     out = torch.empty((), dtype=torch.float64, device=dev)
     ny, nx = a.shape
     check(fn(f"fvx_interior_sum_{sfx(a)}")(P(a), P(b), I(ny), I(nx), D(scale), P(part), P(ticket), P(out),
