@@ -31,18 +31,13 @@ class CGInfo(NamedTuple):
     converged: bool
 
 
-_PART = {}
-
-
 def _dot(a, b) -> torch.Tensor:
     """FP64-accumulated inner product as a device scalar."""
-    dev = a.device
-    if dev not in _PART:
-        _PART[dev] = torch.empty(296, dtype=torch.float64, device=dev)
-    out = torch.empty((), dtype=torch.float64, device=dev)
-    check(fn(f"fvx_dot_{sfx(a)}")(P(a), P(b), ctypes.c_int64(a.numel()), P(_PART[dev]), P(out), stream_ptr()),
-          "dot")
-    return out
+    # the result, then the partial sums of its two launches: the call's own, so
+    # that neither another stream nor another thread writes between them
+    work = torch.empty(297, dtype=torch.float64, device=a.device)
+    check(fn(f"fvx_dot_{sfx(a)}")(P(a), P(b), ctypes.c_int64(a.numel()), P(work[1:]), P(work), stream_ptr()), "dot")
+    return work[0]
 
 
 def _maxabs(a) -> float:

@@ -1,5 +1,5 @@
-"""Domain integrals on several streams at once and in graphs: the bits of the
-same sums alone (their partial sums and tickets are not shared)."""
+"""Domain integrals and inner products on several streams at once and in graphs:
+the bits of the same sums alone (partial sums and tickets are not shared)."""
 
 import pytest
 import torch
@@ -41,3 +41,19 @@ def test_integral_in_a_graph(cuda_ok):
         eager = D.total_energy(f, f, 0.3, 0.2)
         torch.cuda.synchronize()
         assert float(out) == float(out2) == ref and float(eager) == want[0]
+
+
+def test_inner_products_on_streams(cuda_ok):
+    from finitevolx_b200.solvers.iterative import _dot
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    fs = [torch.randn(300 + 200 * k, 700, device="cuda", dtype=torch.float64, generator=gen) for k in range(8)]
+    alone = [float(_dot(f, f)) for f in fs]
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    torch.cuda.synchronize()
+    got = [[] for _ in fs]
+    for _ in range(20):
+        for k, f in enumerate(fs):
+            with torch.cuda.stream(streams[k % 4]):
+                got[k].append(_dot(f, f))
+    torch.cuda.synchronize()
+    assert all(float(x) == ref for xs, ref in zip(got, alone) for x in xs)
