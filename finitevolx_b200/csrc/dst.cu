@@ -9,15 +9,20 @@
 // unnormalised DST-I is 2 S and its inverse S / (N+1), so
 //   psi = 4 / ((Ny+1)(Nx+1)) * S_y ((S_y f S_x) ./ Lambda) S_x.
 //
-// The four products run as one GEMM shape, C = X S (X row-major, S
-// symmetric, so both operands are K-major), whose epilogue stores C
-// transposed: the chain Q -> (Q S_x)^T -> (S_y Q S_x ./ Lambda) ->
-// (. S_x)^T -> psi needs no transpose kernels and every operand is a
-// K-major TMA tile.  Precision: 3xBF16 split (X = Xh + Xl, S = Sh + Sl,
-// C = Xh Sh + Xh Sl + Xl Sh) with FP32 accumulation in TMEM; the epilogue
-// writes the next product's operand already split into bf16 hi/lo.  An FP64
-// form of the same chain (dst_f64.cuh) is the correctness path, and the FP64
-// solve recovers full accuracy by iterative refinement with an FP64 residual.
+// The four products run as one GEMM shape whose epilogue stores C transposed:
+// the chain Q -> (Q S_x)^T -> (S_y Q S_x ./ Lambda) -> (. S_x)^T -> psi needs
+// no transpose kernels and every operand is a K-major TMA tile.  Each product
+// is folded by parity into two of half the length (the algebra, also for the
+// cosine and periodic transforms, in dst_f64.cuh).  Precision: 3xBF16 split (X
+// = Xh + Xl, S = Sh + Sl, C = Xh Sh + Xh Sl + Xl Sh) with FP32 accumulation in
+// TMEM; the epilogue writes the next product's operand already split into bf16
+// hi/lo, odd columns after the even ones.  Kernels: gemm_sym_bf16_kernel (128
+// x 128 tiles, sizes that are multiples of 256; gemm_sym_tiles_kernel where
+// there are more tiles than SMs, the pair form by choice), gemm_fold_bf16_kernel
+// (dst_fold.cuh; sides that are multiples of 8, 128 x 32 .. 128 tiles) and, for
+// the allocation-free entry only, the dense gemm_split_bf16_kernel.  An FP64 form of the same chain
+// (dst_f64.cuh) is the correctness path, and the FP64 solve recovers full
+// accuracy by iterative refinement with an FP64 residual.
 #include "dst_f64.cuh"
 
 #include <cuda.h>
@@ -46,7 +51,7 @@ constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 constexpr int THREADS = 192;                               // TMA warp, MMA warp, 4 epilogue warps
 constexpr long long kWaitCycles = 4000000000LL;            // default bound on every spin-wait (~2 s)
 
-enum EpiMode { EPI_SPLIT = 0, EPI_F32 = 1, EPI_F64 = 2, EPI_F64_ACC = 3, EPI_F32_ACC = 4 };
+enum EpiMode { EPI_SPLIT, EPI_F32, EPI_F64_ACC, EPI_F32_ACC };
 
 struct Epi {
   int mode;
@@ -57,7 +62,6 @@ struct Epi {
   void* out1;              // lo output (split mode)
   long long batch_stride;  // elements between batches in the output
   long long ld;            // elements between consecutive n rows of the (transposed) output
-  int off_n, off_r;        // index offsets into the output (e.g. a ghost ring)
   double alpha;
   const float* inv_eig;    // [n_eig][N][R] scale 1/Lambda, or null
   int n_eig;               // batch b uses grid b % n_eig
@@ -246,7 +250,7 @@ DEV int deinterleave(int r, int R) { return (r & 1) ? (R >> 1) + (r >> 1) : (r >
 
 DEV void epi_store(const Epi& ep, int b, int r, int n, float acc) {
   const int rs = ep.perm_r ? deinterleave(r, ep.rows_per_batch) : r;
-  long long idx = (long long)b * ep.batch_stride + (long long)(n + ep.off_n) * ep.ld + (rs + ep.off_r);
+  const long long idx = (long long)b * ep.batch_stride + (long long)n * ep.ld + rs;
   switch (ep.mode) {
     case EPI_SPLIT: {
       float x = acc * (float)ep.alpha;
@@ -263,9 +267,6 @@ DEV void epi_store(const Epi& ep, int b, int r, int n, float acc) {
       ((float*)ep.out0)[idx] = x;
       break;
     }
-    case EPI_F64:
-      ((double*)ep.out0)[idx] = (double)acc * ep.alpha;
-      break;
     case EPI_F32_ACC:
       ((float*)ep.out0)[idx] += acc * (float)ep.alpha;
       break;
@@ -275,7 +276,7 @@ DEV void epi_store(const Epi& ep, int b, int r, int n, float acc) {
   }
 }
 
-// ---- the tcgen05 GEMM -------------------------------------------------------
+// ---- the dense tcgen05 GEMM (allocation-free entry) -------------------------------------------------------
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_bf16_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
                        const __grid_constant__ CUtensorMap mBh, const __grid_constant__ CUtensorMap mBl, int K,
@@ -1350,8 +1351,8 @@ static int gemm_sym(int kind, const bf16* Xh, const bf16* Xl, int M, int K, cons
   const long long tiles = (long long)(KH / SBN) * ((M + BM - 1) / BM);
   bool walk = kind == 0 && tiles > kSMs && tiles <= INT_MAX;
   const uint32_t box_n = walk ? T_COLS : 16;
-  if ((ep.mode == EPI_SPLIT || ep.mode == EPI_F32) && R % BM == 0 && M % R == 0 && ep.off_n == 0 &&
-      ep.off_r == 0 && ep.n_cols == K && (ep.mode == EPI_F32 || ep.perm_r)) {
+  if ((ep.mode == EPI_SPLIT || ep.mode == EPI_F32) && R % BM == 0 && M % R == 0 && ep.n_cols == K &&
+      (ep.mode == EPI_F32 || ep.perm_r)) {
     const uint64_t B = (uint64_t)(M / R);
     bool okm = ep.mode == EPI_SPLIT
                    ? make_out_map(&o0, ep.out0, false, R, K, B, ep.ld, ep.batch_stride, 64, box_n) &&
@@ -1778,10 +1779,10 @@ extern "C" int fvx_dst_plan_inject_stall(fvx_dst_plan* p, int on) {
 }
 
 static Epi make_epi(fvx_dst_plan* p, int mode, int R, int M, int N, void* o0, void* o1, long long bstride,
-                    long long ld, int off_n, int off_r, double alpha, bool eig) {
+                    long long ld, double alpha, bool eig) {
   Epi e;
   e.mode = mode; e.rows_per_batch = R; e.m_total = M; e.n_cols = N; e.out0 = o0; e.out1 = o1;
-  e.batch_stride = bstride; e.ld = ld; e.off_n = off_n; e.off_r = off_r; e.alpha = alpha;
+  e.batch_stride = bstride; e.ld = ld; e.alpha = alpha;
   e.inv_eig = eig ? p->inv32 : nullptr; e.n_eig = p->n_lam;
   e.err = p->err;
   e.wait_cycles = p->wait_cycles;
@@ -1823,7 +1824,7 @@ static Epi operand_epi(fvx_dst_plan* p, int k, int B, bf16* oh, bf16* ol) {
   const int R = along_x ? p->ky : p->kx;             // rows per batch
   const int N = k == 2 ? p->nx : (along_x ? p->kx : p->ky);  // output rows
   const int pitch = 2 * (along_x ? p->halfy : p->halfx);
-  Epi e = make_epi(p, EPI_SPLIT, R, B * R, N, oh, ol, (long long)N * pitch, pitch, 0, 0, 1.0, k == 1);
+  Epi e = make_epi(p, EPI_SPLIT, R, B * R, N, oh, ol, (long long)N * pitch, pitch, 1.0, k == 1);
   e.perm_r = 1;
   return e;
 }
@@ -1847,7 +1848,7 @@ static int chain_split(fvx_dst_plan* p, int B, int out_mode, void* out, long lon
   if ((rc = split_product(p, ah, al, true, false, operand_epi(p, 0, B, bh, bl), st))) return rc;
   if ((rc = split_product(p, bh, bl, false, false, operand_epi(p, 1, B, ah, al), st))) return rc;
   if ((rc = split_product(p, ah, al, true, true, operand_epi(p, 2, B, bh, bl), st))) return rc;
-  Epi e4 = make_epi(p, out_mode, p->nx, B * p->nx, p->ny, out, nullptr, ob, old, 0, 0, p->cfin, false);
+  Epi e4 = make_epi(p, out_mode, p->nx, B * p->nx, p->ny, out, nullptr, ob, old, p->cfin, false);
   return split_product(p, bh, bl, false, true, e4, st);
 }
 
@@ -2224,7 +2225,7 @@ extern "C" int fvx_dst_solve_noalloc_f32(const float* rhs, long long rhs_ld, flo
                  bool eig) {
     Epi e;
     e.mode = mode; e.rows_per_batch = R; e.m_total = M; e.n_cols = N; e.out0 = o0; e.out1 = o1;
-    e.batch_stride = bs; e.ld = ld; e.off_n = 0; e.off_r = 0; e.alpha = alpha;
+    e.batch_stride = bs; e.ld = ld; e.alpha = alpha;
     e.inv_eig = eig ? inv : nullptr; e.n_eig = 1; e.err = err;
     return e;
   };

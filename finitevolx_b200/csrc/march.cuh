@@ -1,5 +1,5 @@
 // Column marches over a shared-memory tile, shared by the fused QG stage
-// (qg_stage.cuh) and the advection kernel (stencil.cu).
+// (qg_stage.cuh) and the advection kernel (advect.cu).
 //
 // A thread owns one column of the tile and walks RW of its rows.  Per row it
 // evaluates the east and the north face of its cell from two register
@@ -11,44 +11,10 @@
 // whose cells all have the scheme's full reach takes the branch-free form;
 // one that touches an edge (or, masked, a coast) picks each face's order.
 #pragma once
+#include "f32x2.cuh"
 #include "recon.cuh"
 
 namespace fvx {
-
-// ---- packed FP32 pairs (Blackwell f32x2 arithmetic) -----------------------
-// Two independent values per instruction; each lane is an IEEE round-to-
-// nearest FP32 operation, the same as its scalar form.
-DEV unsigned long long f2pack(float2 a) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-  return r;
-}
-DEV float2 f2unpack(unsigned long long r) {
-  float2 d;
-  asm("mov.b64 {%0,%1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
-  return d;
-}
-DEV float2 f2fma(float2 a, float2 b, float2 c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(f2pack(a)), "l"(f2pack(b)), "l"(f2pack(c)));
-  return f2unpack(d);
-}
-DEV float2 f2add(float2 a, float2 b) {
-  unsigned long long d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2pack(a)), "l"(f2pack(b)));
-  return f2unpack(d);
-}
-DEV float2 f2mul(float2 a, float2 b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2pack(a)), "l"(f2pack(b)));
-  return f2unpack(d);
-}
-DEV float2 f2sub(float2 a, float2 b) {
-  unsigned long long d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(f2pack(a)), "l"(f2pack(b)));
-  return f2unpack(d);
-}
-DEV float2 f2s(float c) { return make_float2(c, c); }
 
 // WENO5 / WENO-Z5 (weno5<float, Z> in recon.cuh, the same formulas) on two
 // stencils at once: 38 packed operations and one reciprocal per lane for

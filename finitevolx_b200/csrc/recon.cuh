@@ -1,9 +1,11 @@
 // Face-value reconstructions for flux-form advection on the C-grid.
 //
 // Point formulas restate finitevolX advection/weno.py (WENO3/5 JS and Z,
-// WENO7/9 via the generic Jiang-Shu form) and advection/limiters.py, with
-// the same operation order so the FP64 build tracks the reference to
-// rounding.  The boundary fallback ladders of advection/reconstruction.py
+// WENO7/9 via the generic Jiang-Shu form) and advection/limiters.py.  They are
+// reassociated (WENO3/5 on differences of neighbouring cells, weights over a
+// common denominator, van Leer as one quotient): FP64 results agree with the
+// reference's order of operations to 1e-12 of the largest flux, not to the
+// last bit.  The boundary fallback ladders of advection/reconstruction.py
 // (WENO5 :834-864, WENO7/9 :74-236, upwind2/3 and TVD east-boundary
 // fallbacks) all reduce to one rule, used by face_value() below:
 //
@@ -26,10 +28,9 @@ DEV float rcp_approx(float b) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
   return r;
 }
-// Division in the reconstruction formulas: exact IEEE division in FP64 (the
-// correctness path tracks the reference's operation order), a times the
-// approximate reciprocal of b in FP32 (<= 2 ulp; its 2^126 < |b| < 2^128
-// corner maps to the weights an FP32 reference overflows on anyway).
+// Division in the reconstruction formulas: exact IEEE division in FP64, a times
+// the approximate reciprocal of b in FP32 (<= 2 ulp for |b| <= 2^126; WENO3/5
+// keep their denominators below that, WENO7/9 weights beyond it become 0).
 template <typename T> DEV T fdiv(T a, T b) {
   if constexpr (sizeof(T) == 8) return a / b;
   else return a * rcp_approx(b);
@@ -296,8 +297,6 @@ template <int S> struct SchemeInfo {
   static constexpr bool zfam = (S == FVX_WENOZ3 || S == FVX_WENOZ5);
   static constexpr bool tvd = (S == FVX_MINMOD || S == FVX_VAN_LEER || S == FVX_SUPERBEE || S == FVX_MC);
   // cells read on each side of the face's left cell i: [i - lo, i + hi]
-  static constexpr int halo_lo = is_weno ? reach + 1 : 1;
-  static constexpr int halo_hi = is_weno ? reach + 1 : 2;
 };
 
 // Face value at face i (between cells i and i+1) of a line of N cells.

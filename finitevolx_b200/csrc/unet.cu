@@ -8,7 +8,7 @@
 // upsample (from an h/2 x w/2 tensor), adds a bias and an optional skip
 // tensor, and applies ReLU.  The reference has no learned component; this
 // is new work measured against its multigrid preconditioner.
-#include "fvx_common.cuh"
+#include "f32x2.cuh"
 
 #include <cuda_bf16.h>
 
@@ -26,30 +26,6 @@ constexpr int CMAX = 32;
 
 // value of the conv input (channel plane ``src`` of the source tensor) at
 // conv-grid pixel (y, x); zero outside [0, h) x [0, w)
-// Two FP32 fused multiply-adds (or sums) per instruction, each lane an IEEE
-// operation: the convolutions' inner loops are bound by instruction issue.
-typedef unsigned long long f2;
-DEV f2 f2_pack(float x, float y) {
-  f2 r;
-  asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-DEV float2 f2_unpack(f2 a) {
-  float2 r;
-  asm("mov.b64 {%0,%1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
-  return r;
-}
-DEV f2 f2_fma(f2 a, f2 b, f2 c) {
-  f2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-DEV f2 f2_add(f2 a, f2 b) {
-  f2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 DEV float in_at(const float* src, int mode, int h, int w, int y, int x) {
   if (y < 0 || y >= h || x < 0 || x >= w) return 0.f;
   if (mode == IN_DIRECT) return src[(size_t)y * w + x];
@@ -847,7 +823,7 @@ conv_batch_kernel(const float* __restrict__ in, int mode, int cin, const WT* __r
           ws[(k - co * row) * WP + co] = v;
         });
   }
-  f2 acc2[kBcPX][kBcCO / 2];  // channel pairs
+  f32x2 acc2[kBcPX][kBcCO / 2];  // channel pairs
 #pragma unroll
   for (int p = 0; p < kBcPX; ++p)
 #pragma unroll
@@ -870,7 +846,7 @@ conv_batch_kernel(const float* __restrict__ in, int mode, int cin, const WT* __r
       const float* wr = ws + (size_t)(c0 + cc) * 9 * WP + g * kBcCO;
 #pragma unroll
       for (int dy = 0; dy < 3; ++dy) {
-        f2 row[kBcPX + 2];  // each input twice
+        f32x2 row[kBcPX + 2];  // each input twice
 #pragma unroll
         for (int j = 0; j < kBcPX + 2; j += 2) {
           const float2 v = *(const float2*)(xr + dy * kBcPitch + j);
@@ -881,7 +857,7 @@ conv_batch_kernel(const float* __restrict__ in, int mode, int cin, const WT* __r
         for (int dx = 0; dx < 3; ++dx) {
           const ulonglong2 wa = *(const ulonglong2*)(wr + (dy * 3 + dx) * WP);
           const ulonglong2 wb = *(const ulonglong2*)(wr + (dy * 3 + dx) * WP + 4);
-          const f2 wv[kBcCO / 2] = {wa.x, wa.y, wb.x, wb.y};
+          const f32x2 wv[kBcCO / 2] = {wa.x, wa.y, wb.x, wb.y};
 #pragma unroll
           for (int p = 0; p < kBcPX; ++p)
 #pragma unroll

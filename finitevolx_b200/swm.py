@@ -2,10 +2,12 @@
 Vorticity2D (operators/vorticity.py:14-235) and MomentumAdvection2D
 (diffusion/momentum.py:35-216).
 
-Each method is one fused libfvx.so launch (``fvx_sw2d_*``) that recomputes
-the staggered intermediates the reference materialises (interpolations,
-curl, kinetic energy and its gradient), with the same arithmetic, zero ghost
-rings and pass-down mask rules, so nothing but the outputs is written.
+Each method is one fused libfvx.so launch (``fvx_sw2d_*``): a march down the
+columns forms each staggered intermediate the reference materialises
+(interpolations, curl, kinetic energy and its gradient) once, in registers,
+with the same zero ghost rings and pass-down mask rules, so nothing but the
+outputs is written.  Quotients by dx and dy are products with their
+reciprocals.
 """
 
 from __future__ import annotations
