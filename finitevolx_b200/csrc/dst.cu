@@ -1596,19 +1596,23 @@ __global__ void inv_eig_kernel(const double* __restrict__ ey, const double* __re
 }
 
 // A plan may be created while a stream of the process is being captured: its
-// set-up runs on a stream of its own, and this thread may allocate meanwhile.
+// set-up runs on a stream of its own (one per device, made once), and this
+// thread may allocate meanwhile.
 struct PlanSetup {
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaStream_t st = nullptr;
-  bool ok;
+  bool ok = false;
   PlanSetup() {
+    static std::mutex mu;
+    static cudaStream_t streams[128] = {};
     cudaThreadExchangeStreamCaptureMode(&mode);
-    ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return;
+    std::lock_guard<std::mutex> lock(mu);
+    ok = streams[dev] || cudaStreamCreateWithFlags(&streams[dev], cudaStreamNonBlocking) == cudaSuccess;
+    st = streams[dev];
   }
-  ~PlanSetup() {
-    if (ok) cudaStreamDestroy(st);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-  }
+  ~PlanSetup() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
 extern "C" int fvx_spectral_plan_create(int kind, int ny, int nx, double dx, double dy, int batch_max,
