@@ -1447,7 +1447,7 @@ extern "C" int fvx_nn_conv_bwd(const float* in, int mode, int batch, int cin, co
   dim3 gr((w + TILE - 1) / TILE, (h + TILE - 1) / TILE, batch);
   // weight and bias gradients: P partial rows, then their fixed-order sum
   const int cot = wgrad_cot(cin, cout), sr = wgrad_strip(cin, cout, batch, h, w);
-  const int nrows = fvx_nn_conv_bwd_rows(batch, cin, cout, h, w);
+  const int nrows = std::max(1, fvx_nn_conv_bwd_rows(batch, cin, cout, h, w));  // (no samples: zero gradients)
   const size_t wsm = wgrad_smem(cin, cout, cot, sr);
   const int wrc = cot == 4   ? launch_wgrad<4>(sr, nrows, wsm, st, in, mode, cin, g, cout, h, w, batch, part)
                   : cot == 2 ? launch_wgrad<2>(sr, nrows, wsm, st, in, mode, cin, g, cout, h, w, batch, part)
