@@ -76,6 +76,11 @@ def stream_ptr() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
+def capturing() -> bool:
+    """Whether the current stream (of an initialised device) is being captured."""
+    return torch._C._cuda_isCurrentStreamCapturing()
+
+
 def P(t) -> ctypes.c_void_p:
     """Device pointer of a tensor (None -> NULL)."""
     if t is None:

@@ -105,7 +105,7 @@ def _sum_work(dev):
     def make():
         return (torch.empty(296, dtype=torch.float64, device=dev), torch.zeros(1, dtype=torch.int32, device=dev))
 
-    if torch.cuda.is_current_stream_capturing():
+    if L.capturing():
         return make()
     key = (dev, torch._C._cuda_getCurrentRawStream(dev.index))
     work = _SUM_WORK.get(key)

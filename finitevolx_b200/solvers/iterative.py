@@ -36,7 +36,8 @@ def _dot(a, b) -> torch.Tensor:
     # the result, then the partial sums of its two launches: the call's own, so
     # that neither another stream nor another thread writes between them
     work = torch.empty(297, dtype=torch.float64, device=a.device)
-    check(fn(f"fvx_dot_{sfx(a)}")(P(a), P(b), ctypes.c_int64(a.numel()), P(work[1:]), P(work), stream_ptr()), "dot")
+    check(fn(f"fvx_dot_{sfx(a)}")(P(a), P(b), ctypes.c_int64(a.numel()),
+                                  ctypes.c_void_p(work.data_ptr() + 8), P(work), stream_ptr()), "dot")
     return work[0]
 
 

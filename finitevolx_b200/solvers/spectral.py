@@ -250,7 +250,7 @@ def get_plan(ny, nx, dx, dy, lambdas, batch, fp64=True, bc: str = "dst") -> DSTH
     dev = torch.cuda.current_device()
     key = (bc, ny, nx, float(dx), float(dy), _lambda_tuple(lambdas), dev)
     stream, capture = torch._C._cuda_getCurrentRawStream(dev), 0
-    if torch.cuda.is_current_stream_capturing():
+    if L.capturing():
         cid = ctypes.c_ulonglong()
         check(fn("fvx_capture_id")(ctypes.c_void_p(stream), ctypes.byref(cid)), "capture")
         capture = cid.value
